@@ -1,0 +1,704 @@
+"""Performance cases of the explicit-dynamics framework.
+
+A case is one thing a user's program has the framework do, through its public
+entry points:
+
+  explicit   a SolidMechanicsModel advanced by `steps` graph-replayed steps
+             between two outputs, then the output itself: displacement and
+             velocity on the host, kinetic and potential energy;
+  loop       the same model stepped call by call: prescribed displacements, a
+             step and a queued kinetic energy per step, as a script that
+             drives a loading history does;
+  batch      many independent plates advanced together (BatchModel);
+  rve        periodic micro problems relaxed for their homogenised stresses;
+  train      an epoch of the surrogate's training on tensor cores;
+  stress     the surrogate's stresses at the Gauss points of a macro model;
+  macro      steps of an FE^2 macro block with the surrogate as its material.
+
+Inputs come from the seed; sizes are those of the repository's workloads or
+smaller and odd ones of the same kind.
+"""
+import math
+import os
+
+import numpy as np
+import torch
+
+import akantu_b200 as aka
+from akantu_b200 import _abi, fe2
+from akantu_b200.batch import BatchModel
+from akantu_b200.model import material_from_dict, torch_stream
+from akantu_b200.surrogate import MLPSurrogate
+
+WEIGHTS = os.path.join("akantu_b200", "data", "rve_surrogate.npz")
+DEVICE = "cuda:0"
+
+PRECISION = {"reference": aka.MODE_FP64_REFERENCE, "fp64": aka.MODE_FP64,
+             "fp32": aka.MODE_FP32_BULK}
+TYPE = {"seg2": aka.SEGMENT_2, "tri3": aka.TRIANGLE_3, "tet4": aka.TETRAHEDRON_4,
+        "hex8": aka.HEXAHEDRON_8}
+DIM = {"seg2": 1, "tri3": 2, "tet4": 3, "hex8": 3}
+CORNERS = {"seg2": 2, "tri3": 3, "tet4": 4, "hex8": 8}
+POINTS = {"seg2": 1, "tri3": 1, "tet4": 1, "hex8": 8}
+# time step over (smallest edge / wave speed): below the stable step of each type
+COURANT = {"seg2": 0.8, "tri3": 0.4, "tet4": 0.3, "hex8": 0.6}
+# arithmetic operations of one element's force, rounded (gradient, law, force)
+ELEMENT_FLOPS = {"seg2": 12, "tri3": 90, "tet4": 260, "hex8": 3200}
+
+
+# ------------------------------------------------------------------ the cases
+def listed():
+    return [
+        # a small 2D plane-strain plate (8000 elements) driven step by step from a script
+        dict(name="plate_tri3_loop", kind="loop", mesh="tri3", nx=200, ny=20, nz=0,
+             precision="fp64", law="elastic", load=False, distort=False, steps=100),
+        # the default precision of a model: the reference's operation order, an odd box
+        dict(name="box_tet4_reference", kind="explicit", mesh="tet4", nx=37, ny=29, nz=41,
+             precision="reference", law="elastic", load=False, distort=False, steps=100),
+        # a mid-size part under an external load
+        dict(name="box_tet4_load", kind="explicit", mesh="tet4", nx=40, ny=33, nz=27,
+             precision="fp64", law="elastic", load=True, distort=False, steps=200),
+        # the 6 M-element cube: the largest single model
+        dict(name="cube_tet4", kind="explicit", mesh="tet4", nx=100, ny=100, nz=100,
+             precision="fp64", law="elastic", load=False, distort=False, steps=200),
+        # FP32 element arithmetic with FP64 nodal state, ragged sizes
+        dict(name="box_tet4_fp32", kind="explicit", mesh="tet4", nx=61, ny=47, nz=53,
+             precision="fp32", law="elastic", load=False, distort=False, steps=200),
+        # finite-strain neo-Hookean block, 8 Gauss points per element
+        dict(name="block_hex8", kind="explicit", mesh="hex8", nx=64, ny=64, nz=64,
+             precision="fp64", law="neohookean", load=False, distort=False, steps=200),
+        dict(name="block_hex8_fp32", kind="explicit", mesh="hex8", nx=75, ny=75, nz=75,
+             precision="fp32", law="neohookean", load=False, distort=False, steps=200),
+        # hexahedra of a general mesh (no two alike)
+        dict(name="distorted_hex8", kind="explicit", mesh="hex8", nx=37, ny=31, nz=33,
+             precision="fp64", law="neohookean", load=False, distort=True, steps=200),
+        # independent plates of uneven size (a design study), all in one launch per step
+        dict(name="plates_batch", kind="batch", count=512, precision="fp64", steps=250),
+        # labels of the surrogate: the micro problems of sampled gradients
+        dict(name="rve_solve", kind="rve", cells=16, count=1024, precision="fp32"),
+        # the surrogate's training: an epoch of four minibatches
+        dict(name="surrogate_train", kind="train", samples=32768, batch=8192),
+        # FE^2 with the surrogate: 32^3 hexahedra, 262144 Gauss points
+        dict(name="fe2_macro", kind="macro", cells=32, steps=10),
+    ]
+
+
+def _log(rng, lo, hi):
+    return math.exp(rng.uniform(math.log(lo), math.log(hi)))
+
+
+def draw(rng):
+    kind = rng.choices(["explicit", "loop", "batch", "rve", "train", "stress", "macro"],
+                       [9, 2, 2, 1, 1, 1, 1])[0]
+    if kind == "batch":
+        return dict(kind=kind, count=int(_log(rng, 24, 700)), precision=rng.choice(["fp64", "fp32"]),
+                    steps=rng.randint(60, 250))
+    if kind == "rve":
+        return dict(kind=kind, cells=rng.choice([8, 12, 16, 16]), count=int(_log(rng, 5, 1024)),
+                    precision="fp32")
+    if kind == "train":
+        batch = rng.choice([1024, 2048, 4096, 8192, 16384, rng.randint(1000, 9000)])
+        return dict(kind=kind, samples=batch * rng.randint(1, 4) + rng.randint(0, batch - 1),
+                    batch=batch)
+    if kind == "stress":
+        return dict(kind=kind, points=int(_log(rng, 500, 500000)))
+    if kind == "macro":
+        return dict(kind=kind, cells=rng.randint(7, 32), steps=rng.randint(5, 12))
+    mesh = rng.choice(["tri3", "tri3", "tet4", "tet4", "tet4", "hex8", "hex8", "seg2"])
+    precision = rng.choice(["fp64", "fp64", "fp32", "reference"])
+    ne = _log(rng, 300, {"seg2": 20000, "tri3": 500000, "tet4": 1500000, "hex8": 300000}[mesh])
+    if kind == "loop":
+        ne = min(ne, 100000)
+    if mesh == "seg2":
+        nx, ny, nz = int(ne), 0, 0
+    elif mesh == "tri3":
+        ratio = rng.uniform(1.0, 8.0)
+        nx, ny, nz = int(math.sqrt(ne * ratio / 2)), max(2, int(math.sqrt(ne / ratio / 2))), 0
+    else:
+        edge = (ne / (6.0 if mesh == "tet4" else 1.0)) ** (1.0 / 3.0)
+        nx, ny, nz = (max(2, int(edge * rng.uniform(0.75, 1.25))) for _ in range(3))
+    return dict(kind=kind, mesh=mesh, nx=nx, ny=ny, nz=nz, precision=precision,
+                law="neohookean" if mesh == "hex8" and rng.random() < 0.8 else "elastic",
+                load=rng.random() < 0.25, distort=mesh in ("tri3", "hex8") and rng.random() < 0.4,
+                steps=rng.randint(40, 150))
+
+
+# -------------------------------------------------------------------- meshes
+def _grid(nx, ny, nz, dim):
+    """Nodes (x fastest, unit spacing) and the cells' lowest corner ids."""
+    counts = [nx + 1, ny + 1, nz + 1][:dim]
+    axes = np.meshgrid(*[np.arange(c, dtype=np.float64) for c in reversed(counts)], indexing="ij")
+    nodes = np.stack([a.ravel() for a in reversed(axes)], 1)
+    cells = np.meshgrid(*[np.arange(c - 1) for c in reversed(counts)], indexing="ij")
+    stride, base = 1, 0
+    for c, n in zip(reversed(cells), counts):
+        base = base + c.ravel() * stride
+        stride *= n
+    return nodes, base
+
+
+def mesh_of(c, seed):
+    """Nodes, connectivity and the smallest edge of a case's mesh: a bar, plate
+    or box of cells of edge 1 / (largest count), triangles and tetrahedra by
+    cutting cells along their diagonal; `distort` moves the inner nodes."""
+    kind, dim = c["mesh"], DIM[c["mesh"]]
+    nx, ny, nz = c["nx"], c["ny"], c["nz"]
+    nodes, base = _grid(nx, ny, nz, dim)
+    dx, dy, dz = 1, nx + 1, (nx + 1) * (ny + 1)
+    if kind == "seg2":
+        conn = np.stack([base, base + dx], 1)
+    elif kind == "tri3":
+        conn = np.stack([np.stack([base, base + dx, base + dx + dy], 1),
+                         np.stack([base, base + dx + dy, base + dy], 1)], 1).reshape(-1, 3)
+    elif kind == "tet4":
+        top = base + dx + dy + dz
+        tets = []
+        for a, b, even in ((dx, dy, 1), (dx, dz, 0), (dy, dx, 0), (dy, dz, 1), (dz, dx, 1),
+                           (dz, dy, 0)):
+            p, q = base + a, base + a + b
+            tets.append(np.stack([base, p, q, top] if even else [base, q, p, top], 1))
+        conn = np.stack(tets, 1).reshape(-1, 4)
+    else:
+        low = [base, base + dx, base + dx + dy, base + dy]
+        conn = np.stack(low + [b + dz for b in low], 1)
+    if c["distort"]:
+        rng = np.random.default_rng(seed + 77)
+        inner = np.ones(len(nodes), dtype=bool)
+        for k, n in enumerate([nx, ny, nz][:dim]):
+            inner &= (nodes[:, k] > 0) & (nodes[:, k] < n)
+        nodes[inner] += rng.uniform(-0.12, 0.12, (int(inner.sum()), dim))
+    h = 1.0 / max(nx, ny, nz)
+    return nodes * h, conn.astype(np.uint32), h * (0.6 if c["distort"] else 1.0)
+
+
+def inputs_of(c, seed):
+    """Material, time step, boundary and initial conditions of a case."""
+    rng = np.random.default_rng(seed)
+    X, conn, h = mesh_of(c, seed)
+    dim = X.shape[1]
+    if c["law"] == "neohookean":
+        lam, mu, rho = 1.0e6 * rng.uniform(0.8, 1.2), 0.4e6, 1100.0
+        E, nu = mu * (3 * lam + 2 * mu) / (lam + mu), lam / (2 * (lam + mu))
+    else:
+        E, nu, rho = rng.uniform(60e9, 210e9), rng.uniform(0.2, 0.35), rng.uniform(2500.0, 7900.0)
+        if dim == 1:
+            nu = 0.0
+        lam, mu = nu * E / ((1 + nu) * (1 - 2 * nu)), E / (2 * (1 + nu))
+    wave = math.sqrt((lam + 2 * mu) / rho)
+    blocked = np.zeros(X.shape, dtype=np.uint8)
+    blocked[X[:, 0] == 0.0] = 1
+    u0, v0 = np.zeros(X.shape), np.zeros(X.shape)
+    speed = 1e-4 * wave if c["law"] == "elastic" else 2e-2
+    size = X.max(0)
+    for i in range(dim):  # a few smooth modes and, for rubber, nodal noise
+        for mode in range(1, 4):
+            phase = rng.uniform(0, 2 * math.pi, dim)
+            wave_i = np.ones(len(X))
+            for k in range(dim):
+                wave_i *= np.sin(mode * math.pi * X[:, k] / size[k] + phase[k])
+            u0[:, i] += 2e-5 / mode * rng.uniform(0.5, 1.0) * wave_i * X[:, 0]
+            v0[:, i] += speed / mode * rng.uniform(-1.0, 1.0) * wave_i
+    if c["law"] == "neohookean":
+        v0 += rng.normal(0.0, 0.05, X.shape)
+    u0[blocked != 0] = 0.0
+    v0[blocked != 0] = 0.0
+    fext = None
+    if c["load"]:  # a traction on the far face, alike on its nodes
+        fext = np.zeros(X.shape)
+        end = np.nonzero(X[:, 0] == X[:, 0].max())[0]
+        fext[end] = rng.uniform(-1.0, 1.0, dim) * 1e-4 * E * h ** (dim - 1)
+    return dict(X=X, conn=conn, E=E, nu=nu, lam=lam, mu=mu, rho=rho,
+                dt=COURANT[c["mesh"]] * h / wave, blocked=blocked, u0=u0, v0=v0, fext=fext,
+                face=np.nonzero(X[:, 0] == 0.0)[0].astype(np.uint32))
+
+
+def plates_of(c, seed):
+    """Plates of uneven size: element counts log-uniform in [100, 20000]."""
+    rng = np.random.default_rng(seed)
+    plates = []
+    # the sizes belong to the case, the materials and states to the seed
+    sizes = np.random.default_rng(c["count"])
+    for _ in range(c["count"]):
+        ne, ratio = math.exp(sizes.uniform(math.log(100), math.log(20000))), sizes.uniform(1, 8)
+        nx = max(1, round(math.sqrt(ne * ratio / 2)))
+        ny = max(1, round(math.sqrt(ne / (2 * ratio))))
+        X, conn, h = mesh_of(dict(mesh="tri3", nx=nx, ny=ny, nz=0, distort=False), seed)
+        E, nu, rho = rng.uniform(1e9, 200e9), rng.uniform(0.2, 0.4), rng.uniform(1e3, 8e3)
+        lam, mu = nu * E / ((1 + nu) * (1 - 2 * nu)), E / (2 * (1 + nu))
+        blocked = np.zeros(X.shape, dtype=np.uint8)
+        blocked[X[:, 0] == 0.0] = 1
+        length = X[:, 0].max()
+        u0 = np.zeros(X.shape)
+        u0[:, 0] = 1e-4 * length * rng.uniform(0.5, 1.0) * np.sin(math.pi * X[:, 0] / length)
+        u0[blocked != 0] = 0.0
+        plates.append(dict(X=X, conn=conn, E=E, nu=nu, lam=lam, mu=mu, rho=rho, blocked=blocked,
+                           u0=u0, dt=COURANT["tri3"] * h / math.sqrt((lam + 2 * mu) / rho)))
+    return plates
+
+
+# ------------------------------------------------------------------- the calls
+def _model(c, seed):
+    s = inputs_of(c, seed)
+    mesh = aka.Mesh(DIM[c["mesh"]], TYPE[c["mesh"]], s["X"], s["conn"])
+    law = aka.MaterialNeohookean if c["law"] == "neohookean" else aka.MaterialElastic
+    m = aka.SolidMechanicsModel(mesh, [law(rho=s["rho"], E=s["E"], nu=s["nu"])],
+                                precision=PRECISION[c["precision"]])
+    m.initFull(_analysis_method=aka._explicit_lumped_mass)
+    m.setBlockedDOFs(s["blocked"])
+    m.setField(_abi.FIELD_DISPLACEMENT, s["u0"])
+    m.setField(_abi.FIELD_VELOCITY, s["v0"])
+    if s["fext"] is not None:
+        m.setField(_abi.FIELD_EXTERNAL_FORCE, s["fext"])
+    m.setTimeStep(s["dt"])
+    return m, s
+
+
+def _gradients(count, seed):
+    return torch.as_tensor(fe2.sample_gradients(count, seed=seed), device=DEVICE)
+
+
+def _surrogate_samples(count, seed):
+    """Features (H / r, log r) and normalised stresses of a smooth law."""
+    g = torch.Generator(device=DEVICE).manual_seed(seed)
+    H = 0.6 * torch.rand((count, 3, 3), device=DEVICE, dtype=torch.float64, generator=g) - 0.3
+    r = torch.linalg.norm(H.reshape(-1, 9), dim=1)
+    tr = H.diagonal(dim1=1, dim2=2).sum(1)
+    P = 0.4 * (H + H.transpose(1, 2)) + 0.3 * H @ H.transpose(1, 2) + \
+        (tr + tr * tr)[:, None, None] * torch.eye(3, device=DEVICE, dtype=torch.float64)
+    x = torch.cat([H.transpose(1, 2).reshape(-1, 9) / r[:, None], torch.log(r)[:, None]], 1)
+    y = P.transpose(1, 2).reshape(-1, 9) / r[:, None]
+    return x.contiguous(), y.contiguous()
+
+
+def prepare(c, seed):
+    kind = c["kind"]
+    if kind in ("explicit", "loop"):
+        m, s = _model(c, seed)
+        st = dict(kind=kind, model=m, steps=c["steps"])
+        if kind == "loop":
+            st.update(face=s["face"], values=np.zeros(len(s["face"])), dim=DIM[c["mesh"]],
+                      energy=torch.zeros(c["steps"], dtype=torch.float64).pin_memory())
+        return st
+    if kind == "batch":
+        plates = plates_of(c, seed)
+        b = BatchModel([aka.Mesh(2, aka.TRIANGLE_3, p["X"], p["conn"]) for p in plates],
+                       [aka.MaterialElastic(rho=p["rho"], E=p["E"], nu=p["nu"]) for p in plates],
+                       precision=PRECISION[c["precision"]])
+        b.initFull()
+        b.setBlockedDOFs(np.concatenate([p["blocked"] for p in plates]))
+        b.setField(_abi.FIELD_DISPLACEMENT, np.concatenate([p["u0"] for p in plates]))
+        b.setTimeSteps([p["dt"] for p in plates])
+        return dict(kind=kind, model=b, steps=c["steps"])
+    if kind == "rve":
+        rve, _, _ = fe2.spec_rve(c["cells"], precision=PRECISION[c["precision"]])
+        return dict(kind=kind, rve=rve, H=_gradients(c["count"], seed))
+    if kind == "train":
+        net = MLPSurrogate(seed=seed)
+        x, y = _surrogate_samples(c["samples"], seed)
+        net.fit_scaling(x.cpu().numpy(), y.cpu().numpy())
+        return dict(kind=kind, net=net, x=x, y=y, batch=c["batch"])
+    if kind == "stress":
+        net = MLPSurrogate.load(WEIGHTS)
+        H = _gradients(c["points"], seed).transpose(1, 2).reshape(-1, 9).contiguous()
+        n = H.shape[0]
+        return dict(kind=kind, net=net, H=H, P=torch.empty_like(H),
+                    index=torch.empty(n, dtype=torch.int32, device=DEVICE),
+                    count=torch.zeros(1, dtype=torch.int32, device=DEVICE))
+    # macro: the block of fe2.macro_block with a small initial motion
+    rve, mats, vf = fe2.spec_rve(16)
+    provider = fe2.MaterialFE2(rve, MLPSurrogate.load(WEIGHTS))
+    m = fe2.macro_block(provider.material(mats, [1 - vf, vf]), c["cells"])
+    m.setField(_abi.FIELD_VELOCITY, _macro_velocity(c, seed))
+    m.setTimeStep(_macro_dt(c))
+    return dict(kind=kind, model=m, provider=provider, steps=c["steps"], at=0)
+
+
+def run(s):
+    kind = s["kind"]
+    if kind == "explicit":
+        m = s["model"]
+        m.solveSteps(s["steps"])
+        e = [m.getEnergy("kinetic"), m.getEnergy("potential")]
+        return dict(u=m.getDisplacement(), v=m.getVelocity(), energy=np.array(e))
+    if kind == "loop":
+        m, energy = s["model"], s["energy"]
+        at = energy.data_ptr()
+        for k in range(s["steps"]):
+            m.applyDirichlet(s["face"], 0, s["values"])
+            m.solveStep()
+            m.getEnergyAsync("kinetic", at + 8 * k)
+        m.synchronize()
+        return dict(u=m.getDisplacement(), v=m.getVelocity(), energy=energy)
+    if kind == "batch":
+        b = s["model"]
+        b.solveSteps(s["steps"])
+        return dict(u=b.getDisplacement(), v=b.getVelocity(), energy=b.getEnergies("kinetic"))
+    if kind == "rve":
+        out = s["rve"].solve(s["H"])
+        return dict(stress=out["stress"], iterations=out["iterations"], residual=out["residual"])
+    if kind == "train":
+        net = s["net"]
+        losses = net.train(s["x"], s["y"], epochs=1, batch=s["batch"], lr=1e-3, lr_final=1e-5)
+        return dict(losses=np.array(losses), parameters=net.get_parameters())
+    if kind == "stress":
+        s["net"].stress_into(s["H"], s["P"], envelope=(0.3, 0.5), fallback=(s["index"], s["count"]))
+        return dict(P=s["P"], count=s["count"])
+    m = s["model"]
+    for k in range(s["steps"]):
+        s["at"] += 1
+        fe2.macro_step(m, s["at"])
+    return dict(u=m.getDisplacement(), v=m.getVelocity())
+
+
+# ------------------------------------------------------------------- the work
+def _sizes(c):
+    n = CORNERS[c["mesh"]]
+    cells = c["nx"] * max(c["ny"], 1) * max(c["nz"], 1)
+    ne = cells * {"seg2": 1, "tri3": 2, "tet4": 6, "hex8": 1}[c["mesh"]]
+    nn = (c["nx"] + 1) * (c["ny"] + 1 if c["ny"] else 1) * (c["nz"] + 1 if c["nz"] else 1)
+    return ne, nn, n, DIM[c["mesh"]]
+
+
+def work(c):
+    """Per step: the connectivity, X, u, v, a (read and written), 1 / M and the
+    blocked flags; per output: u and v (and X and the connectivity once more
+    for the potential energy). An RVE iteration has no bytes of its own."""
+    kind = c["kind"]
+    if kind in ("explicit", "loop"):
+        ne, nn, n, d = _sizes(c)
+        step = ne * n * 4 + nn * (d * 8 * 7 + 8 + d)
+        return dict(bytes=c["steps"] * step + nn * d * 8 * 4 + ne * n * 4,
+                    flops=c["steps"] * (ne * ELEMENT_FLOPS[c["mesh"]] + nn * d * 12))
+    if kind == "batch":
+        sizes = np.random.default_rng(c["count"])
+        ne = nn = 0
+        for _ in range(c["count"]):
+            e, ratio = math.exp(sizes.uniform(math.log(100), math.log(20000))), sizes.uniform(1, 8)
+            nx = max(1, round(math.sqrt(e * ratio / 2)))
+            ny = max(1, round(math.sqrt(e / (2 * ratio))))
+            ne += 2 * nx * ny
+            nn += (nx + 1) * (ny + 1)
+        return dict(bytes=c["steps"] * (ne * 12 + nn * (2 * 8 * 7 + 10)) + nn * 64,
+                    flops=c["steps"] * (ne * ELEMENT_FLOPS["tri3"] + nn * 24))
+    if kind == "rve":  # about 260 updates of 8 Gauss points of 250 operations per voxel
+        return dict(bytes=c["count"] * 9 * 8 * 2, flops=c["count"] * c["cells"] ** 3 * 260 * 2000)
+    flop = 2 * (10 * 256 + 2 * 256 * 256 + 256 * 9)
+    if kind == "train":
+        n = c["batch"] * max(1, c["samples"] // c["batch"])
+        return dict(bytes=n * 19 * 8 + (n // c["batch"]) * 136713 * 4 * 7, flops=3.0 * n * flop)
+    if kind == "stress":
+        return dict(bytes=c["points"] * 18 * 8, flops=c["points"] * flop)
+    ne, nn = c["cells"] ** 3, (c["cells"] + 1) ** 3
+    return dict(bytes=c["steps"] * (ne * (32 + 8 * 9 * 8 * 2) + nn * 3 * 8 * 7) + nn * 48,
+                flops=c["steps"] * ne * 8 * (flop + 400))
+
+
+# ----------------------------------------------------- the same in plain torch
+def _t(a, dtype=torch.float64):
+    return torch.as_tensor(np.ascontiguousarray(a), device=DEVICE).to(dtype)
+
+
+def _points(mesh):
+    """Shape functions N (q, n), their natural derivatives (q, n, d), weights."""
+    if mesh == "seg2":
+        return [[0.5, 0.5]], [[[-0.5], [0.5]]], [2.0]
+    if mesh == "tri3":
+        return [[1 / 3] * 3], [[[-1, -1], [1, 0], [0, 1]]], [0.5]
+    if mesh == "tet4":
+        return [[0.25] * 4], [[[-1, -1, -1], [1, 0, 0], [0, 1, 0], [0, 0, 1]]], [1 / 6]
+    corner = np.array([[-1, -1, -1], [1, -1, -1], [1, 1, -1], [-1, 1, -1],
+                       [-1, -1, 1], [1, -1, 1], [1, 1, 1], [-1, 1, 1]], dtype=float)
+    N, dN = [], []
+    for q in range(8):
+        xi = np.array([1 if q >> k & 1 else -1 for k in range(3)]) / math.sqrt(3)
+        f = 1 + corner * xi
+        N.append(f.prod(1) / 8)
+        dN.append(np.stack([corner[:, k] * f[:, (k + 1) % 3] * f[:, (k + 2) % 3] / 8
+                            for k in range(3)], 1))
+    return N, dN, [1.0] * 8
+
+
+class _Body:
+    """Shape gradients, volumes and the lumped mass of a mesh, in chunks of elements."""
+
+    def __init__(self, mesh, X, conn, rho, chunk=1 << 20):
+        N, dN, w = (_t(a) for a in _points(mesh))
+        self.X, self.conn, self.chunk = _t(X), _t(conn.astype(np.int64), torch.int64), chunk
+        self.dN, self.w, self.dim = dN, w, X.shape[1]
+        self.mass = torch.zeros(len(X), dtype=torch.float64, device=DEVICE)
+        for cn in self.conn.split(chunk):
+            det = self.geometry(cn)[1]
+            self.mass.index_add_(0, cn.reshape(-1), (rho * det @ N).reshape(-1))
+
+    def geometry(self, cn):
+        J = torch.einsum("qak,eaj->eqkj", self.dN, self.X[cn])
+        return torch.einsum("eqjk,qak->eqaj", torch.linalg.inv(J), self.dN), \
+            torch.linalg.det(J) * self.w
+
+    def forces(self, u, law):
+        f = torch.zeros_like(u)
+        energy = 0.0
+        for k, cn in enumerate(self.conn.split(self.chunk)):
+            B, wd = self.geometry(cn) if len(self.conn) > self.chunk else self._kept(cn)
+            P, W = law(torch.einsum("eai,eqaj->eqij", u[cn], B), slice(k * self.chunk, None))
+            fe = -torch.einsum("eqij,eqaj,eq->eai", P, B, wd)
+            f.index_add_(0, cn.reshape(-1), fe.reshape(-1, self.dim))
+            energy += float((W * wd).sum()) if W is not None else 0.0
+        return f, energy
+
+    def _kept(self, cn):
+        if not hasattr(self, "_g"):
+            self._g = self.geometry(cn)
+        return self._g
+
+
+def _law(s, finite):
+    lam, mu, E = s["lam"], s["mu"], s["E"]
+
+    def per(v, at, nd):  # a scalar, or a value per element
+        return v if not torch.is_tensor(v) else v[at].reshape((-1,) + (1,) * (nd - 1))
+
+    def stress(g, at):
+        d = g.shape[-1]
+        one = torch.eye(d, dtype=torch.float64, device=DEVICE)
+        if finite:
+            F = g + one
+            Fi = torch.linalg.inv(F).transpose(-1, -2)
+            lj = torch.log(torch.linalg.det(F))[..., None, None]
+            P = mu * (F - Fi) + lam * lj * Fi
+            lj = lj[..., 0, 0]
+            return P, 0.5 * lam * lj * lj - mu * lj + \
+                0.5 * mu * ((F * F).sum((-1, -2)) - 3.0)
+        if d == 1:
+            P = E * g
+        else:
+            l, m = per(lam, at, g.dim()), per(mu, at, g.dim())
+            tr = g.diagonal(dim1=-1, dim2=-2).sum(-1)[..., None, None]
+            P = l * tr * one + m * (g + g.transpose(-1, -2))
+        return P, 0.5 * (P * g).sum((-1, -2))
+    return stress
+
+
+def _advance(forces, mass, blocked, dt, u, v, steps, fext=None, each=None, before=None):
+    """Central differences with a lumped mass; the acceleration starts at zero.
+    dt: a number or a column per node."""
+    a = torch.zeros_like(u)
+    free = (blocked == 0).to(torch.float64)
+    for k in range(steps):
+        if before is not None:
+            before(k, u)
+        u += free * (dt * v + 0.5 * dt * dt * a)
+        v += free * dt * a
+        f = forces(u)
+        if fext is not None:
+            f = f + fext
+        new = f / mass[:, None]
+        v += free * 0.5 * dt * (new - a)
+        a = torch.where(free > 0, new, a)
+        if each is not None:
+            each(k, u, v)
+    return u, v
+
+
+def _kinetic(mass, v):
+    return float(0.5 * (mass[:, None] * v * v).sum())
+
+
+def exact(c, seed):
+    if not torch.cuda.is_available():
+        return None
+    kind = c["kind"]
+    if kind in ("explicit", "loop"):
+        s = inputs_of(c, seed)
+        body = _Body(c["mesh"], s["X"], s["conn"], s["rho"])
+        law = _law(s, c["law"] == "neohookean")
+        u, v = _t(s["u0"]), _t(s["v0"])
+        energy = []
+        each = None if kind == "explicit" else lambda k, u, v: energy.append(_kinetic(body.mass, v))
+        u, v = _advance(lambda x: body.forces(x, law)[0], body.mass, _t(s["blocked"]), s["dt"], u, v,
+                        c["steps"], None if s["fext"] is None else _t(s["fext"]), each)
+        if kind == "explicit":
+            energy = [_kinetic(body.mass, v), body.forces(u, law)[1]]
+        return dict(u=u, v=v, energy=np.array(energy))
+    if kind == "batch":
+        plates = plates_of(c, seed)
+        off = np.cumsum([0] + [len(p["X"]) for p in plates])
+        conn = np.concatenate([p["conn"].astype(np.int64) + o for p, o in zip(plates, off)])
+        el = [len(p["conn"]) for p in plates]
+        nodes = [len(p["X"]) for p in plates]
+        s = {k: _t(np.repeat([p[k] for p in plates], el)) for k in ("lam", "mu", "E")}
+        body = _Body("tri3", np.concatenate([p["X"] for p in plates]), conn, 1.0, chunk=1 << 23)
+        # one density per plate scales that plate's mass
+        mass = body.mass * _t(np.repeat([p["rho"] for p in plates], nodes))
+        dt = _t(np.repeat([p["dt"] for p in plates], nodes))[:, None]
+        u = _t(np.concatenate([p["u0"] for p in plates]))
+        law = _law(s, False)
+        u, v = _advance(lambda x: body.forces(x, law)[0], mass,
+                        _t(np.concatenate([p["blocked"] for p in plates])), dt, u,
+                        torch.zeros_like(u), c["steps"])
+        per = torch.zeros(len(plates), dtype=torch.float64, device=DEVICE)
+        per.index_add_(0, _t(np.repeat(np.arange(len(plates)), nodes), torch.int64),
+                       0.5 * (mass[:, None] * v * v).sum(1))
+        return dict(u=u, v=v, energy=per)
+    if kind == "rve":
+        return dict(stress=_relaxed(c, seed), iterations=None, residual=None)
+    if kind == "train":
+        return _trained(c, seed)
+    if kind == "stress":
+        H = _gradients(c["points"], seed).transpose(1, 2).reshape(-1, 9)
+        return dict(P=_network_stress(_weights(), H), count=None)
+    n = c["cells"]
+    X, conn, _ = mesh_of(dict(mesh="hex8", nx=n, ny=n, nz=n, distort=False), 0)
+    body = _Body("hex8", X, conn, 1100.0)
+    blocked = np.zeros(X.shape)
+    blocked[X[:, 0] == 0] = 1
+    right = X[:, 0] > 1 - 0.5 / n
+    blocked[right, 0] = 1
+    right = _t(right, torch.bool)
+    net = _weights()
+
+    def law(g, at):
+        P = _network_stress(net, g.transpose(-1, -2).reshape(-1, 9))
+        return P.reshape(g.shape).transpose(-1, -2), None
+
+    def pull(k, u):
+        u[right, 0] = 0.05 * min((k + 1) / 200, 1.0)
+    u, v = _advance(lambda x: body.forces(x, law)[0], body.mass, _t(blocked), _macro_dt(c), _t(0 * X),
+                    _t(_macro_velocity(c, seed)), c["steps"], before=pull)
+    return dict(u=u, v=v)
+
+
+def _macro_dt(c):
+    """Half of edge / wave speed of the mixture's upper-bound moduli (20 % of
+    an inclusion 10 times stiffer: 2.8 times the matrix's moduli)."""
+    return 0.5 / c["cells"] / math.sqrt(2.8 * 1.8e6 / 1100.0)
+
+
+def _macro_velocity(c, seed):
+    n = c["cells"]
+    X = _grid(n, n, n, 3)[0] / n
+    rng = np.random.default_rng(seed)
+    v = np.zeros(X.shape)
+    for i in range(3):
+        p = rng.uniform(0.5, 1.5, 3)
+        v[:, i] = rng.uniform(0.2, 1.0) * np.sin(p[0] * math.pi * X[:, 0]) * \
+            np.cos(p[1] * math.pi * X[:, 1]) * np.cos(p[2] * math.pi * X[:, 2])
+    v[X[:, 0] == 0] = 0.0
+    v[X[:, 0] == 1, 0] = 0.0
+    return v
+
+
+def _weights():
+    d = np.load(WEIGHTS)
+    return _unpack(_t(d["params"]), [int(k) for k in d["shape"]]) + \
+        ({k: _t(d[k]) for k in ("in_shift", "in_scale", "out_shift", "out_scale")},)
+
+
+def _unpack(p, shape):
+    nin, nout, w, nh = shape
+    out, at = [], 0
+    for l in range(nh + 1):
+        k, n = (w if l else nin), (nout if l == nh else w)
+        out += [(p[at:at + n * k].reshape(n, k), p[at + n * k:at + n * k + n])]
+        at += n * k + n
+    return (out,)
+
+
+def _forward(layers, x):
+    for l, (W, b) in enumerate(layers):
+        x = x @ W.T + b
+        if l + 1 < len(layers):
+            x = x * torch.sigmoid(x)
+    return x
+
+
+def _network_stress(net, H):
+    layers, s = net
+    out = []
+    for h in H.split(65536):
+        r = torch.linalg.norm(h, dim=1, keepdim=True)
+        rr = r.clamp_min(1e-8)
+        x = (torch.cat([h / rr, torch.log(rr)], 1) - s["in_shift"]) * s["in_scale"]
+        out.append(r * (_forward(layers, x) * s["out_scale"] + s["out_shift"]))
+    return torch.cat(out)
+
+
+def _trained(c, seed):
+    """The epoch in 64 bits: the same minibatches, Adam."""
+    x, y = _surrogate_samples(c["samples"], seed)
+    xn = (x - _t(x.cpu().numpy().mean(0))) / _t(x.cpu().numpy().std(0))
+    yn = (y - _t(y.cpu().numpy().mean(0))) / _t(y.cpu().numpy().std(0))
+    rng = np.random.default_rng(seed)
+    parts = []
+    for k, n in [(10, 256), (256, 256), (256, 256), (256, 9)]:
+        a = np.sqrt(6.0 / (k + n))
+        parts += [rng.uniform(-a, a, n * k), np.zeros(n)]
+    p = _t(np.concatenate(parts).astype(np.float32))
+    m1, m2 = torch.zeros_like(p), torch.zeros_like(p)
+    batch, n = c["batch"], c["samples"]
+    g = torch.Generator(device=DEVICE).manual_seed(0)
+    perm = torch.randperm(n, device=DEVICE, generator=g)
+    steps = max(1, n // batch)
+    losses = []
+    for k in range(steps):
+        idx = perm[k * batch:(k + 1) * batch]
+        q = p.clone().requires_grad_(True)
+        loss = ((_forward(_unpack(q, [10, 9, 256, 3])[0], xn[idx]) - yn[idx]) ** 2).mean()
+        loss.backward()
+        losses.append(float(loss))
+        m1 = 0.9 * m1 + 0.1 * q.grad
+        m2 = 0.999 * m2 + 0.001 * q.grad ** 2
+        lr = 1e-5 + 0.5 * (1e-3 - 1e-5) * (1 + math.cos(math.pi * k / steps))
+        p = p - lr * (m1 / (1 - 0.9 ** (k + 1))) / ((m2 / (1 - 0.999 ** (k + 1))).sqrt() + 1e-8)
+    return dict(losses=np.array([sum(losses) / steps]), parameters=p)
+
+
+def _relaxed(c, seed, chunk=256):
+    """Homogenised stresses of the periodic cube with a centred sphere (a
+    fifth of the volume, 10 times stiffer) at equilibrium: damped leapfrog on
+    the fluctuation with a step well below the stable one."""
+    n = c["cells"]
+    H = _gradients(c["count"], seed)
+    h = 1.0 / n
+    x = (np.arange(n) + 0.5) * h - 0.5
+    z, y, xx = np.meshgrid(x, x, x, indexing="ij")
+    stiff = np.where(xx * xx + y * y + z * z <= (0.2 * 3 / (4 * math.pi)) ** (2 / 3), 10.0, 1.0)
+    stiff = _t(stiff)  # (z, y, x)
+    lam, mu = (1.0e6 * stiff)[None], (0.4e6 * stiff)[None]
+    _, dN, _ = _points("hex8")
+    B = _t(np.array(dN)) * 2.0 / h  # (q, a, j)
+    corner = [(0, 0, 0), (1, 0, 0), (1, 1, 0), (0, 1, 0), (0, 0, 1), (1, 0, 1), (1, 1, 1), (0, 1, 1)]
+    mass = sum(torch.roll(stiff, (o[2], o[1], o[0]), (0, 1, 2)) for o in corner) * 1.8e6 * h ** 3 / 8
+    Bm = B.permute(1, 0, 2).reshape(8, 24)
+
+    def force(w, g0):
+        uc = torch.stack([torch.roll(w, (-o[2], -o[1], -o[0]), (2, 3, 4)) for o in corner], -1)
+        g = (uc @ Bm).reshape(uc.shape[:-1] + (8, 3))  # (b, i, z, y, x, q, j)
+        F = [[g[:, i, ..., j] + g0[:, i, j, None, None, None, None] for j in range(3)]
+             for i in range(3)]
+        cof = [[F[(i + 1) % 3][(j + 1) % 3] * F[(i + 2) % 3][(j + 2) % 3] -
+                F[(i + 1) % 3][(j + 2) % 3] * F[(i + 2) % 3][(j + 1) % 3] for j in range(3)]
+               for i in range(3)]
+        J = F[0][0] * cof[0][0] + F[0][1] * cof[0][1] + F[0][2] * cof[0][2]
+        t = (lam[..., None] * torch.log(J) - mu[..., None]) / J
+        P = torch.stack([torch.stack([mu[..., None] * F[i][j] + t * cof[i][j] for j in range(3)], -1)
+                         for i in range(3)], 1) * (h ** 3 / 8)  # (b, i, z, y, x, q, j)
+        fc = P.reshape(P.shape[:-2] + (24,)) @ Bm.T
+        f = sum(torch.roll(fc[..., a], (o[2], o[1], o[0]), (2, 3, 4)) for a, o in enumerate(corner))
+        return -f, P.sum((2, 3, 4, 5))
+    out = []
+    for Hc in H.split(chunk):
+        b = Hc.shape[0]
+        F = Hc + torch.eye(3, device=DEVICE, dtype=torch.float64)
+        smin = torch.linalg.svdvals(F)[:, -1]
+        press = (-torch.log(torch.linalg.det(F))).clamp_min(0.0)
+        dt = (0.25 * h * smin / torch.sqrt(1 + 2 * press * 1.0e6 / 1.8e6)).reshape(-1, 1, 1, 1, 1)
+        damp = 0.6 * 4 * math.pi * math.sqrt(0.4 / 1.8)
+        w = torch.zeros((b, 3, n, n, n), device=DEVICE, dtype=torch.float64)
+        v = torch.zeros_like(w)
+        for _ in range(600):
+            f, _p = force(w, F)
+            v = ((1 - 0.5 * damp * dt) * v + dt * f / mass) / (1 + 0.5 * damp * dt)
+            w = w + dt * v
+        out.append(force(w, F)[1])
+    return torch.cat(out)
