@@ -75,7 +75,7 @@ def listed():
         # independent plates of uneven size (a design study), all in one launch per step
         dict(name="plates_batch", kind="batch", count=512, precision="fp64", steps=250),
         # labels of the surrogate: the micro problems of sampled gradients
-        dict(name="rve_solve", kind="rve", cells=16, count=1024, precision="fp32"),
+        dict(name="rve_solve", kind="rve", cells=16, count=512, precision="fp32"),
         # the surrogate's training: an epoch of four minibatches
         dict(name="surrogate_train", kind="train", samples=32768, batch=8192),
         # FE^2 with the surrogate: 32^3 hexahedra, 262144 Gauss points
@@ -94,7 +94,7 @@ def draw(rng):
         return dict(kind=kind, count=int(_log(rng, 24, 700)), precision=rng.choice(["fp64", "fp32"]),
                     steps=rng.randint(60, 250))
     if kind == "rve":
-        return dict(kind=kind, cells=rng.choice([8, 12, 16, 16]), count=int(_log(rng, 5, 1024)),
+        return dict(kind=kind, cells=rng.choice([8, 12, 16, 16]), count=int(_log(rng, 5, 512)),
                     precision="fp32")
     if kind == "train":
         batch = rng.choice([1024, 2048, 4096, 8192, 16384, rng.randint(1000, 9000)])
@@ -656,7 +656,7 @@ def _trained(c, seed):
 def _relaxed(c, seed, chunk=256):
     """Homogenised stresses of the periodic cube with a centred sphere (a
     fifth of the volume, 10 times stiffer) at equilibrium: damped leapfrog on
-    the fluctuation with a step well below the stable one."""
+    the fluctuation."""
     n = c["cells"]
     H = _gradients(c["count"], seed)
     h = 1.0 / n
@@ -686,19 +686,27 @@ def _relaxed(c, seed, chunk=256):
         fc = P.reshape(P.shape[:-2] + (24,)) @ Bm.T
         f = sum(torch.roll(fc[..., a], (o[2], o[1], o[0]), (2, 3, 4)) for a, o in enumerate(corner))
         return -f, P.sum((2, 3, 4, 5))
-    out = []
-    for Hc in H.split(chunk):
-        b = Hc.shape[0]
-        F = Hc + torch.eye(3, device=DEVICE, dtype=torch.float64)
-        smin = torch.linalg.svdvals(F)[:, -1]
-        press = (-torch.log(torch.linalg.det(F))).clamp_min(0.0)
-        dt = (0.25 * h * smin / torch.sqrt(1 + 2 * press * 1.0e6 / 1.8e6)).reshape(-1, 1, 1, 1, 1)
-        damp = 0.6 * 4 * math.pi * math.sqrt(0.4 / 1.8)
-        w = torch.zeros((b, 3, n, n, n), device=DEVICE, dtype=torch.float64)
-        v = torch.zeros_like(w)
-        for _ in range(600):
-            f, _p = force(w, F)
-            v = ((1 - 0.5 * damp * dt) * v + dt * f / mass) / (1 + 0.5 * damp * dt)
-            w = w + dt * v
-        out.append(force(w, F)[1])
-    return torch.cat(out)
+    damp = 0.6 * 4 * math.pi * math.sqrt(0.4 / 1.8)
+    F = H + torch.eye(3, device=DEVICE, dtype=torch.float64)
+    press = (-torch.log(torch.linalg.det(F))).clamp_min(0.0)
+    step = h * torch.linalg.svdvals(F)[:, -1] / torch.sqrt(1 + 2 * press * 1.0e6 / 1.8e6)
+    P = torch.empty_like(H)
+    left = torch.arange(len(H), device=DEVICE)
+    # a smaller step for the few whose strain concentrates until the first one is unstable
+    for factor, count in ((0.3, 500), (0.15, 1000), (0.07, 2000)):
+        again = []
+        for at in left.split(chunk):
+            dt = (factor * step[at]).reshape(-1, 1, 1, 1, 1)
+            w = torch.zeros((len(at), 3, n, n, n), device=DEVICE, dtype=torch.float64)
+            v = torch.zeros_like(w)
+            for _ in range(count):
+                v = ((1 - 0.5 * damp * dt) * v + dt * force(w, F[at])[0] / mass) / \
+                    (1 + 0.5 * damp * dt)
+                w = w + dt * v
+            f, P[at] = force(w, F[at])
+            f = f.flatten(1).abs().max(1)[0]
+            again.append(at[~(f <= 1e-3 * h * h * 4.0e6 * H[at].flatten(1).abs().max(1)[0])])
+        left = torch.cat(again)
+        if not len(left):
+            break
+    return P
