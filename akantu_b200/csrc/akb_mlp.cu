@@ -29,6 +29,7 @@
 // tensor memory and returns.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <memory>
 #include <vector>
@@ -588,19 +589,89 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   if (warp == 0) tmem_free(tmem, 256);
 }
 
-// Partial weight gradients G[m][n] = sum_s A[s][m] B[s][n] over the tiles
-// [tile0, tile1) of this CTA: A tiles with ca columns (128 or 256), B tiles
-// with cb columns (16..256); written to part[blockIdx.x][ca][cb].
+// Weight and bias gradients of every layer, in one launch: blockIdx.y is the
+// layer; its first nbias CTAs sum columns of dZ (the bias gradient), the
+// others take ranges of tiles and write the partials
+// G[m][n] = sum_s A[s][m] B[s][n] (A tiles with ca columns, 128 or 256, B
+// tiles with cb columns, 16..256; the output layer as its transpose, since M
+// must be 128 or 256).
+//
+// The bias sums keep one serial chain per column over the samples, in sample
+// order: a chain of nb dependent FP32 additions (4 cycles each: 17 us at 8192
+// samples) bounds them, so they start first and run beside the partials,
+// whose bound is the loads of their tiles. As a kernel of its own, with a
+// thread per column loading from global memory, the sums took 283 us a layer
+// at 8192 samples, 1.13 of the 1.43 ms of a training step's kernels.
+struct GradArgs {
+  const unsigned char *A[kMaxLayers], *B[kMaxLayers];
+  float* part[kMaxLayers];
+  int ca[kMaxLayers], cb[kMaxLayers];
+  int dz_is_b[kMaxLayers];
+  int rows[kMaxLayers];      // real biases of the layer
+  float* bias[kMaxLayers];   // their gradients
+};
+
+constexpr int kBiasCols = 64;    // columns of a bias CTA: two warps of chains
+constexpr int kBiasStages = 4;   // tiles in flight
+constexpr int kBiasRow = kBiasCols * 2 + 16;  // bytes of a staged row: padded, 16-byte aligned
+
+// Column sums of dZ over all tiles, columns [c0, c0 + 64): the tiles' columns
+// are copied to shared memory row by row (cp.async, four tiles ahead), where
+// the 32 lanes of a warp read 64 consecutive bytes; thread n < 64 adds column
+// c0 + n.
+__device__ inline void bias_columns(const unsigned char* dz, int cols, int real, int c0,
+                                    int64_t ntiles, unsigned char* smem, float* grad) {
+  const int tid = threadIdx.x;
+  const int groups = min(kBiasCols, cols - c0) >> 3;  // core matrices in a row
+  auto fetch = [&](int64_t t) {
+    if (t < ntiles) {
+      const unsigned char* src = dz + t * (size_t)kTile * cols * 2;
+      unsigned char* dst = smem + (t % kBiasStages) * (size_t)(kTile * kBiasRow);
+      for (int k = tid; k < kTile * groups; k += kThreads) {  // 8 rows of a core matrix together
+        const int r = (k / (8 * groups)) * 8 + (k & 7), g = (k >> 3) % groups;
+        const uint32_t d = saddr(dst + r * kBiasRow + g * 16);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d),
+                     "l"(src + pk_off(r, c0 + 8 * g, cols))
+                     : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int t = 0; t < kBiasStages - 1; ++t) fetch(t);
+  float acc = 0.0f;
+  for (int64_t t = 0; t < ntiles; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kBiasStages - 2) : "memory");
+    __syncthreads();  // tile t has landed; the stage of tile t - 1 is free
+    fetch(t + kBiasStages - 1);
+    if (tid < 8 * groups) {
+      const unsigned char* col = smem + (t % kBiasStages) * (size_t)(kTile * kBiasRow) + tid * 2;
+#pragma unroll 32
+      for (int r = 0; r < kTile; ++r)
+        acc += __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(col + r * kBiasRow) << 16);
+    }
+  }
+  if (tid < 8 * groups && c0 + tid < real) grad[c0 + tid] = acc;
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
-    k_wgrad(const unsigned char* __restrict__ A, int ca, const unsigned char* __restrict__ B,
-            int cb, int64_t ntiles, int tiles_per_cta, float* part, int* error) {
+    k_wgrad(GradArgs g, int nbias, int64_t ntiles, int tiles_per_cta, int* error) {
   extern __shared__ __align__(1024) unsigned char smem[];
+  if ((int)blockIdx.x < nbias) {
+    const int b = blockIdx.y, c0 = (int)blockIdx.x * kBiasCols;
+    const int cols = g.dz_is_b[b] ? g.cb[b] : g.ca[b];
+    if (c0 < cols)
+      bias_columns(g.dz_is_b[b] ? g.B[b] : g.A[b], cols, g.rows[b], c0, ntiles, smem, g.bias[b]);
+    return;
+  }
+  const int block = (int)blockIdx.x - nbias;
   unsigned char* sa = smem;
   unsigned char* sb = smem + (size_t)kTile * kMaxWidth * 2;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sb + (size_t)kTile * kMaxWidth * 2);
   uint32_t* holder = reinterpret_cast<uint32_t*>(mbar + 2);
   const uint32_t mb_mma = saddr(mbar), mb_t = saddr(mbar + 1);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, l = blockIdx.y;
+  const unsigned char *A = g.A[l], *B = g.B[l];
+  const int ca = g.ca[l], cb = g.cb[l];
   if (warp == 0) tmem_alloc(saddr(holder), 512);
   if (tid == 0) {
     mbar_init(mb_mma);
@@ -610,7 +681,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   fence_after();
   const uint32_t tmem = *holder;
-  const int64_t t0 = (int64_t)blockIdx.x * tiles_per_cta;
+  const int64_t t0 = (int64_t)block * tiles_per_cta;
   const int64_t t1 = t0 + tiles_per_cta < ntiles ? t0 + tiles_per_cta : ntiles;
   const int halves = ca / kTile;
   const uint32_t id = idesc(kTile, cb, true, true);
@@ -623,29 +694,33 @@ __global__ void __launch_bounds__(kThreads, 1)
                  B + t * (size_t)kTile * cb * 2, (uint32_t)(kTile * cb * 2), mb_t);
     t_pending = true;
     ok = mbar_wait(mb_t, pt);
-    if (!ok) break;
-    pt ^= 1;
-    t_pending = false;
-    if (tid == 0) {
-      fence_after();
-      for (int h = 0; h < halves; ++h)
-        for (int s = 0; s < kTile / 16; ++s)
-          mma(tmem + h * cb,
-              sdesc(saddr(sa) + h * (kTile / 8) * 128 + s * 2 * 16 * ca, 16 * ca, 128),
-              sdesc(saddr(sb) + s * 2 * 16 * cb, 16 * cb, 128), id, (t > t0 || s > 0) ? 1u : 0u);
-      mma_commit(mb_mma);
+    if (ok) {
+      pt ^= 1;
+      t_pending = false;
+      if (tid == 0) {
+        fence_after();
+        for (int h = 0; h < halves; ++h)
+          for (int s = 0; s < kTile / 16; ++s)
+            mma(tmem + h * cb,
+                sdesc(saddr(sa) + h * (kTile / 8) * 128 + s * 2 * 16 * ca, 16 * ca, 128),
+                sdesc(saddr(sb) + s * 2 * 16 * cb, 16 * cb, 128), id, (t > t0 || s > 0) ? 1u : 0u);
+        mma_commit(mb_mma);
+      }
+      m_pending = true;
+      ok = mbar_wait(mb_mma, pm);
+      if (ok) {
+        pm ^= 1;
+        m_pending = false;
+        fence_after();
+      }
     }
-    m_pending = true;
-    ok = mbar_wait(mb_mma, pm);
-    if (!ok) break;
-    pm ^= 1;
-    m_pending = false;
-    fence_after();
-    __syncthreads();  // shared tiles free for the next copy
+    // shared tiles free for the next copy; a wait that gave up in one thread
+    // ends the loop in all
+    if (__syncthreads_or(!ok)) ok = false;
   }
-  if (ok && t1 > t0) {
+  if (ok) {
+    float* out = g.part[l] + (size_t)block * ca * cb;
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    float* out = part + (size_t)blockIdx.x * ca * cb;
     for (int h = 0; h < halves; ++h)
       for (int c0 = 0; c0 < cb; c0 += 16) {
         float v[16];
@@ -656,9 +731,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int q = 0; q < 4; ++q)
           o4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
       }
-  } else if (t1 <= t0) {
-    float* out = part + (size_t)blockIdx.x * ca * cb;
-    for (int k = tid; k < ca * cb; k += kThreads) out[k] = 0.0f;
   }
   if (!ok) {  // drain what is still in flight before leaving (bounded)
     if (t_pending) mbar_wait(mb_t, pt);
@@ -670,44 +742,55 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) tmem_free(tmem, 512);
 }
 
-// grad[m][n] (real rows/cols, row stride ncols) = sum over CTAs of the
-// partials, in CTA order; TRANSPOSE reads part[.][n][m].
-__global__ void k_sum_partials(const float* part, int nparts, int ca, int cb, int rows, int cols,
-                               bool transpose, float* grad) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= rows * cols) return;
-  const int m = k / cols, n = k % cols;
-  const size_t idx = transpose ? (size_t)n * cb + m : (size_t)m * cb + n;
+// Where each layer's weights (N x K row-major) and biases sit in the flat
+// parameter array.
+struct Layout {
+  int64_t w_off[kMaxLayers], b_off[kMaxLayers];
+};
+
+// The weight gradients from the partials, summed in CTA order; blockIdx.y is
+// the layer, one thread per entry of a partial (the output layer's hold the
+// transpose).
+__global__ void k_sum_partials(Net net, GradArgs g, int nparts, Layout lay, float* grad) {
+  const int l = blockIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int ca = g.ca[l], cb = g.cb[l];
+  if (k >= ca * cb) return;
+  const int a = k / cb, b = k % cb;
+  const int m = g.dz_is_b[l] ? b : a, n = g.dz_is_b[l] ? a : b;
+  if (m >= net.Nr[l] || n >= net.Kr[l]) return;
   float acc = 0.0f;
-  for (int p = 0; p < nparts; ++p) acc += part[(size_t)p * ca * cb + idx];
-  grad[k] = acc;
+  const float* part = g.part[l] + k;
+#pragma unroll 8
+  for (int p = 0; p < nparts; ++p) acc += part[(size_t)p * ca * cb];
+  grad[lay.w_off[l] + (int64_t)m * net.Kr[l] + n] = acc;
 }
 
-// Bias gradient of a layer: sum over samples of the packed BF16 dZ tiles.
-__global__ void k_bias_grad(const unsigned char* dz, int cols, int real, int64_t ntiles,
-                            float* grad) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= real) return;
-  float acc = 0.0f;
-  for (int64_t t = 0; t < ntiles; ++t) {
-    const unsigned char* tile = dz + t * (size_t)kTile * cols * 2;
-    for (int r = 0; r < kTile; ++r)
-      acc += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(tile + pk_off(r, n, cols)));
-  }
-  grad[n] = acc;
-}
-
-// Adam (Kingma & Ba 2015) on the FP32 master parameters.
-__global__ void k_adam(float* p, const float* g, float* m1, float* m2, int64_t n, float lr,
-                       float b1, float b2, float eps, float c1, float c2) {
-  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k >= n) return;
+// Adam (Kingma & Ba 2015) on the FP32 master parameters, and the BF16 copies
+// of the updated weights (the padding of W, Wt and b is written once, by
+// k_pack, and stays); blockIdx.y is the layer, one thread per parameter.
+__global__ void k_adam(Net net, Layout lay, float* p, const float* g, float* m1, float* m2,
+                       float lr, float b1, float b2, float eps, float c1, float c2) {
+  const int l = blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nw = net.Nr[l] * net.Kr[l];
+  if (t >= nw + net.Nr[l]) return;
+  const int64_t k = t < nw ? lay.w_off[l] + t : lay.b_off[l] + (t - nw);
   const float gk = g[k];
   const float a = b1 * m1[k] + (1.0f - b1) * gk;
   const float b = b2 * m2[k] + (1.0f - b2) * gk * gk;
   m1[k] = a;
   m2[k] = b;
-  p[k] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+  const float x = p[k] - lr * (a / c1) / (sqrtf(b / c2) + eps);
+  p[k] = x;
+  if (t >= nw) {
+    const_cast<float*>(net.b[l])[t - nw] = x;
+    return;
+  }
+  const int r = t / net.Kr[l], c = t % net.Kr[l];
+  const __nv_bfloat16 h = __float2bfloat16_rn(x);
+  *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(const_cast<__nv_bfloat16*>(net.W[l])) +
+                                    pk_off(r, c, net.K[l])) = h;
+  *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(const_cast<__nv_bfloat16*>(net.Wt[l])) +
+                                    pk_off(c, r, net.N[l])) = h;
 }
 
 // Packed BF16 W (N x K) and W^T (K x N) of one layer from the real FP32
@@ -745,9 +828,9 @@ struct akb_mlp {
   int64_t cap_tiles = 0;
   std::vector<void*> work;
   Bufs bufs{};
-  float* d_part = nullptr;
+  float* d_part = nullptr;  // partial gradients of all layers
   size_t part_cap = 0;
-  float* h_loss = nullptr;  // pinned, one float per tile
+  float* h_loss = nullptr;  // pinned: one float per tile, then the error flag
 };
 
 namespace {
@@ -778,6 +861,15 @@ akb_status repack(akb_mlp* m) {
   return AKB_OK;
 }
 
+Layout layout_of(const akb_mlp* m) {
+  Layout lay{};
+  for (int l = 0; l < m->net.nl; ++l) {
+    lay.w_off[l] = m->w_off[l];
+    lay.b_off[l] = m->b_off[l];
+  }
+  return lay;
+}
+
 akb_status ensure_workspace(akb_mlp* m, int64_t ntiles) {
   if (ntiles <= m->cap_tiles) return AKB_OK;
   for (void* p : m->work) cudaFree(p);
@@ -794,7 +886,7 @@ akb_status ensure_workspace(akb_mlp* m, int64_t ntiles) {
   AKB_CUDA_TRY(dmalloc(m->work, &b.loss_tiles, (size_t)ntiles));
   m->bufs = b;
   if (m->h_loss) cudaFreeHost(m->h_loss);
-  AKB_CUDA_TRY(cudaMallocHost((void**)&m->h_loss, ntiles * sizeof(float)));
+  AKB_CUDA_TRY(cudaMallocHost((void**)&m->h_loss, ntiles * sizeof(float) + sizeof(int)));
   m->cap_tiles = ntiles;
   return AKB_OK;
 }
@@ -815,35 +907,47 @@ akb_status gradients(akb_mlp* m, int64_t nb, const double* x, const double* targ
   // so a few more tiles per CTA cost less than more partials to write and sum
   const int tpc = (int)std::min<int64_t>(ntiles, std::max<int64_t>(4, (ntiles + 147) / 148));
   const int nparts = (int)((ntiles + tpc - 1) / tpc);
+  GradArgs g{};
+  size_t need = 0;
+  int widest = 0, nbias = 0;
   for (int l = 0; l < n.nl; ++l) {
     const bool last = l == n.nl - 1;
     // dW_l = dZ_l^T H_l (the output layer as its transpose: M must be 128 or 256)
-    const unsigned char* A = last ? m->bufs.act[l] : m->bufs.dz[l];
-    const unsigned char* B = last ? m->bufs.dz[l] : m->bufs.act[l];
-    const int ca = last ? n.K[l] : n.N[l], cb = last ? n.N[l] : n.K[l];
-    const size_t need = (size_t)nparts * ca * cb;
-    if (need > m->part_cap) {
-      if (m->d_part) cudaFree(m->d_part);
-      m->d_part = nullptr;
-      AKB_CUDA_TRY(cudaMalloc((void**)&m->d_part, need * sizeof(float)));
-      m->part_cap = need;
-    }
-    k_wgrad<<<nparts, kThreads, kWgradSmem, m->stream>>>(A, ca, B, cb, ntiles, tpc, m->d_part,
-                                                         m->d_error);
-    AKB_CUDA_TRY(cudaGetLastError());
-    const int cnt = n.Nr[l] * n.Kr[l];
-    k_sum_partials<<<(cnt + 255) / 256, 256, 0, m->stream>>>(m->d_part, nparts, ca, cb, n.Nr[l],
-                                                             n.Kr[l], last, m->d_grad + m->w_off[l]);
-    AKB_CUDA_TRY(cudaGetLastError());
-    k_bias_grad<<<(n.Nr[l] + 127) / 128, 128, 0, m->stream>>>(m->bufs.dz[l], n.N[l], n.Nr[l],
-                                                               ntiles, m->d_grad + m->b_off[l]);
-    AKB_CUDA_TRY(cudaGetLastError());
+    g.A[l] = last ? m->bufs.act[l] : m->bufs.dz[l];
+    g.B[l] = last ? m->bufs.dz[l] : m->bufs.act[l];
+    g.ca[l] = last ? n.K[l] : n.N[l];
+    g.cb[l] = last ? n.N[l] : n.K[l];
+    g.dz_is_b[l] = last;
+    g.rows[l] = n.Nr[l];
+    g.bias[l] = m->d_grad + m->b_off[l];
+    need += (size_t)nparts * g.ca[l] * g.cb[l];
+    widest = std::max(widest, g.ca[l] * g.cb[l]);
+    nbias = std::max(nbias, (n.N[l] + kBiasCols - 1) / kBiasCols);
   }
+  if (need > m->part_cap) {
+    if (m->d_part) cudaFree(m->d_part);
+    m->d_part = nullptr;
+    m->part_cap = 0;
+    AKB_CUDA_TRY(cudaMalloc((void**)&m->d_part, need * sizeof(float)));
+    m->part_cap = need;
+  }
+  float* at = m->d_part;
+  for (int l = 0; l < n.nl; ++l) {
+    g.part[l] = at;
+    at += (size_t)nparts * g.ca[l] * g.cb[l];
+  }
+  k_wgrad<<<dim3(nbias + nparts, n.nl), kThreads, kWgradSmem, m->stream>>>(g, nbias, ntiles, tpc,
+                                                                           m->d_error);
+  AKB_CUDA_TRY(cudaGetLastError());
+  k_sum_partials<<<dim3((widest + 255) / 256, n.nl), 256, 0, m->stream>>>(n, g, nparts, layout_of(m),
+                                                                          m->d_grad);
+  AKB_CUDA_TRY(cudaGetLastError());
+  int* h_err = reinterpret_cast<int*>(m->h_loss + m->cap_tiles);
   AKB_CUDA_TRY(cudaMemcpyAsync(m->h_loss, m->bufs.loss_tiles, ntiles * sizeof(float),
                                cudaMemcpyDeviceToHost, m->stream));
-  int err = 0;
-  AKB_CUDA_TRY(cudaMemcpyAsync(&err, m->d_error, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  AKB_CUDA_TRY(cudaMemcpyAsync(h_err, m->d_error, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   AKB_CUDA_TRY(cudaStreamSynchronize(m->stream));
+  const int err = *h_err;
   if (err) return fail(AKB_ERR_TIMEOUT, "tensor-core MMA completion wait timed out");
   double acc = 0.0;
   for (int64_t t = 0; t < ntiles; ++t) acc += m->h_loss[t];
@@ -1058,10 +1162,14 @@ akb_status akb_mlp_apply_gradients(akb_mlp* m, float learning_rate) {
   m->adam_step += 1;
   const float c1 = 1.0f - std::pow(b1, (float)m->adam_step);
   const float c2 = 1.0f - std::pow(b2, (float)m->adam_step);
-  k_adam<<<(unsigned)((m->nparams + 255) / 256), 256, 0, m->stream>>>(
-      m->d_params, m->d_grad, m->d_m1, m->d_m2, m->nparams, learning_rate, b1, b2, eps, c1, c2);
+  int widest = 0;
+  for (int l = 0; l < m->net.nl; ++l)
+    widest = std::max(widest, m->net.Nr[l] * m->net.Kr[l] + m->net.Nr[l]);
+  k_adam<<<dim3((widest + 255) / 256, m->net.nl), 256, 0, m->stream>>>(
+      m->net, layout_of(m), m->d_params, m->d_grad, m->d_m1, m->d_m2, learning_rate, b1, b2, eps,
+      c1, c2);
   AKB_CUDA_TRY(cudaGetLastError());
-  return repack(m);
+  return AKB_OK;
 }
 
 akb_status akb_mlp_train_step(akb_mlp* m, int64_t nb, const double* x, const double* target,
