@@ -47,6 +47,7 @@ struct akb_model {
   bool stresses_valid = false;
   // user materials: stresses come from the caller between step_begin/end
   bool user = false;
+  bool linear = false;  // every material small-strain elastic
   bool in_step = false;
   double* d_scratch = nullptr;  // reduction partials
   int scratch_len = 0;
@@ -243,6 +244,20 @@ void patch_params(int type, int* target, int* max_nodes) {
 template <typename T>
 akb_status upload(akb_model* m, const std::vector<T>& v, const T** out);
 
+// The same for fan records: patches of at most max_fans fans of at most
+// fan_cap elements.
+void fan_params(int type, int* target, int* max_nodes, int* fan_cap, int* max_fans) {
+  *fan_cap = 8;
+  *max_fans = 128;
+  if (type == AKB_TRIANGLE_3) {
+    *target = 768;
+    *max_nodes = 500;
+  } else {
+    *target = 768;
+    *max_nodes = 320;
+  }
+}
+
 // Patch plan of the fused step on the host (mesh in the caller's node
 // order): a single mesh, a partitioned part (its interface nodes forced to
 // be finished outside the fused step), or a batch (patches built per
@@ -250,8 +265,10 @@ akb_status upload(akb_model* m, const std::vector<T>& v, const T** out);
 // patch_inst / orphan_inst: the instance of each patch and node of no
 // element (batches only).
 akb_status plan_patches(akb_model* m, const akb_mesh_desc* mesh, const BatchLayout* batch,
-                        const PartLayout* part, PatchHost& P, std::vector<uint32_t>& patch_inst,
-                        std::vector<uint32_t>& orphan_inst) {
+                        const PartLayout* part, bool fans, PatchHost& P,
+                        std::vector<uint32_t>& patch_inst, std::vector<uint32_t>& orphan_inst) {
+  patch_inst.clear();
+  orphan_inst.clear();
   int target, max_nodes;
   patch_params(m->dm.type, &target, &max_nodes);
   if (fp32(m) && m->dm.type == AKB_TETRAHEDRON_4) {
@@ -261,6 +278,8 @@ akb_status plan_patches(akb_model* m, const akb_mesh_desc* mesh, const BatchLayo
     target = 768;
     max_nodes = 320;
   }
+  int fan_cap = 0, max_fans = 0;
+  if (fans) fan_params(m->dm.type, &target, &max_nodes, &fan_cap, &max_fans);
   if (m->opt_patch_elements <= 0) {
     // small meshes: patches of down to one chunk, so that there are about two
     // per SM (measured on the 8000-element plate: 12.7 ms for 1000 steps at
@@ -280,7 +299,10 @@ akb_status plan_patches(akb_model* m, const akb_mesh_desc* mesh, const BatchLayo
       }
     }
   }
-  if (m->opt_patch_elements > 0) target = std::min(m->opt_patch_elements, 8191);
+  if (m->opt_patch_elements > 0) {
+    target = std::min(m->opt_patch_elements, 8191);
+    max_fans = target;
+  }
   if (m->opt_patch_nodes > 0) max_nodes = std::min(m->opt_patch_nodes, 60000);
   const int cbytes = fp32(m) ? 4 : 8;  // element vector precision
   try {
@@ -292,11 +314,12 @@ akb_status plan_patches(akb_model* m, const akb_mesh_desc* mesh, const BatchLayo
       }
       P = build_patches(mesh->nodes, mesh->connectivity, mesh->nb_nodes, mesh->nb_elements,
                         m->dm.dim, m->dm.nnpe, target, max_nodes, cbytes,
-                        part ? force.data() : nullptr);
+                        part ? force.data() : nullptr, fan_cap, max_fans);
       return AKB_OK;
     }
     const int dd = m->dm.dim, nn_ = m->dm.nnpe;
     P = PatchHost{};
+    P.fans = fans;
     P.elem_ptr.push_back(0);
     P.sh_ptr.push_back(0);
     std::vector<uint32_t> lconn;
@@ -306,7 +329,7 @@ akb_status plan_patches(akb_model* m, const akb_mesh_desc* mesh, const BatchLayo
       lconn.assign(mesh->connectivity + e0 * nn_, mesh->connectivity + (e0 + nei) * nn_);
       for (auto& c : lconn) c -= (uint32_t)n0;
       PatchHost Q = build_patches(mesh->nodes + n0 * dd, lconn.data(), nni, nei, dd, nn_, target,
-                                  max_nodes, cbytes);
+                                  max_nodes, cbytes, nullptr, fan_cap, max_fans);
       const int64_t ebase = (int64_t)P.sgid.size();
       const int64_t chbase = (int64_t)P.chunks.size();
       const uint32_t dbase16 = (uint32_t)(P.cdata.size() / 8);
@@ -359,6 +382,8 @@ akb_status build_device_patches(akb_model* m, const PatchHost& P,
                                 const PartLayout* part) {
   DevPatches& d = m->patches;
   d = DevPatches{};
+  d.fans = P.fans;
+  d.linear = m->linear;
   d.npatch = P.npatch;
   d.grid = m->opt_patch_grid > 0 ? m->opt_patch_grid : 0;
   d.max_nodes = P.max_nodes;
@@ -436,6 +461,16 @@ akb_status build_device_patches(akb_model* m, const PatchHost& P,
     std::vector<uint32_t> em(P.elem_order.size());
     for (size_t i = 0; i < em.size(); ++i) em[i] = element_material[P.elem_order[i]];
     if ((st = upload(m, em, &d.emat)) != AKB_OK) return st;
+    if (P.fans) {
+      std::vector<uint32_t> pm(P.npatch);
+      for (int p = 0; p < P.npatch; ++p) {
+        pm[p] = em[P.elem_ptr[p]];
+        for (int32_t i = P.elem_ptr[p]; i < P.elem_ptr[p + 1]; ++i)
+          if (em[i] != pm[p]) pm[p] = kMixed;
+      }
+      if ((st = upload(m, pm, &d.patch_mat)) != AKB_OK) return st;
+    }
+    AKB_CUDA_TRY(cudaStreamSynchronize(m->stream));  // host vectors go out of scope
   }
   {
     double* ke;
@@ -462,8 +497,9 @@ akb_status build_device_patches(akb_model* m, const PatchHost& P,
     if ((st = upload(m, li, &d.list_inst)) != AKB_OK) return st;
   }
   AKB_CUDA_TRY(cudaStreamSynchronize(m->stream));  // host vectors go out of scope
-  d.nbuf = patch_buffers(d, m->dm.type, fp32(m));
-  const size_t smem = patch_smem_bytes(d, m->dm.dim, fp32(m), d.nbuf);
+  d.nbuf = P.fans ? 1 : patch_buffers(d, m->dm.type, fp32(m));
+  const size_t smem = P.fans ? fan_smem_bytes(d.max_nodes, d.contrib_slots, d.chunk_bytes, m->dm.dim)
+                             : patch_smem_bytes(d, m->dm.dim, fp32(m), d.nbuf);
   if (smem > 227 * 1024)
     return fail(AKB_ERR_UNSUPPORTED, "patch does not fit in shared memory");
   AKB_CUDA_TRY(patch_configure(m->dm, d, fp32(m)));
@@ -711,6 +747,9 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
     std::vector<MatParams> table(nb_materials);
     for (int k = 0; k < nb_materials; ++k) table[k] = make_params(materials[k], d);
     for (int k = 0; k < nb_materials && k < kMaxMaterials; ++k) dm.mats[k] = table[k];
+    m->linear = true;
+    for (const MatParams& t : table)
+      m->linear = m->linear && t.kind == AKB_MATERIAL_ELASTIC && !t.finite;
     if ((st = upload(m.get(), table, &dm.mat_table)) != AKB_OK) return st;
     AKB_CUDA_TRY(cudaStreamSynchronize(m->stream));
   }
@@ -727,7 +766,17 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
   const double* mesh_X = mesh->nodes;
   const uint32_t* mesh_C = mesh->connectivity;
   if (patched) {
-    if ((st = plan_patches(m.get(), mesh, batch, part, plan, patch_inst, orphan_inst)) != AKB_OK)
+    // FP64 triangles and tetrahedra step on fan records; a plan whose record or
+    // contributions do not fit an SM (patch sizes far above the defaults)
+    // steps chunk by chunk
+    bool fans = m->mode == AKB_MODE_FP64 && (type == AKB_TRIANGLE_3 || type == AKB_TETRAHEDRON_4);
+    if (fans) {
+      st = plan_patches(m.get(), mesh, batch, part, true, plan, patch_inst, orphan_inst);
+      fans = st == AKB_OK && fan_smem_bytes(plan.max_nodes, plan.contrib_slots, plan.chunk_bytes, d) <=
+                                 227 * 1024;
+    }
+    if (!fans &&
+        (st = plan_patches(m.get(), mesh, batch, part, false, plan, patch_inst, orphan_inst)) != AKB_OK)
       return st;
     Xr.resize(ndof);
     for (int64_t i = 0; i < nn; ++i)

@@ -591,6 +591,373 @@ __global__ void __launch_bounds__(kThreads, (PatchOccupancy<T, S>::value))
   }
 }
 
+// ------------------------------------------------------------- fan records
+// The fused step on fan records (akb_patch.cuh: FP64 triangles and
+// tetrahedra). As k_patch_step, with two differences:
+//  - a thread computes a fan, a row of elements around a hinge, keeping the
+//    hinge and the last ring node in registers: each further element loads one
+//    node and writes one contribution. An element costs about 105 FP64
+//    operations (the hinge's cross products are shared between neighbours)
+//    and a quarter of the shared-memory traffic of its corner-by-corner form;
+//  - all contributions of the patch stay in shared memory, so that the node
+//    sums run once per patch and feed the finish directly: two barriers a
+//    patch instead of two per 256 elements, and no force accumulators.
+constexpr int kFanThreads = 128;
+
+struct FanLayout {
+  size_t xs, ws, c, rec, mbar, total;
+};
+__host__ __device__ inline FanLayout fan_layout(int Lmax, int slots, int rec_bytes, int d) {
+  FanLayout s;
+  const size_t nb = align16(16 + (size_t)Lmax * d * sizeof(double));
+  s.xs = 0;
+  s.ws = nb;
+  s.c = 2 * nb;
+  s.rec = align128(s.c + (size_t)slots * d * sizeof(double));
+  s.mbar = s.rec + align16((size_t)rec_bytes);
+  s.total = s.mbar + 16;
+  return s;
+}
+__host__ __device__ inline FanLayout fan_layout(const DevPatches& p, int d) {
+  return fan_layout(p.max_nodes, p.contrib_slots, p.chunk_bytes, d);
+}
+
+// CTAs per SM each instantiation is built for (register budget).
+template <int D, bool LIN> struct FanOccupancy { static constexpr int value = 3; };
+template <> struct FanOccupancy<3, true> { static constexpr int value = 4; };
+template <> struct FanOccupancy<2, true> { static constexpr int value = 6; };
+template <> struct FanOccupancy<2, false> { static constexpr int value = 5; };
+
+// w P of one element from G = det * grad u (row-major), P the Cauchy (small
+// strain) or first Piola stress, w the reference volume of the simplex.
+template <int d, bool LIN>
+__device__ inline void fan_stress(const MatParams& mp, const double* G, double det, double* P) {
+  constexpr double w = d == 3 ? 1.0 / 6.0 : 0.5;
+  if constexpr (LIN) {
+    const double s = w / det, mu = mp.mu * s;
+    double tr = G[0] + G[d + 1];
+    if (d == 3) tr += G[2 * d + 2];
+    tr *= mp.lambda * s;
+#pragma unroll
+    for (int i = 0; i < d; ++i) {
+      P[i * d + i] = fma(2.0 * mu, G[i * d + i], tr);
+#pragma unroll
+      for (int j = 0; j < i; ++j) P[i * d + j] = P[j * d + i] = mu * (G[i * d + j] + G[j * d + i]);
+    }
+  } else {
+    const double idet = 1.0 / det;
+    double g[d * d];
+#pragma unroll
+    for (int k = 0; k < d * d; ++k) g[k] = G[k] * idet;
+    fast::stress_P<d, double>(mp, g, P);
+#pragma unroll
+    for (int k = 0; k < d * d; ++k) P[k] *= w;
+  }
+}
+
+__device__ inline void cross3(const double* a, const double* b, double* c) {
+  c[0] = a[1] * b[2] - a[2] * b[1];
+  c[1] = a[2] * b[0] - a[0] * b[2];
+  c[2] = a[0] * b[1] - a[1] * b[0];
+}
+
+// Contributions of fan t of a staged patch. The simplex (hinge, r_t, r_{t+1})
+// has the edges e1 (tetrahedra: to the hinge's second node), e2, e3 from the
+// hinge's first node; the columns of the adjugate of J are e2 x e3, e3 x e1 =
+// -c3 and e1 x e2 = c2, c3 being the next element's c2.
+template <int d, bool LIN>
+__device__ __forceinline__ void fan_forces(const uint16_t* rec, int t, const double* xs,
+                                           const double* ws, double* C, const MatParams& mp0,
+                                           const MatParams* table, const uint32_t* emat) {
+  constexpr int H = d - 1;
+  const uint16_t* ro = rec + rec[2];
+  const uint16_t* node = rec + rec[3];
+  const uint32_t info = reinterpret_cast<const uint32_t*>(rec + rec[4])[t];
+  const int k = (int)(info & 0x7fff);
+  const bool closed = info & 0x8000;
+  const int ja = node[t], j0 = node[ro[H] + t];
+  double xa[d], ua[d], e1[3], d1[3], e2[d], d2[d], c2[3], fa[d], fb[3], ft[d];
+  auto load = [&](int j, double* x, double* u) {
+    if constexpr (d == 2) {
+      const double2 p = reinterpret_cast<const double2*>(xs)[j];
+      const double2 q = reinterpret_cast<const double2*>(ws)[j];
+      x[0] = p.x;
+      x[1] = p.y;
+      u[0] = q.x;
+      u[1] = q.y;
+    } else {
+#pragma unroll
+      for (int i = 0; i < d; ++i) {
+        x[i] = xs[d * j + i];
+        u[i] = ws[d * j + i];
+      }
+    }
+  };
+  auto edge = [&](int j, double* e, double* u) {
+    load(j, e, u);
+#pragma unroll
+    for (int i = 0; i < d; ++i) {
+      e[i] -= xa[i];
+      u[i] -= ua[i];
+    }
+  };
+  auto store = [&](int s, const double* f) {
+    if constexpr (d == 2) {
+      reinterpret_cast<double2*>(C)[s] = make_double2(f[0], f[1]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < d; ++i) C[d * s + i] = f[i];
+    }
+  };
+  load(ja, xa, ua);
+  edge(j0, e2, d2);
+  if constexpr (d == 3) {
+    edge(node[ro[1] + t], e1, d1);
+    cross3(e1, e2, c2);
+  }
+#pragma unroll
+  for (int i = 0; i < d; ++i) fa[i] = ft[i] = 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) fb[i] = 0.0;
+#pragma unroll 1
+  for (int s = 0; s < k; ++s) {
+    const int jn = closed && s == k - 1 ? j0 : node[ro[H + 1 + s] + t];
+    const MatParams& mp = emat ? table[emat[(info >> 16) + s]] : mp0;
+    double e3[d], d3[d], fn[d], G[d * d], P[d * d];
+    edge(jn, e3, d3);
+    if constexpr (d == 3) {
+      double x[3], c3[3];
+      cross3(e2, e3, x);
+      cross3(e1, e3, c3);
+      const double det = e1[0] * x[0] + e1[1] * x[1] + e1[2] * x[2];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) G[i * 3 + j] = d1[i] * x[j] - d2[i] * c3[j] + d3[i] * c2[j];
+      fan_stress<d, LIN>(mp, G, det, P);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        fb[i] += P[i * 3] * x[0] + P[i * 3 + 1] * x[1] + P[i * 3 + 2] * x[2];
+        ft[i] -= P[i * 3] * c3[0] + P[i * 3 + 1] * c3[1] + P[i * 3 + 2] * c3[2];
+        fn[i] = P[i * 3] * c2[0] + P[i * 3 + 1] * c2[1] + P[i * 3 + 2] * c2[2];
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i) c2[i] = c3[i];
+    } else {
+      const double det = e2[0] * e3[1] - e2[1] * e3[0];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {  // adjugate columns (e3y, -e3x), (-e2y, e2x)
+        G[i * 2] = d2[i] * e3[1] - d3[i] * e2[1];
+        G[i * 2 + 1] = d3[i] * e2[0] - d2[i] * e3[0];
+      }
+      fan_stress<d, LIN>(mp, G, det, P);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        ft[i] += P[i * 2] * e3[1] - P[i * 2 + 1] * e3[0];
+        fn[i] = P[i * 2 + 1] * e2[0] - P[i * 2] * e2[1];
+      }
+    }
+    store(ro[H + s] + t, ft);
+#pragma unroll
+    for (int i = 0; i < d; ++i) {  // the forces of an element add up to zero
+      fa[i] -= ft[i];
+      ft[i] = fn[i];
+      e2[i] = e3[i];
+      d2[i] = d3[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < d; ++i) {
+    fa[i] -= ft[i];
+    if (d == 3) fa[i] -= fb[i];
+  }
+  if (closed) {  // r_0's contribution, written by this thread above
+    const int s = ro[H] + t;
+#pragma unroll
+    for (int i = 0; i < d; ++i) C[d * s + i] += ft[i];
+  } else {
+    store(ro[H + k] + t, ft);
+  }
+  store(t, fa);
+  if constexpr (d == 3) store(ro[1] + t, fb);
+}
+
+// One patch p, by the whole CTA; stages: patches it staged before (the phase
+// of the mbarrier). Returns false when a bounded wait gave up.
+template <int d, bool LIN, bool FEXT>
+__device__ __forceinline__ bool fan_body(const DevModel& m, const DevPatches& P, double dt0, int p,
+                                         unsigned char* smem, uint32_t& stages) {
+  constexpr int T = kFanThreads;
+  const double dt = P.inst_dt ? P.inst_dt[P.patch_inst[p]] : dt0;
+  const int ib = P.ibeg[p], nint = P.nint[p];
+  const int s0 = P.sh_ptr[p], nsh = P.sh_ptr[p + 1] - s0;
+  const FanLayout lay = fan_layout(P, d);
+  // the interior slices of X and w (see patch_body) and the record
+  const size_t row = (size_t)d * sizeof(double);
+  const size_t s_lo = (size_t)ib * row, s_hi = (size_t)(ib + nint) * row;
+  const size_t c_lo = s_lo & ~size_t(15), c_hi = s_hi & ~size_t(15);
+  const int o = (int)((s_lo - c_lo) / sizeof(double));
+  double* xs = reinterpret_cast<double*>(smem + lay.xs) + o;
+  double* ws = reinterpret_cast<double*>(smem + lay.ws) + o;
+  double* C = reinterpret_cast<double*>(smem + lay.c);
+  const uint16_t* rec = reinterpret_cast<const uint16_t*>(smem + lay.rec);
+  const int tid = threadIdx.x;
+  const uint32_t mb = saddr(smem + lay.mbar);
+  if (tid == 0) {
+    // the previous patch's generic-proxy accesses of these buffers (ordered
+    // before this point by the CTA barrier) come before the bulk copies
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    const uint2 cd = __ldg(reinterpret_cast<const uint2*>(&P.chunks[p]));  // off16, bytes
+    const uint32_t bytes = nint > 0 && c_hi > c_lo ? (uint32_t)(c_hi - c_lo) : 0;
+    expect_tx(mb, 2 * bytes + cd.y);
+    bulk_copy(saddr(smem + lay.rec), P.cdata + (size_t)cd.x * 8, cd.y, mb);
+    if (bytes) {
+      bulk_copy(saddr(smem + lay.xs), reinterpret_cast<const char*>(m.X) + c_lo, bytes, mb);
+      bulk_copy(saddr(smem + lay.ws), reinterpret_cast<const char*>(P.w) + c_lo, bytes, mb);
+    }
+    if (nint > 0) {  // inputs of the interior nodes' finish
+      prefetch_l2(m.v, s_lo, s_hi);
+      prefetch_l2(m.a, s_lo, s_hi);
+      prefetch_l2(m.inv_mass, (size_t)ib * 8, (size_t)(ib + nint) * 8);
+      prefetch_l2(m.blocked, (size_t)ib * d, (size_t)(ib + nint) * d);
+      if (FEXT) prefetch_l2(m.fext, s_lo, s_hi);
+    }
+  }
+  if (tid == T - 1 && nint > 0 && c_hi < s_hi && c_hi >= s_lo) {  // the tail double
+    const size_t k = (c_hi - s_lo) / sizeof(double);
+    cp_async8(xs + k, m.X + (size_t)ib * d + k);
+    cp_async8(ws + k, P.w + (size_t)ib * d + k);
+  } else if (tid == T - 1 && nint > 0 && c_hi < s_lo) {  // slice within one 16 bytes
+    for (size_t k = 0; k < (size_t)nint * d; ++k) {
+      cp_async8(xs + k, m.X + (size_t)ib * d + k);
+      cp_async8(ws + k, P.w + (size_t)ib * d + k);
+    }
+  }
+  for (int t = tid; t < nsh; t += T) {
+    const int64_t g = P.sgid[s0 + t];
+    const int j = nint + t;
+    if constexpr (d == 2) {
+      cp_async16(xs + 2 * j, m.X + g * 2);
+      cp_async16(ws + 2 * j, P.w + g * 2);
+    } else {
+#pragma unroll
+      for (int i = 0; i < d; ++i) {
+        cp_async8(xs + d * j + i, m.X + g * d + i);
+        cp_async8(ws + d * j + i, P.w + g * d + i);
+      }
+    }
+  }
+  cp_async_wait_all();
+  {
+    const bool ok = mbar_wait(mb, stages & 1u);
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0) {
+        atomicExch(P.err, 1);
+        mbar_wait(mb, stages & 1u);
+      }
+      return false;
+    }
+  }
+  ++stages;
+
+  // element forces, one thread per fan
+  {
+    const uint32_t pm = P.patch_mat ? P.patch_mat[p] : 0;
+    const bool mixed = pm == kMixed;
+    const MatParams& mp = P.patch_mat && !mixed ? m.mat_table[pm] : m.mats[0];
+    const uint32_t* emat = mixed ? P.emat + P.elem_ptr[p] : nullptr;
+    const int nf = rec[0];
+    for (int t = tid; t < nf; t += T)
+      fan_forces<d, LIN>(rec, t, xs, ws, C, mp, m.mat_table, emat);
+  }
+
+  // finish: the interior nodes one thread per DOF, contiguous in the global
+  // arrays, their inputs requested before the barrier; then the shared nodes'
+  // partials to their slots (the second pass adds them)
+  const int items = nint * d;
+  double v[kBatch], a[kBatch], im[kBatch], fx[kBatch];
+  uint8_t bl[kBatch];
+  auto request = [&](int base) {
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int k = base + b * T + tid;
+      if (k < items) {
+        const int64_t q = (int64_t)ib * d + k;
+        bl[b] = m.blocked[q];
+        v[b] = m.v[q];
+        a[b] = m.a[q];
+        im[b] = m.inv_mass[ib + k / d];
+        fx[b] = FEXT ? m.fext[q] : 0.0;
+      }
+    }
+  };
+  request(0);
+  grid_launch_dependents();  // the second pass may start launching (it waits for this grid)
+  __syncthreads();
+  const uint16_t* ptr = rec + rec[5];
+  const uint16_t* idx = rec + rec[6];
+  auto force = [&](int j, int i) {  // minus the sum of the node's contributions
+    double f = 0.0;
+    const int e = ptr[j + 1];
+#pragma unroll 4
+    for (int q = ptr[j]; q < e; ++q) f -= C[d * idx[q] + i];
+    return f;
+  };
+  double ke = 0.0;  // M v^2 of this thread's DOFs after the step
+  for (int base = 0; base < items; base += T * kBatch) {
+    if (base > 0) request(base);
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int k = base + b * T + tid;
+      if (k >= items) continue;
+      if (!bl[b]) {  // blocked DOFs keep u, v, a (and w = u)
+        const int j = k / d, i = k - j * d;
+        const int64_t q = (int64_t)ib * d + k;
+        const double f = force(j, i);
+        double u, wn;
+        finish_dof(dt, FEXT ? f + fx[b] : f, im[b], ws[k], v[b], a[b], u, wn);
+        m.u[q] = u;
+        m.v[q] = v[b];
+        m.a[q] = a[b];
+        P.w[q] = wn;
+      }
+      ke += ke_term(v[b], im[b]);
+    }
+  }
+  for (int k = tid; k < nsh * d; k += T) {
+    const int t = k / d, i = k - t * d;
+    P.partial[(size_t)P.sslot[s0 + t] * d + i] = force(nint + t, i);
+  }
+  if (P.ke_part) {
+    __shared__ double warp_sums[T / 32];
+    const double s = cta_sum(ke, warp_sums);
+    if (tid == 0) P.ke_part[p] = s;
+  }
+  return true;
+}
+
+template <int d, bool LIN, bool FEXT, bool PERSIST>
+__global__ void __launch_bounds__(kFanThreads, (FanOccupancy<d, LIN>::value))
+    k_fan_step(DevModel m, DevPatches P, double dt0) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(smem + fan_layout(P, d).mbar))
+                 : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  grid_wait();  // the previous step's (or update's) writes of w, v, a, u
+  uint32_t stages = 0;
+  if constexpr (PERSIST) {
+    for (int p = blockIdx.x; p < P.npatch; p += gridDim.x) {
+      if (p != (int)blockIdx.x) __syncthreads();  // shared memory of the previous patch is free
+      if (!fan_body<d, LIN, FEXT>(m, P, dt0, p, smem, stages)) return;
+    }
+  } else {
+    fan_body<d, LIN, FEXT>(m, P, dt0, blockIdx.x, smem, stages);
+  }
+}
+
 // Listed nodes, one thread per (entry, component): the sum of the entry's
 // partials in rank order (none for a node of no element), then the same
 // finish as in the fused step, from the node's stored w; and the block's sum
@@ -829,6 +1196,38 @@ cudaError_t raise_smem_limit(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// f(kernel) for the fan step's instantiation of a plan.
+template <int d, typename F>
+cudaError_t with_fan_kernel(bool lin, bool fext, bool persist, F f) {
+  if (lin)
+    return fext ? (persist ? f(k_fan_step<d, true, true, true>) : f(k_fan_step<d, true, true, false>))
+                : (persist ? f(k_fan_step<d, true, false, true>) : f(k_fan_step<d, true, false, false>));
+  return fext ? (persist ? f(k_fan_step<d, false, true, true>) : f(k_fan_step<d, false, true, false>))
+              : (persist ? f(k_fan_step<d, false, false, true>) : f(k_fan_step<d, false, false, false>));
+}
+
+template <int d>
+cudaError_t launch_fan(const DevModel& m, const DevPatches& p, double dt, bool fext, cudaStream_t s) {
+  const int grid = grid_of(p);
+  const size_t bytes = fan_layout(p, d).total;
+  return with_fan_kernel<d>(p.linear, fext, grid < p.npatch, [&](auto kernel) {
+    return launch_pdl(kernel, grid, kFanThreads, bytes, s, m, p, dt);
+  });
+}
+
+template <int d>
+cudaError_t configure_fan(const DevPatches& p) {
+  const size_t bytes = fan_layout(p, d).total;
+  std::lock_guard<std::mutex> lock(g_attr_mutex);
+  for (int k = 0; k < 4; ++k) {
+    const cudaError_t e = with_fan_kernel<d>(p.linear, k & 1, k & 2, [&](auto kernel) {
+      return raise_smem_limit(kernel, bytes);
+    });
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 template <int T, typename S>
 cudaError_t configure(const DevPatches& p) {
   const SmemLayout lay = layout(p, ET<T>::dim, sizeof(S), p.nbuf);
@@ -844,6 +1243,10 @@ cudaError_t configure(const DevPatches& p) {
 
 size_t patch_smem_bytes(const DevPatches& p, int dim, bool fp32, int nbuf) {
   return layout(p, dim, fp32 ? 4 : 8, nbuf).total;
+}
+
+size_t fan_smem_bytes(int max_nodes, int slots, int record_bytes, int dim) {
+  return fan_layout(max_nodes, slots, record_bytes, dim).total;
 }
 
 int patch_buffers(const DevPatches& p, int type, bool fp32) {
@@ -869,6 +1272,7 @@ int patch_buffers(const DevPatches& p, int type, bool fp32) {
 }
 
 cudaError_t patch_configure(const DevModel& m, const DevPatches& p, bool fp32) {
+  if (p.fans) return m.dim == 2 ? configure_fan<2>(p) : configure_fan<3>(p);
   switch (m.type) {
   case AKB_SEGMENT_2: return fp32 ? configure<AKB_SEGMENT_2, float>(p) : configure<AKB_SEGMENT_2, double>(p);
   case AKB_TRIANGLE_3: return fp32 ? configure<AKB_TRIANGLE_3, float>(p) : configure<AKB_TRIANGLE_3, double>(p);
@@ -880,6 +1284,7 @@ cudaError_t patch_configure(const DevModel& m, const DevPatches& p, bool fp32) {
 cudaError_t patch_step(const DevModel& m, const DevPatches& p, double dt, bool fp32,
                        bool fext, cudaStream_t s) {
   if (p.npatch == 0) return cudaSuccess;
+  if (p.fans) return m.dim == 2 ? launch_fan<2>(m, p, dt, fext, s) : launch_fan<3>(m, p, dt, fext, s);
   switch (m.type) {
   case AKB_SEGMENT_2:
     return fp32 ? launch_patch<AKB_SEGMENT_2, float>(m, p, dt, fext, s)

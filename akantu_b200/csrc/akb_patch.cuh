@@ -78,6 +78,22 @@ inline int place_group(int dim) { return dim == 2 ? 8 : 16; }
 // runs (one sum instruction) hit G different banks (G = 16 for 8-byte
 // contributions, 32 for 4-byte ones), and the runs of a group have their
 // nodes at distinct positions mod 16 where the build could arrange it.
+// Fan record (FP64 triangles and tetrahedra): one per patch, staged by one
+// bulk copy. A fan is a row of elements around a hinge (a node of triangles, an
+// edge of tetrahedra), element t having the hinge and the ring nodes r_t and
+// r_{t+1}; one thread computes a fan, loading each of its nodes once and
+// writing one contribution per node, so that a fan of six tetrahedra loads 8
+// nodes and writes 8 contributions instead of 24 and 24. Contents (uint16,
+// every section on 16 bytes, offsets in uint16 units):
+//   header   nf, rows, o_row, o_node, o_info, o_ptr, o_idx, slots
+//   rowoff   rows + 1: first slot of row j (row j: node j of the fans that
+//            have one, hinge first; fans by descending row count)
+//   node     slots: the position of the node of slot rowoff[j] + t (row j of
+//            fan t), which is also where its contribution goes
+//   info     per fan: elements | 0x8000 if the ring closes (the last element
+//            ends on r_0, whose contribution it adds to), first element of
+//            the fan within the patch
+//   ptr, idx per position its contribution slots idx[ptr[j] .. ptr[j + 1])
 // Partial slot of rank r of shared node s (ns shared nodes; over: the node's
 // first slot for ranks >= 2).
 __host__ __device__ inline uint32_t partial_slot(uint32_t ns, uint32_t s, uint32_t over,
@@ -91,6 +107,7 @@ struct ChunkDesc {
 };
 
 struct PatchHost {
+  bool fans = false;      // fan records instead of chunk records
   int npatch = 0;
   int max_nodes = 0;      // largest local node count of a patch
   int max_interior = 0;   // largest interior node count of a patch
@@ -124,13 +141,22 @@ struct PatchHost {
 // patch; max_nodes: local node cap (<= 60000); contrib_bytes: element vector
 // precision (8: FP64, 4: FP32); force_shared (per node, or null): nodes treated as shared
 // (finished by the second pass from their partials) even when one patch holds
-// them (the interface nodes of a partitioned mesh).
+// them (the interface nodes of a partitioned mesh). fan_cap > 0 (triangles,
+// tetrahedra): fans of at most fan_cap elements, at most max_fans of them in a
+// patch, with fan records (throws std::length_error when a record does not
+// fit).
 PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64_t ne, int dim,
                         int nnpe, int target_elems, int max_nodes, int contrib_bytes,
-                        const uint8_t* force_shared = nullptr);
+                        const uint8_t* force_shared = nullptr, int fan_cap = 0,
+                        int max_fans = 0);
+
+// patch_mat of a patch with several materials
+constexpr uint32_t kMixed = 0xffffffffu;
 
 // Device copy of a PatchHost.
 struct DevPatches {
+  int fans;  // fan records: the step runs k_fan_step
+  int linear;  // fans: every material is small-strain elastic
   int npatch;
   int grid;  // 0: one CTA per patch; > 0: persistent grid of that many CTAs
   int nbuf;  // chunk record buffers in shared memory (2: next chunk prefetched)
@@ -145,6 +171,7 @@ struct DevPatches {
   const uint2* chunks;     // ChunkDesc per chunk
   const uint16_t* cdata;   // chunk records (16-byte aligned)
   const uint32_t* emat;    // material of each patch-ordered element, or null
+  const uint32_t* patch_mat;  // fans: a patch's only material, kMixed, or null (one material)
   int* err;                // set when a bounded wait gave up
   double* partial;         // nslots x dim
   double* w;               // nn x dim predicted displacement
@@ -178,6 +205,8 @@ struct DevPatches {
 void assign_partial_slots(PatchHost& P, int64_t nn);
 
 size_t patch_smem_bytes(const DevPatches& p, int dim, bool fp32, int nbuf);
+// Shared memory of k_fan_step for a plan.
+size_t fan_smem_bytes(int max_nodes, int slots, int record_bytes, int dim);
 // Chunk record buffers (1 or 2) that keep the most CTAs per SM.
 int patch_buffers(const DevPatches& p, int type, bool fp32);
 cudaError_t patch_configure(const DevModel& m, const DevPatches& p, bool fp32);

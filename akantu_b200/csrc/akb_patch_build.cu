@@ -34,9 +34,12 @@ inline uint64_t spread2(uint64_t x) {  // 31 bits -> every second bit
 // elements in one instruction; each distinct node of such a group should sit
 // at its own position mod G (place_group). Greedy in first-touch order: a
 // node takes, within its range, the residue least used by the groups it
-// belongs to, then the one with the most free positions left.
+// belongs to, then the one with the most free positions left. Entries equal to
+// kNoNode are absent (fans of different lengths); with `first`, the nodes are
+// taken in that order instead.
+constexpr uint16_t kNoNode = 0xffff;
 void place_nodes(const std::vector<uint16_t>& lc, int ne, int nnpe, int L, int nint, int G,
-                 uint16_t* pos) {
+                 uint16_t* pos, const std::vector<int32_t>* first = nullptr) {
   const int nhalf = (ne + G - 1) / G;
   std::vector<std::pair<int32_t, int32_t>> mem;  // (node, group), each pair once
   mem.reserve((size_t)ne * nnpe);
@@ -45,6 +48,7 @@ void place_nodes(const std::vector<uint16_t>& lc, int ne, int nnpe, int L, int n
       const int e0 = h * G, e1 = std::min(ne, e0 + G);
       for (int e = e0; e < e1; ++e) {
         const int v = lc[(size_t)e * nnpe + a];
+        if (v == kNoNode) continue;
         bool dup = false;
         for (int f = e0; f < e && !dup; ++f) dup = lc[(size_t)f * nnpe + a] == v;
         if (!dup) mem.push_back({v, h * nnpe + a});
@@ -58,10 +62,14 @@ void place_nodes(const std::vector<uint16_t>& lc, int ne, int nnpe, int L, int n
   std::vector<int32_t> order;
   order.reserve(L);
   std::vector<char> seen(L, 0);
-  for (int e = 0; e < ne; ++e)
+  if (first) {
+    order = *first;
+    std::fill(seen.begin(), seen.end(), 1);
+  }
+  for (int e = 0; e < ne && !first; ++e)
     for (int a = 0; a < nnpe; ++a) {
       const int v = lc[(size_t)e * nnpe + a];
-      if (!seen[v]) {
+      if (v != kNoNode && !seen[v]) {
         seen[v] = 1;
         order.push_back(v);
       }
@@ -152,12 +160,164 @@ class BipartiteColouring {
   std::vector<int32_t> at_l_, at_r_, eu_, ev_, col_, path_;
 };
 
+// Fans of a simplex mesh: elements in a row around a hinge (triangles around a
+// node, tetrahedra around an edge), each sharing all but one node with the one
+// before. Fan f: its elements elem[eptr[f] .. eptr[f + 1]) in ring order, its
+// nodes node[nptr[f] .. nptr[f + 1]): the hinge (1 or 2 nodes), then the ring
+// r_0 .. r_k (without r_k when the ring closes on r_0); element t has the
+// nodes hinge, r_t, r_{t+1}, in an even permutation of its own order.
+struct Fans {
+  std::vector<int32_t> eptr{0}, nptr{0};
+  std::vector<uint32_t> elem, node;
+  std::vector<uint8_t> closed;
+  int count() const { return (int)closed.size(); }
+  int elems(int f) const { return eptr[f + 1] - eptr[f]; }
+  int rows(int f) const { return nptr[f + 1] - nptr[f]; }
+};
+
+// Greedy in the given element order: an element not yet in a fan tries each of
+// its hinges and takes the one with the best n^2 / m (n of the hinge's m
+// elements still free: long fans, and hinges whose elements are not half used
+// up, which on a structured mesh finds the cover by whole rings), the longest
+// edge among equals; every free element of that hinge then goes into fans of
+// at most `cap` elements.
+Fans build_fans(const double* X, const uint32_t* conn, int64_t nn, int64_t ne, int dim, int cap,
+                const std::vector<uint32_t>& order) {
+  const int n = dim + 1;
+  std::vector<int32_t> ptr(nn + 1, 0);
+  for (int64_t k = 0; k < ne * n; ++k) ++ptr[conn[k] + 1];
+  for (int64_t i = 0; i < nn; ++i) ptr[i + 1] += ptr[i];
+  std::vector<int32_t> ent((size_t)ne * n);
+  {
+    std::vector<int32_t> fill(ptr.begin(), ptr.end() - 1);
+    for (int64_t k = 0; k < ne * n; ++k) ent[fill[conn[k]]++] = (int32_t)(k / n);
+  }
+  Fans F;
+  F.elem.reserve(ne);
+  F.node.reserve((size_t)ne * 2);
+  std::vector<char> used(ne, 0);
+  constexpr size_t kMostLinks = 64;  // elements taken from one hinge at a time
+  auto slot = [&](uint32_t e, uint32_t v) {  // position of v among e's nodes, -1 if absent
+    const uint32_t* c = conn + (int64_t)e * n;
+    for (int a = 0; a < n; ++a)
+      if (c[a] == v) return a;
+    return -1;
+  };
+  auto valence = [&](uint32_t v) { return ptr[v + 1] - ptr[v]; };
+  struct Link {
+    uint32_t from, to, elem;
+  };
+  std::vector<Link> links;
+  std::vector<int> from_of, seq;
+  std::vector<char> taken;
+  for (uint32_t seed : order) {
+    if (used[seed]) continue;
+    const uint32_t* c = conn + (int64_t)seed * n;
+    uint32_t ha = c[0], hb = dim == 3 ? c[1] : c[0];
+    double best = -1.0, best_len = -1.0;
+    for (int a = 0; a < n; ++a)
+      for (int b = dim == 3 ? a + 1 : a; b < (dim == 3 ? n : a + 1); ++b) {
+        int m = 0, free = 0;
+        // an edge's elements are among those of its end with the fewest
+        const uint32_t u = valence(c[a]) <= valence(c[b]) ? c[a] : c[b], o = u == c[a] ? c[b] : c[a];
+        for (int32_t k = ptr[u]; k < ptr[u + 1]; ++k) {
+          const int32_t e = ent[k];
+          if (dim == 3 && slot(e, o) < 0) continue;
+          ++m;
+          free += !used[e];
+        }
+        double len = 0.0;
+        for (int i = 0; i < dim; ++i) {
+          const double t = X[(int64_t)c[a] * dim + i] - X[(int64_t)c[b] * dim + i];
+          len += t * t;
+        }
+        const double score = (double)free * free / m;
+        if (score > best || (score == best && len > best_len)) {
+          best = score;
+          best_len = len;
+          ha = u;
+          hb = o;
+        }
+      }
+    // the free elements of the hinge as directed links r_t -> r_{t+1}
+    links.clear();
+    for (int32_t k = ptr[ha]; k < ptr[ha + 1] && links.size() < kMostLinks; ++k) {
+      const uint32_t e = (uint32_t)ent[k];
+      if (used[e] || (!links.empty() && links.back().elem == e)) continue;
+      const uint32_t* q = conn + (int64_t)e * n;
+      const int a = slot(e, ha);
+      if (dim == 2) {
+        links.push_back({q[(a + 1) % 3], q[(a + 2) % 3], e});
+        continue;
+      }
+      const int b = slot(e, hb);
+      if (b < 0) continue;
+      int o[2], w = 0;
+      for (int t = 0; t < 4; ++t)
+        if (t != a && t != b) o[w++] = t;
+      const int p[4] = {a, b, o[0], o[1]};
+      int inv = 0;  // parity of (a, b, o0, o1) as a permutation of 0..3
+      for (int x = 0; x < 4; ++x)
+        for (int y = x + 1; y < 4; ++y) inv += p[x] > p[y];
+      if (inv & 1) std::swap(o[0], o[1]);
+      links.push_back({q[o[0]], q[o[1]], e});
+    }
+    const int nl = (int)links.size();
+    taken.assign(nl, 0);
+    auto next_of = [&](uint32_t v) {  // a free link leaving v
+      for (int t = 0; t < nl; ++t)
+        if (!taken[t] && links[t].from == v) return t;
+      return -1;
+    };
+    for (int left = nl; left > 0;) {
+      // start where no free link arrives; a ring that closes starts anywhere
+      int first = -1, any = -1;
+      for (int t = 0; t < nl && first < 0; ++t) {
+        if (taken[t]) continue;
+        if (any < 0) any = t;
+        bool arrives = false;
+        for (int q = 0; q < nl && !arrives; ++q) arrives = !taken[q] && links[q].to == links[t].from;
+        if (!arrives) first = t;
+      }
+      if (first < 0) first = any;
+      seq.clear();
+      for (int t = first; t >= 0 && (int)seq.size() < cap; t = next_of(links[t].to)) {
+        taken[t] = 1;
+        seq.push_back(t);
+      }
+      left -= (int)seq.size();
+      const bool closed = seq.size() > 2 && links[seq.back()].to == links[seq[0]].from;
+      F.node.push_back(ha);
+      if (dim == 3) F.node.push_back(hb);
+      for (int t : seq) {
+        F.node.push_back(links[t].from);
+        F.elem.push_back(links[t].elem);
+        used[links[t].elem] = 1;
+      }
+      if (!closed) F.node.push_back(links[seq.back()].to);
+      F.eptr.push_back((int32_t)F.elem.size());
+      F.nptr.push_back((int32_t)F.node.size());
+      F.closed.push_back(closed);
+    }
+    if (!used[seed]) {  // an element that names a node twice: a fan of its own
+      used[seed] = 1;
+      F.elem.push_back(seed);
+      F.node.insert(F.node.end(), c, c + n);
+      F.eptr.push_back((int32_t)F.elem.size());
+      F.nptr.push_back((int32_t)F.node.size());
+      F.closed.push_back(0);
+    }
+  }
+  return F;
+}
+
 }  // namespace
 
 PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64_t ne, int dim,
                         int nnpe, int target_elems, int max_nodes, int contrib_bytes,
-                        const uint8_t* force_shared) {
+                        const uint8_t* force_shared, int fan_cap, int max_fans) {
   PatchHost P;
+  P.fans = fan_cap > 0;
   // 1. element centroids and their Morton keys
   double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
   for (int64_t i = 0; i < nn; ++i)
@@ -194,41 +354,78 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
   //    nodes with their neighbours than cuts of one space-filling curve
   //    (tetrahedral cube, 1024-element parts: 10 % fewer patch-local nodes,
   //    17 % fewer shared-node partials).
+  //    With fans, the units that are bisected are whole fans.
   std::vector<int32_t> stamp(nn, -1);
-  P.elem_order.resize(ne);
-  for (int64_t i = 0; i < ne; ++i) P.elem_order[i] = (uint32_t)i;
-  P.elem_ptr.push_back(0);
+  Fans F;
+  std::vector<uint32_t> unit_order;  // units (elements or fans) in patch order
+  std::vector<int32_t> unit_ptr{0};  // units of each patch
+  int64_t nu = ne;
+  if (P.fans) {
+    std::vector<std::pair<uint64_t, uint32_t>> keyed(ne);
+    for (int64_t e = 0; e < ne; ++e) keyed[e] = {mkey[e], (uint32_t)e};
+    if (!std::is_sorted(keyed.begin(), keyed.end())) std::sort(keyed.begin(), keyed.end());
+    std::vector<uint32_t> by_key(ne);
+    for (int64_t e = 0; e < ne; ++e) by_key[e] = keyed[e].second;
+    F = build_fans(X, conn, nn, ne, dim, std::min(fan_cap, std::max(target_elems, 1)), by_key);
+    nu = F.count();
+    // a fan's centroid and key: those of its elements' mean, and of its first element
+    std::vector<double> fcen((size_t)nu * 3, 0.0);
+    std::vector<uint64_t> fkey(nu);
+    for (int64_t f = 0; f < nu; ++f) {
+      for (int32_t i = F.eptr[f]; i < F.eptr[f + 1]; ++i)
+        for (int k = 0; k < dim; ++k) fcen[(size_t)f * 3 + k] += cen[(size_t)F.elem[i] * 3 + k];
+      for (int k = 0; k < dim; ++k) fcen[(size_t)f * 3 + k] /= F.elems((int)f);
+      fkey[f] = mkey[F.elem[F.eptr[f]]];
+    }
+    cen.swap(fcen);
+    mkey.swap(fkey);
+  }
+  auto unit_elems = [&](uint32_t u) { return P.fans ? F.elems((int)u) : 1; };
+  auto unit_nodes = [&](uint32_t u, const uint32_t** v) {
+    *v = P.fans ? &F.node[F.nptr[u]] : conn + (int64_t)u * nnpe;
+    return P.fans ? F.rows((int)u) : nnpe;
+  };
+  unit_order.resize(nu);
+  for (int64_t i = 0; i < nu; ++i) unit_order[i] = (uint32_t)i;
   {
-    uint32_t* ord = P.elem_order.data();
+    uint32_t* ord = unit_order.data();
     int32_t tag = 0;
     std::vector<std::pair<int64_t, int64_t>> todo;
-    if (ne > 0) todo.push_back({0, ne});
+    if (nu > 0) todo.push_back({0, nu});
     while (!todo.empty()) {
       const int64_t b = todo.back().first, e = todo.back().second;
       todo.pop_back();
       const int64_t n = e - b;
-      bool leaf = n <= target_elems;
+      int64_t elems = n;
+      if (P.fans) {
+        elems = 0;
+        for (int64_t i = b; i < e; ++i) elems += unit_elems(ord[i]);
+      }
+      bool leaf = n == 1 || (elems <= target_elems && (!P.fans || n <= max_fans));
       if (leaf && n > 1) {
         int nodes = 0;
-        for (int64_t i = b; i < e; ++i)
-          for (int a = 0; a < nnpe; ++a) {
-            const uint32_t v = conn[(int64_t)ord[i] * nnpe + a];
-            if (stamp[v] != tag) {
-              stamp[v] = tag;
+        for (int64_t i = b; i < e; ++i) {
+          const uint32_t* v;
+          const int rows = unit_nodes(ord[i], &v);
+          for (int a = 0; a < rows; ++a)
+            if (stamp[v[a]] != tag) {
+              stamp[v[a]] = tag;
               ++nodes;
             }
-          }
+        }
         ++tag;
         leaf = nodes <= max_nodes;
       }
       if (leaf) {
         std::sort(ord + b, ord + e, [&](uint32_t x, uint32_t y) {
+          if (P.fans && F.rows((int)x) != F.rows((int)y)) return F.rows((int)x) > F.rows((int)y);
           return mkey[x] != mkey[y] ? mkey[x] < mkey[y] : x < y;
         });
-        P.elem_ptr.push_back((int32_t)e);
+        unit_ptr.push_back((int32_t)e);
         continue;
       }
-      const int64_t parts = std::max<int64_t>(2, (n + target_elems - 1) / target_elems);
+      int64_t parts = std::max<int64_t>(2, (elems + target_elems - 1) / target_elems);
+      if (P.fans) parts = std::max<int64_t>(parts, (n + max_fans - 1) / max_fans);
       const int64_t k = std::max<int64_t>(1, n * (parts / 2) / parts);
       double clo[3] = {1e300, 1e300, 1e300}, chi[3] = {-1e300, -1e300, -1e300};
       for (int64_t i = b; i < e; ++i)
@@ -246,6 +443,20 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
       todo.push_back({b + k, e});
       todo.push_back({b, b + k});
     }
+  }
+  P.elem_ptr.push_back(0);
+  if (P.fans) {
+    P.elem_order.reserve(ne);
+    for (size_t p = 0; p + 1 < unit_ptr.size(); ++p) {
+      for (int32_t i = unit_ptr[p]; i < unit_ptr[p + 1]; ++i) {
+        const uint32_t f = unit_order[i];
+        P.elem_order.insert(P.elem_order.end(), &F.elem[F.eptr[f]], &F.elem[F.eptr[f]] + F.elems((int)f));
+      }
+      P.elem_ptr.push_back((int32_t)P.elem_order.size());
+    }
+  } else {
+    P.elem_order = unit_order;
+    P.elem_ptr = unit_ptr;
   }
   mkey.clear();
   mkey.shrink_to_fit();
@@ -324,7 +535,30 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
       for (int a = 0; a < nnpe; ++a) lcl[(size_t)(i - eb) * nnpe + a] = (uint16_t)lidx[c[a]];
     }
     pos.assign(L, 0);
-    place_nodes(lcl, ne_p, nnpe, L, nint, GP, pos.data());
+    int nf = 0, rows = 0;
+    if (P.fans) {
+      // the fans' nodes, row by row (lcl: local node of row j of fan t, kNoNode
+      // past its end); nodes of many contributions take the first positions,
+      // so that the threads of a warp sum about as many each
+      nf = unit_ptr[p + 1] - unit_ptr[p];
+      for (int32_t i = unit_ptr[p]; i < unit_ptr[p + 1]; ++i)
+        rows = std::max(rows, F.rows((int)unit_order[i]));
+      lcl.assign((size_t)nf * rows, kNoNode);
+      std::vector<int32_t> uses(L, 0), first(L);
+      for (int t = 0; t < nf; ++t) {
+        const uint32_t f = unit_order[unit_ptr[p] + t];
+        for (int j = 0; j < F.rows((int)f); ++j) {
+          const int v = lidx[F.node[F.nptr[f] + j]];
+          lcl[(size_t)t * rows + j] = (uint16_t)v;
+          ++uses[v];
+        }
+      }
+      std::iota(first.begin(), first.end(), 0);
+      std::stable_sort(first.begin(), first.end(), [&](int32_t x, int32_t y) { return uses[x] > uses[y]; });
+      place_nodes(lcl, nf, rows, L, nint, GP, pos.data(), &first);
+    } else {
+      place_nodes(lcl, ne_p, nnpe, L, nint, GP, pos.data());
+    }
     P.ibeg.push_back((int32_t)next_id);
     P.nint.push_back(nint);
     const size_t e0 = entry_user.size();
@@ -343,6 +577,49 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
     next_id += nint;
     P.sh_ptr.push_back((int32_t)entry_user.size());
     P.chunk_base.push_back((int32_t)P.chunks.size());
+    if (P.fans) {  // the patch's one record (akb_patch.cuh), offsets in uint16
+      std::vector<int32_t> rowoff(rows + 1, 0);
+      for (int j = 0; j < rows; ++j) {
+        int cnt = 0;  // fans by descending rows: those with row j come first
+        while (cnt < nf && lcl[(size_t)cnt * rows + j] != kNoNode) ++cnt;
+        rowoff[j + 1] = rowoff[j] + cnt;
+      }
+      const int slots = rowoff[rows];
+      auto up8 = [](int x) { return (x + 7) / 8 * 8; };
+      const int o_row = 8, o_node = o_row + up8(rows + 1), o_info = o_node + up8(slots);
+      const int o_ptr = o_info + up8(2 * nf), o_idx = o_ptr + up8(L + 1), o_end = o_idx + up8(slots);
+      if (o_end > 65535 || slots > 65535 || L > 65534)
+        throw std::length_error("fan record above 128 KB");
+      rec.assign(o_end, 0);
+      const int hdr[8] = {nf, rows, o_row, o_node, o_info, o_ptr, o_idx, slots};
+      for (int k = 0; k < 8; ++k) rec[k] = (uint16_t)hdr[k];
+      for (int j = 0; j <= rows; ++j) rec[o_row + j] = (uint16_t)rowoff[j];
+      gbase.assign(L + 1, 0);
+      int32_t ebase = 0;
+      for (int t = 0; t < nf; ++t) {
+        const uint32_t f = unit_order[unit_ptr[p] + t];
+        rec[o_info + 2 * t] = (uint16_t)(F.elems((int)f) | (F.closed[f] ? 0x8000 : 0));
+        rec[o_info + 2 * t + 1] = (uint16_t)ebase;
+        ebase += F.elems((int)f);
+        for (int j = 0; j < F.rows((int)f); ++j) {
+          const uint16_t at = pos[lcl[(size_t)t * rows + j]];
+          rec[o_node + rowoff[j] + t] = at;
+          ++gbase[at + 1];
+        }
+      }
+      for (int j = 0; j < L; ++j) gbase[j + 1] += gbase[j];
+      for (int j = 0; j <= L; ++j) rec[o_ptr + j] = (uint16_t)gbase[j];
+      for (int k = 0; k < slots; ++k)  // a node's contributions by ascending slot
+        rec[o_idx + gbase[rec[o_node + k]]++] = (uint16_t)k;
+      P.contrib_slots = std::max(P.contrib_slots, slots);
+      ChunkDesc cd;
+      cd.off16 = (uint32_t)(P.cdata.size() / 8);
+      cd.bytes = (uint32_t)rec.size() * 2;
+      P.chunks.push_back(cd);
+      P.cdata.insert(P.cdata.end(), rec.begin(), rec.end());
+      P.chunk_bytes = std::max(P.chunk_bytes, (int)cd.bytes);
+      continue;
+    }
     for (int c0 = 0; c0 < ne_p; c0 += kChunk) {
       const int nec = std::min(ne_p - c0, kChunk), ncorner = nec * nnpe;
       // runs: the chunk's corners sorted by (local node, element, corner);
