@@ -248,13 +248,14 @@ akb_status upload(akb_model* m, const std::vector<T>& v, const T** out);
 // fan_cap elements.
 void fan_params(int type, int* target, int* max_nodes, int* fan_cap, int* max_fans) {
   *fan_cap = 8;
-  *max_fans = 128;
-  if (type == AKB_TRIANGLE_3) {
+  if (type == AKB_TRIANGLE_3) {  // a fan per thread of the CTA (FanThreads)
+    *max_fans = 128;
     *target = 768;
     *max_nodes = 500;
   } else {
-    *target = 768;
-    *max_nodes = 320;
+    *max_fans = 256;
+    *target = 1536;
+    *max_nodes = 640;
   }
 }
 
@@ -387,6 +388,7 @@ akb_status build_device_patches(akb_model* m, const PatchHost& P,
   d.npatch = P.npatch;
   d.grid = m->opt_patch_grid > 0 ? m->opt_patch_grid : 0;
   d.max_nodes = P.max_nodes;
+  d.max_interior = P.max_interior;
   d.max_shared = P.max_shared;
   d.node_stride = P.node_stride;
   d.contrib_slots = P.contrib_slots;
@@ -461,16 +463,32 @@ akb_status build_device_patches(akb_model* m, const PatchHost& P,
     std::vector<uint32_t> em(P.elem_order.size());
     for (size_t i = 0; i < em.size(); ++i) em[i] = element_material[P.elem_order[i]];
     if ((st = upload(m, em, &d.emat)) != AKB_OK) return st;
-    if (P.fans) {
-      std::vector<uint32_t> pm(P.npatch);
-      for (int p = 0; p < P.npatch; ++p) {
-        pm[p] = em[P.elem_ptr[p]];
-        for (int32_t i = P.elem_ptr[p]; i < P.elem_ptr[p + 1]; ++i)
-          if (em[i] != pm[p]) pm[p] = kMixed;
-      }
-      if ((st = upload(m, pm, &d.patch_mat)) != AKB_OK) return st;
-    }
     AKB_CUDA_TRY(cudaStreamSynchronize(m->stream));  // host vectors go out of scope
+  }
+  if (P.fans) {
+    std::vector<FanDesc> desc(P.npatch);
+    for (int p = 0; p < P.npatch; ++p) {
+      FanDesc& f = desc[p];
+      f = FanDesc{};
+      f.ibeg = P.ibeg[p];
+      f.nint = P.nint[p];
+      f.s0 = P.sh_ptr[p];
+      f.nsh = P.sh_ptr[p + 1] - P.sh_ptr[p];
+      f.rec_off16 = P.chunks[P.chunk_base[p]].off16;
+      f.rec_bytes = P.chunks[P.chunk_base[p]].bytes;
+      f.elem0 = P.elem_ptr[p];
+      f.inst = batch ? patch_inst[p] : 0;
+      for (int32_t i = P.elem_ptr[p]; element_material && i < P.elem_ptr[p + 1]; ++i) {
+        const uint32_t em = element_material[P.elem_order[i]];
+        f.mat = i == P.elem_ptr[p] || em == f.mat ? em : kMixed;
+        if (f.mat == kMixed) break;
+      }
+    }
+    std::vector<uint2> ent(P.sgid.size());
+    for (size_t t = 0; t < ent.size(); ++t) ent[t] = make_uint2(P.sgid[t], P.sslot[t]);
+    if ((st = upload(m, desc, &d.desc)) != AKB_OK) return st;
+    if ((st = upload(m, ent, &d.entries)) != AKB_OK) return st;
+    AKB_CUDA_TRY(cudaStreamSynchronize(m->stream));
   }
   {
     double* ke;
@@ -497,12 +515,16 @@ akb_status build_device_patches(akb_model* m, const PatchHost& P,
     if ((st = upload(m, li, &d.list_inst)) != AKB_OK) return st;
   }
   AKB_CUDA_TRY(cudaStreamSynchronize(m->stream));  // host vectors go out of scope
-  d.nbuf = P.fans ? 1 : patch_buffers(d, m->dm.type, fp32(m));
-  const size_t smem = P.fans ? fan_smem_bytes(d.max_nodes, d.contrib_slots, d.chunk_bytes, m->dm.dim)
-                             : patch_smem_bytes(d, m->dm.dim, fp32(m), d.nbuf);
-  if (smem > 227 * 1024)
-    return fail(AKB_ERR_UNSUPPORTED, "patch does not fit in shared memory");
-  AKB_CUDA_TRY(patch_configure(m->dm, d, fp32(m)));
+  if (P.fans) {
+    AKB_CUDA_TRY(fan_configure(m->dm, d, m->device, d.resident));
+    if (d.resident[1] < 1) return fail(AKB_ERR_UNSUPPORTED, "patch does not fit in shared memory");
+  } else {
+    d.nbuf = patch_buffers(d, m->dm.type, fp32(m));
+    const size_t smem = patch_smem_bytes(d, m->dm.dim, fp32(m), d.nbuf);
+    if (smem > 227 * 1024)
+      return fail(AKB_ERR_UNSUPPORTED, "patch does not fit in shared memory");
+    AKB_CUDA_TRY(patch_configure(m->dm, d, fp32(m)));
+  }
   m->use_patches = true;
   return AKB_OK;
 }
@@ -772,8 +794,7 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
     bool fans = m->mode == AKB_MODE_FP64 && (type == AKB_TRIANGLE_3 || type == AKB_TETRAHEDRON_4);
     if (fans) {
       st = plan_patches(m.get(), mesh, batch, part, true, plan, patch_inst, orphan_inst);
-      fans = st == AKB_OK && fan_smem_bytes(plan.max_nodes, plan.contrib_slots, plan.chunk_bytes, d) <=
-                                 227 * 1024;
+      fans = st == AKB_OK && fan_smem_bytes(plan, d) <= 227 * 1024;
     }
     if (!fans &&
         (st = plan_patches(m.get(), mesh, batch, part, false, plan, patch_inst, orphan_inst)) != AKB_OK)

@@ -244,6 +244,12 @@ __device__ inline double ke_term(double v, double im) {
   return M > DBL_EPSILON ? v * v * M : 0.0;
 }
 
+// The same of a node from its sum of v^2 (one mass for all components).
+__device__ inline double ke_sum(double v2, double im) {
+  const double M = 1.0 / im;
+  return M > DBL_EPSILON ? v2 * M : 0.0;
+}
+
 // Sum of the CTA's per-thread values in a fixed order (lanes by an xor
 // tree, then warps in order), by thread 0; every thread must call it.
 __device__ inline double cta_sum(double x, double* warp_sums) {
@@ -602,31 +608,44 @@ __global__ void __launch_bounds__(kThreads, (PatchOccupancy<T, S>::value))
 //  - all contributions of the patch stay in shared memory, so that the node
 //    sums run once per patch and feed the finish directly: two barriers a
 //    patch instead of two per 256 elements, and no force accumulators.
-constexpr int kFanThreads = 128;
 
+// Shared memory: X and w of the patch's nodes (row-major, 16 bytes of slack in
+// front), the contributions, the record, the interior nodes' finishing inputs
+// (finish_regions), two buffers of the shared entries (node, partial slot)
+// and three of the patch descriptor, two mbarriers (staging, finishing inputs).
 struct FanLayout {
-  size_t xs, ws, c, rec, mbar, total;
+  size_t xs, ws, c, rec, fin, sh, sh_stride, desc, mbar, total;
 };
-__host__ __device__ inline FanLayout fan_layout(int Lmax, int slots, int rec_bytes, int d) {
+__host__ __device__ inline FanLayout fan_layout(int Lmax, int Imax, int SHmax, int slots,
+                                                int rec_bytes, int d, bool fext) {
   FanLayout s;
   const size_t nb = align16(16 + (size_t)Lmax * d * sizeof(double));
   s.xs = 0;
   s.ws = nb;
   s.c = 2 * nb;
   s.rec = align128(s.c + (size_t)slots * d * sizeof(double));
-  s.mbar = s.rec + align16((size_t)rec_bytes);
+  s.fin = align128(s.rec + (size_t)rec_bytes);
+  // v, a, 1 / M, the flags and f_ext, each rounded out to 16 bytes on both sides
+  s.sh = s.fin + align16((size_t)Imax * ((fext ? 3 : 2) * 8 * d + 8 + d)) + 5 * 32;
+  s.sh_stride = align16((size_t)SHmax * sizeof(uint2));
+  s.desc = s.sh + 2 * s.sh_stride;
+  s.mbar = s.desc + 3 * sizeof(FanDesc);
   s.total = s.mbar + 16;
   return s;
 }
-__host__ __device__ inline FanLayout fan_layout(const DevPatches& p, int d) {
-  return fan_layout(p.max_nodes, p.contrib_slots, p.chunk_bytes, d);
+__host__ __device__ inline FanLayout fan_layout(const DevPatches& p, int d, bool fext) {
+  return fan_layout(p.max_nodes, p.max_interior, p.max_shared, p.contrib_slots, p.chunk_bytes, d,
+                    fext);
 }
 
-// CTAs per SM each instantiation is built for (register budget).
-template <int D, bool LIN> struct FanOccupancy { static constexpr int value = 3; };
-template <> struct FanOccupancy<3, true> { static constexpr int value = 4; };
-template <> struct FanOccupancy<2, true> { static constexpr int value = 6; };
-template <> struct FanOccupancy<2, false> { static constexpr int value = 5; };
+// Threads of a CTA and CTAs per SM each instantiation is built for. A thread
+// computes a fan, so a patch has about as many fans as its CTA has threads:
+// larger patches share fewer nodes, smaller ones overlap their phases better.
+// Tetrahedra at 128 registers (16 warps an SM either way; more spill): 256
+// threads 140.6 us a step on the 6 M-element cube, 128 threads 145.3, 192
+// threads 148.7. Triangles (512 plates): 128 threads 47.9 us, 256 threads 48.4.
+template <int D> struct FanThreads { static constexpr int value = D == 3 ? 256 : 128; };
+template <int D, bool LIN> struct FanOccupancy { static constexpr int value = D == 3 ? 2 : LIN ? 6 : 5; };
 
 // w P of one element from G = det * grad u (row-major), P the Cauchy (small
 // strain) or first Piola stress, w the reference volume of the simplex.
@@ -634,7 +653,7 @@ template <int d, bool LIN>
 __device__ inline void fan_stress(const MatParams& mp, const double* G, double det, double* P) {
   constexpr double w = d == 3 ? 1.0 / 6.0 : 0.5;
   if constexpr (LIN) {
-    const double s = w / det, mu = mp.mu * s;
+    const double s = w * (1.0 / det), mu = mp.mu * s;
     double tr = G[0] + G[d + 1];
     if (d == 3) tr += G[2 * d + 2];
     tr *= mp.lambda * s;
@@ -671,12 +690,14 @@ __device__ __forceinline__ void fan_forces(const uint16_t* rec, int t, const dou
                                            const MatParams* table, const uint32_t* emat) {
   constexpr int H = d - 1;
   const uint16_t* ro = rec + rec[2];
-  const uint16_t* node = rec + rec[3];
+  // per entry: position | slot << 16
+  const uint32_t* node = reinterpret_cast<const uint32_t*>(rec + rec[3]);
   const uint32_t info = reinterpret_cast<const uint32_t*>(rec + rec[4])[t];
   const int k = (int)(info & 0x7fff);
   const bool closed = info & 0x8000;
-  const int ja = node[t], j0 = node[ro[H] + t];
-  double xa[d], ua[d], e1[3], d1[3], e2[d], d2[d], c2[3], fa[d], fb[3], ft[d];
+  const uint32_t first = node[ro[H] + t];  // r_0
+  const int ja = (int)(node[t] & 0xffff);
+  double e1[3], d1[3], e2[d], d2[d], c2[3], fa[d], fb[3], ft[d];
   auto load = [&](int j, double* x, double* u) {
     if constexpr (d == 2) {
       const double2 p = reinterpret_cast<const double2*>(xs)[j];
@@ -693,7 +714,9 @@ __device__ __forceinline__ void fan_forces(const uint16_t* rec, int t, const dou
       }
     }
   };
-  auto edge = [&](int j, double* e, double* u) {
+  auto edge = [&](int j, double* e, double* u) {  // (the hinge re-read: 12 registers less)
+    double xa[d], ua[d];
+    load(ja, xa, ua);
     load(j, e, u);
 #pragma unroll
     for (int i = 0; i < d; ++i) {
@@ -709,19 +732,20 @@ __device__ __forceinline__ void fan_forces(const uint16_t* rec, int t, const dou
       for (int i = 0; i < d; ++i) C[d * s + i] = f[i];
     }
   };
-  load(ja, xa, ua);
-  edge(j0, e2, d2);
+  edge((int)(first & 0xffff), e2, d2);
   if constexpr (d == 3) {
-    edge(node[ro[1] + t], e1, d1);
+    edge((int)(node[ro[1] + t] & 0xffff), e1, d1);
     cross3(e1, e2, c2);
   }
 #pragma unroll
   for (int i = 0; i < d; ++i) fa[i] = ft[i] = 0.0;
 #pragma unroll
   for (int i = 0; i < 3; ++i) fb[i] = 0.0;
-#pragma unroll 1
+  uint32_t at = first;
+#pragma unroll 1  // (the ring node's registers swap roles: no moves)
   for (int s = 0; s < k; ++s) {
-    const int jn = closed && s == k - 1 ? j0 : node[ro[H + 1 + s] + t];
+    const uint32_t next = closed && s == k - 1 ? first : node[ro[H + 1 + s] + t];
+    const int jn = (int)(next & 0xffff);
     const MatParams& mp = emat ? table[emat[(info >> 16) + s]] : mp0;
     double e3[d], d3[d], fn[d], G[d * d], P[d * d];
     edge(jn, e3, d3);
@@ -757,7 +781,8 @@ __device__ __forceinline__ void fan_forces(const uint16_t* rec, int t, const dou
         fn[i] = P[i * 2 + 1] * e2[0] - P[i * 2] * e2[1];
       }
     }
-    store(ro[H + s] + t, ft);
+    store((int)(at >> 16), ft);
+    at = next;
 #pragma unroll
     for (int i = 0; i < d; ++i) {  // the forces of an element add up to zero
       fa[i] -= ft[i];
@@ -772,189 +797,284 @@ __device__ __forceinline__ void fan_forces(const uint16_t* rec, int t, const dou
     if (d == 3) fa[i] -= fb[i];
   }
   if (closed) {  // r_0's contribution, written by this thread above
-    const int s = ro[H] + t;
 #pragma unroll
-    for (int i = 0; i < d; ++i) C[d * s + i] += ft[i];
+    for (int i = 0; i < d; ++i) C[d * (int)(first >> 16) + i] += ft[i];
   } else {
-    store(ro[H + k] + t, ft);
+    store((int)(at >> 16), ft);
   }
-  store(t, fa);
-  if constexpr (d == 3) store(ro[1] + t, fb);
+  store((int)(node[t] >> 16), fa);
+  if constexpr (d == 3) store((int)(node[ro[1] + t] >> 16), fb);
 }
 
-// One patch p, by the whole CTA; stages: patches it staged before (the phase
-// of the mbarrier). Returns false when a bounded wait gave up.
+// A node's d values at position j of a row-major array.
+template <int d>
+__device__ inline void get_row(const double* p, int j, double* x) {
+  if constexpr (d == 2) {
+    const double2 q = reinterpret_cast<const double2*>(p)[j];
+    x[0] = q.x;
+    x[1] = q.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < d; ++i) x[i] = p[d * j + i];
+  }
+}
+template <int d>
+__device__ inline void put_row(double* p, int j, const double* x) {
+  if constexpr (d == 2) {
+    reinterpret_cast<double2*>(p)[j] = make_double2(x[0], x[1]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < d; ++i) p[d * j + i] = x[i];
+  }
+}
+
+// The CTAs stride over the patches (one each when the grid covers them). The
+// staging of a patch needs its descriptor, then its shared entries, then the
+// nodes these name: three dependent trips to memory, so the descriptor is
+// fetched two patches ahead and the shared entries one, and the patch's slices
+// and record are prefetched into L2. What does not change between steps (X,
+// record, entries of the CTA's first patch) is staged before the previous
+// grid in the stream has finished.
 template <int d, bool LIN, bool FEXT>
-__device__ __forceinline__ bool fan_body(const DevModel& m, const DevPatches& P, double dt0, int p,
-                                         unsigned char* smem, uint32_t& stages) {
-  constexpr int T = kFanThreads;
-  const double dt = P.inst_dt ? P.inst_dt[P.patch_inst[p]] : dt0;
-  const int ib = P.ibeg[p], nint = P.nint[p];
-  const int s0 = P.sh_ptr[p], nsh = P.sh_ptr[p + 1] - s0;
-  const FanLayout lay = fan_layout(P, d);
-  // the interior slices of X and w (see patch_body) and the record
-  const size_t row = (size_t)d * sizeof(double);
-  const size_t s_lo = (size_t)ib * row, s_hi = (size_t)(ib + nint) * row;
-  const size_t c_lo = s_lo & ~size_t(15), c_hi = s_hi & ~size_t(15);
-  const int o = (int)((s_lo - c_lo) / sizeof(double));
-  double* xs = reinterpret_cast<double*>(smem + lay.xs) + o;
-  double* ws = reinterpret_cast<double*>(smem + lay.ws) + o;
-  double* C = reinterpret_cast<double*>(smem + lay.c);
-  const uint16_t* rec = reinterpret_cast<const uint16_t*>(smem + lay.rec);
-  const int tid = threadIdx.x;
-  const uint32_t mb = saddr(smem + lay.mbar);
-  if (tid == 0) {
-    // the previous patch's generic-proxy accesses of these buffers (ordered
-    // before this point by the CTA barrier) come before the bulk copies
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    const uint2 cd = __ldg(reinterpret_cast<const uint2*>(&P.chunks[p]));  // off16, bytes
-    const uint32_t bytes = nint > 0 && c_hi > c_lo ? (uint32_t)(c_hi - c_lo) : 0;
-    expect_tx(mb, 2 * bytes + cd.y);
-    bulk_copy(saddr(smem + lay.rec), P.cdata + (size_t)cd.x * 8, cd.y, mb);
-    if (bytes) {
-      bulk_copy(saddr(smem + lay.xs), reinterpret_cast<const char*>(m.X) + c_lo, bytes, mb);
-      bulk_copy(saddr(smem + lay.ws), reinterpret_cast<const char*>(P.w) + c_lo, bytes, mb);
-    }
-    if (nint > 0) {  // inputs of the interior nodes' finish
-      prefetch_l2(m.v, s_lo, s_hi);
-      prefetch_l2(m.a, s_lo, s_hi);
-      prefetch_l2(m.inv_mass, (size_t)ib * 8, (size_t)(ib + nint) * 8);
-      prefetch_l2(m.blocked, (size_t)ib * d, (size_t)(ib + nint) * d);
-      if (FEXT) prefetch_l2(m.fext, s_lo, s_hi);
-    }
-  }
-  if (tid == T - 1 && nint > 0 && c_hi < s_hi && c_hi >= s_lo) {  // the tail double
-    const size_t k = (c_hi - s_lo) / sizeof(double);
-    cp_async8(xs + k, m.X + (size_t)ib * d + k);
-    cp_async8(ws + k, P.w + (size_t)ib * d + k);
-  } else if (tid == T - 1 && nint > 0 && c_hi < s_lo) {  // slice within one 16 bytes
-    for (size_t k = 0; k < (size_t)nint * d; ++k) {
-      cp_async8(xs + k, m.X + (size_t)ib * d + k);
-      cp_async8(ws + k, P.w + (size_t)ib * d + k);
-    }
-  }
-  for (int t = tid; t < nsh; t += T) {
-    const int64_t g = P.sgid[s0 + t];
-    const int j = nint + t;
-    if constexpr (d == 2) {
-      cp_async16(xs + 2 * j, m.X + g * 2);
-      cp_async16(ws + 2 * j, P.w + g * 2);
-    } else {
-#pragma unroll
-      for (int i = 0; i < d; ++i) {
-        cp_async8(xs + d * j + i, m.X + g * d + i);
-        cp_async8(ws + d * j + i, P.w + g * d + i);
-      }
-    }
-  }
-  cp_async_wait_all();
-  {
-    const bool ok = mbar_wait(mb, stages & 1u);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) {
-        atomicExch(P.err, 1);
-        mbar_wait(mb, stages & 1u);
-      }
-      return false;
-    }
-  }
-  ++stages;
-
-  // element forces, one thread per fan
-  {
-    const uint32_t pm = P.patch_mat ? P.patch_mat[p] : 0;
-    const bool mixed = pm == kMixed;
-    const MatParams& mp = P.patch_mat && !mixed ? m.mat_table[pm] : m.mats[0];
-    const uint32_t* emat = mixed ? P.emat + P.elem_ptr[p] : nullptr;
-    const int nf = rec[0];
-    for (int t = tid; t < nf; t += T)
-      fan_forces<d, LIN>(rec, t, xs, ws, C, mp, m.mat_table, emat);
-  }
-
-  // finish: the interior nodes one thread per DOF, contiguous in the global
-  // arrays, their inputs requested before the barrier; then the shared nodes'
-  // partials to their slots (the second pass adds them)
-  const int items = nint * d;
-  double v[kBatch], a[kBatch], im[kBatch], fx[kBatch];
-  uint8_t bl[kBatch];
-  auto request = [&](int base) {
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
-      const int k = base + b * T + tid;
-      if (k < items) {
-        const int64_t q = (int64_t)ib * d + k;
-        bl[b] = m.blocked[q];
-        v[b] = m.v[q];
-        a[b] = m.a[q];
-        im[b] = m.inv_mass[ib + k / d];
-        fx[b] = FEXT ? m.fext[q] : 0.0;
-      }
-    }
-  };
-  request(0);
-  grid_launch_dependents();  // the second pass may start launching (it waits for this grid)
-  __syncthreads();
-  const uint16_t* ptr = rec + rec[5];
-  const uint16_t* idx = rec + rec[6];
-  auto force = [&](int j, int i) {  // minus the sum of the node's contributions
-    double f = 0.0;
-    const int e = ptr[j + 1];
-#pragma unroll 4
-    for (int q = ptr[j]; q < e; ++q) f -= C[d * idx[q] + i];
-    return f;
-  };
-  double ke = 0.0;  // M v^2 of this thread's DOFs after the step
-  for (int base = 0; base < items; base += T * kBatch) {
-    if (base > 0) request(base);
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
-      const int k = base + b * T + tid;
-      if (k >= items) continue;
-      if (!bl[b]) {  // blocked DOFs keep u, v, a (and w = u)
-        const int j = k / d, i = k - j * d;
-        const int64_t q = (int64_t)ib * d + k;
-        const double f = force(j, i);
-        double u, wn;
-        finish_dof(dt, FEXT ? f + fx[b] : f, im[b], ws[k], v[b], a[b], u, wn);
-        m.u[q] = u;
-        m.v[q] = v[b];
-        m.a[q] = a[b];
-        P.w[q] = wn;
-      }
-      ke += ke_term(v[b], im[b]);
-    }
-  }
-  for (int k = tid; k < nsh * d; k += T) {
-    const int t = k / d, i = k - t * d;
-    P.partial[(size_t)P.sslot[s0 + t] * d + i] = force(nint + t, i);
-  }
-  if (P.ke_part) {
-    __shared__ double warp_sums[T / 32];
-    const double s = cta_sum(ke, warp_sums);
-    if (tid == 0) P.ke_part[p] = s;
-  }
-  return true;
-}
-
-template <int d, bool LIN, bool FEXT, bool PERSIST>
-__global__ void __launch_bounds__(kFanThreads, (FanOccupancy<d, LIN>::value))
+__global__ void __launch_bounds__(FanThreads<d>::value, (FanOccupancy<d, LIN>::value))
     k_fan_step(DevModel m, DevPatches P, double dt0) {
   extern __shared__ __align__(128) unsigned char smem[];
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(smem + fan_layout(P, d).mbar))
-                 : "memory");
+  constexpr int T = FanThreads<d>::value;
+  __shared__ double warp_sums[T / 32];
+  const FanLayout lay = fan_layout(P, d, FEXT);
+  const int tid = threadIdx.x, G = gridDim.x;
+  const uint32_t mb = saddr(smem + lay.mbar);
+  FanDesc* descs = reinterpret_cast<FanDesc*>(smem + lay.desc);
+  double* C = reinterpret_cast<double*>(smem + lay.c);
+  const uint16_t* rec = reinterpret_cast<const uint16_t*>(smem + lay.rec);
+  auto entries = [&](int it) {
+    return reinterpret_cast<uint2*>(smem + lay.sh + (it & 1) * lay.sh_stride);
+  };
+  auto fetch_desc = [&](int p, int b) {
+    if (p < P.npatch && tid < (int)(sizeof(FanDesc) / 16))
+      cp_async16(reinterpret_cast<char*>(descs + b) + 16 * tid,
+                 reinterpret_cast<const char*>(P.desc + p) + 16 * tid);
+  };
+  auto fetch_entries = [&](int s0, int nsh, int it) {
+    uint2* e = entries(it);
+    for (int t = tid; t < nsh; t += T) cp_async8(e + t, P.entries + s0 + t);
+  };
+  if (tid == 0) {
+    for (int b = 0; b < 2; ++b)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb + 8 * b) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  fetch_desc(blockIdx.x, 0);
+  fetch_desc(blockIdx.x + G, 1);
+  cp_async_wait_all();
   __syncthreads();
-  grid_wait();  // the previous step's (or update's) writes of w, v, a, u
-  uint32_t stages = 0;
-  if constexpr (PERSIST) {
-    for (int p = blockIdx.x; p < P.npatch; p += gridDim.x) {
-      if (p != (int)blockIdx.x) __syncthreads();  // shared memory of the previous patch is free
-      if (!fan_body<d, LIN, FEXT>(m, P, dt0, p, smem, stages)) return;
+  fetch_entries(descs[0].s0, descs[0].nsh, 0);
+  cp_async_wait_all();
+  __syncthreads();
+  int it = 0;
+  constexpr size_t row = (size_t)d * sizeof(double);
+  // the offset in doubles of an interior slice behind its 16-byte boundary
+  auto offset = [](int ib) { return d == 3 ? (int)(ib & 1) : 0; };
+  auto nodes = [&](size_t at, int ib) { return reinterpret_cast<double*>(smem + at) + offset(ib); };
+  int cur = 0;  // the current descriptor's buffer
+  for (int p = blockIdx.x; p < P.npatch; p += G, ++it, cur = cur == 2 ? 0 : cur + 1) {
+    // each phase reads the descriptor again: few registers live across the
+    // element loop
+    {  // 1. staging
+      const FanDesc D = descs[cur];
+      const int ib = D.ibeg, nint = D.nint, nsh = D.nsh;
+      const uint2* ent = entries(it);
+      // the interior slices of X and w (see patch_body) and the record
+      const size_t s_lo = (size_t)ib * row, s_hi = s_lo + nint * row;
+      const size_t c_lo = s_lo & ~size_t(15), c_hi = s_hi & ~size_t(15);
+      const uint32_t slice = nint > 0 && c_hi > c_lo ? (uint32_t)(c_hi - c_lo) : 0;
+      // the doubles of a slice past its last whole 16 bytes, and the shared nodes
+      auto gather = [&](double* to, const double* from) {
+        if (d == 3 && tid == T - 1 && nint > 0)
+          for (size_t k = slice ? (c_hi - s_lo) / sizeof(double) : 0; k < (size_t)nint * d; ++k)
+            cp_async8(to + k, from + (size_t)ib * d + k);
+        for (int t = tid; t < nsh; t += T) {
+          const int64_t g = ent[t].x;
+          const int j = nint + t;
+          if constexpr (d == 2) {
+            cp_async16(to + 2 * j, from + g * 2);
+          } else {
+#pragma unroll
+            for (int i = 0; i < d; ++i) cp_async8(to + d * j + i, from + g * d + i);
+          }
+        }
+      };
+      if (tid == 0) {
+        // the previous patch's generic-proxy accesses of these buffers (ordered
+        // before this point by the CTA barrier) come before the bulk copies
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        expect_tx(mb, 2 * slice + D.rec_bytes);
+        bulk_copy(saddr(rec), P.cdata + (size_t)D.rec_off16 * 8, D.rec_bytes, mb);
+        if (slice)
+          bulk_copy(saddr(smem + lay.xs), reinterpret_cast<const char*>(m.X) + c_lo, slice, mb);
+      }
+      gather(nodes(lay.xs, ib), m.X);
+      if (it == 0) grid_wait();  // the previous step's (or update's) writes of w, v, a, u
+      if (tid == 0) {
+        if (slice)
+          bulk_copy(saddr(smem + lay.ws), reinterpret_cast<const char*>(P.w) + c_lo, slice, mb);
+        if (nint > 0) {  // inputs of the interior nodes' finish
+          const void* src[5] = {m.v, m.a, m.inv_mass, m.blocked, m.fext};
+          uint32_t off[5], lo[5], nbytes[5];
+          expect_tx(mb + 8, finish_regions<d, FEXT>(ib, nint, off, lo, nbytes));
+          uint32_t at = saddr(smem + lay.fin);
+#pragma unroll
+          for (int k = 0; k < (FEXT ? 5 : 4); ++k) {
+            bulk_copy(at, reinterpret_cast<const char*>(src[k]) + lo[k], nbytes[k], mb + 8);
+            at += nbytes[k];
+          }
+        } else {
+          arrive(mb + 8);
+        }
+      }
+      gather(nodes(lay.ws, ib), P.w);
+      cp_async_wait_all();
+      const bool ok = mbar_wait(mb, it & 1);
+      if (__syncthreads_or(!ok)) {
+        if (tid == 0) {
+          atomicExch(P.err, 1);
+          mbar_wait(mb, it & 1);
+          mbar_wait(mb + 8, it & 1);
+        }
+        return;
+      }
     }
-  } else {
-    fan_body<d, LIN, FEXT>(m, P, dt0, blockIdx.x, smem, stages);
+    if (p + G < P.npatch) {
+      // ahead: the descriptor two patches on, the next patch's entries, its
+      // slices and record to L2
+      const FanDesc& N = descs[cur == 2 ? 0 : cur + 1];
+      fetch_entries(N.s0, N.nsh, it + 1);
+      if (tid == 0) {
+        const size_t lo = (size_t)N.ibeg * row, hi = lo + N.nint * row;
+        prefetch_l2(P.cdata, (size_t)N.rec_off16 * 16, (size_t)N.rec_off16 * 16 + N.rec_bytes);
+        if (N.nint > 0) {
+          prefetch_l2(m.X, lo, hi);
+          prefetch_l2(P.w, lo, hi);
+          prefetch_l2(m.v, lo, hi);
+          prefetch_l2(m.a, lo, hi);
+        }
+      }
+      fetch_desc(p + 2 * G, cur == 0 ? 2 : cur - 1);
+    }
+    {  // 2. element forces, one thread per fan
+      const FanDesc& D = descs[cur];
+      const bool mixed = D.mat == kMixed;
+      const MatParams& mp = P.emat && !mixed ? m.mat_table[D.mat] : m.mats[0];
+      const uint32_t* emat = mixed ? P.emat + D.elem0 : nullptr;
+      const double *xs = nodes(lay.xs, D.ibeg), *ws = nodes(lay.ws, D.ibeg);
+      const int nf = rec[0];
+      for (int t = tid; t < nf; t += T)
+        fan_forces<d, LIN>(rec, t, xs, ws, C, mp, m.mat_table, emat);
+    }
+    {
+      const bool ok = mbar_wait(mb + 8, it & 1);  // finishing inputs
+      if (__syncthreads_or(!ok)) {
+        cp_async_wait_all();
+        if (tid == 0) {
+          atomicExch(P.err, 1);
+          mbar_wait(mb + 8, it & 1);
+        }
+        return;
+      }
+    }
+    // the second pass may start launching (it waits for this grid)
+    if (p + G >= P.npatch) grid_launch_dependents();
+    asm volatile("" ::: "memory");
+    // 3. finish, one thread per node, all of it in shared memory: an interior
+    // node's v and a are updated where they were staged, its u is this step's w
+    // (finish_dof) where w was staged, its next w takes X's place, and the four
+    // slices go out by bulk copies (blocked DOFs as they were: w = u there). A
+    // shared node's partial goes to its slot (the second pass adds them).
+    const FanDesc D = descs[cur];
+    const int ib = D.ibeg, nint = D.nint, nsh = D.nsh;
+    const double dt = P.inst_dt ? P.inst_dt[D.inst] : dt0;
+    const uint2* ent = entries(it);
+    const uint16_t* cnt = rec + rec[5];
+    const uint16_t* goff = rec + rec[6];
+    uint32_t off[5];
+    {
+      uint32_t lo[5], nbytes[5];
+      finish_regions<d, FEXT>(ib, nint, off, lo, nbytes);
+    }
+    unsigned char* fin = smem + lay.fin;
+    double* xs = nodes(lay.xs, ib);
+    double* ws = nodes(lay.ws, ib);
+    double* vs = reinterpret_cast<double*>(fin + off[0]);
+    double* as = reinterpret_cast<double*>(fin + off[1]);
+    const double* ims = reinterpret_cast<const double*>(fin + off[2]);
+    const double* fxs = reinterpret_cast<const double*>(fin + off[4]);
+    double ke = 0.0;  // M v^2 of this thread's DOFs after the step
+    for (int j = tid; j < nint + nsh; j += T) {
+      double f[d];
+#pragma unroll
+      for (int i = 0; i < d; ++i) f[i] = 0.0;
+      const int n = cnt[j];
+      const uint16_t* ix = rec + goff[j >> 5] + (j & 31);
+#pragma unroll 2
+      for (int q = 0; q < n; ++q) {
+        double c[d];
+        get_row<d>(C, ix[32 * q], c);
+#pragma unroll
+        for (int i = 0; i < d; ++i) f[i] -= c[i];
+      }
+      if (j < nint) {
+        const double im = ims[j];
+        double w[d], v[d], a[d], u[d], wn[d], v2 = 0.0;
+        get_row<d>(ws, j, w);
+        get_row<d>(vs, j, v);
+        get_row<d>(as, j, a);
+#pragma unroll
+        for (int i = 0; i < d; ++i) {
+          u[i] = wn[i] = w[i];
+          if (!fin[off[3] + d * j + i])
+            finish_dof(dt, FEXT ? f[i] + fxs[d * j + i] : f[i], im, w[i], v[i], a[i], u[i], wn[i]);
+          v2 += v[i] * v[i];
+        }
+        put_row<d>(vs, j, v);
+        put_row<d>(as, j, a);
+        put_row<d>(xs, j, wn);
+#pragma unroll
+        for (int i = 0; i < d; ++i)
+          if (!(u[i] == w[i])) ws[d * j + i] = u[i];  // only where u is not finite
+        ke += ke_sum(v2, im);
+      } else {
+        put_row<d>(P.partial, (int)ent[j - nint].y, f);
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the bulk copies read
+    const double s = cta_sum(ke, warp_sums);  // (also the barrier before the copies)
+    if (tid == 0 && P.ke_part) P.ke_part[p] = s;
+    // the slices' whole 16-byte units by bulk copies, the double before or after
+    // them by itself
+    const size_t s_lo = (size_t)ib * row, s_hi = s_lo + nint * row;
+    const size_t b_lo = (s_lo + 15) & ~size_t(15), b_hi = s_hi & ~size_t(15);
+    double* const dst[4] = {m.u, m.v, m.a, P.w};
+    const double* const src[4] = {ws, vs, as, xs};
+    if (tid == 0 && b_hi > b_lo) {
+      const size_t at = (b_lo - s_lo) / sizeof(double);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
+                         reinterpret_cast<char*>(dst[k]) + b_lo),
+                     "r"(saddr(src[k] + at)), "r"((uint32_t)(b_hi - b_lo))
+                     : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    } else if (d == 3 && tid >= 32 && tid < 40 && nint > 0) {
+      const int k = (tid - 32) & 3;
+      const size_t q = tid < 36 ? s_lo : s_hi - 8;  // the slice's first and last double
+      if ((tid < 36 && b_lo > s_lo) || (tid >= 36 && b_hi < s_hi))
+        dst[k][q / sizeof(double)] = src[k][(q - s_lo) / sizeof(double)];
+    }
+    if (p + G < P.npatch) {
+      cp_async_wait_all();  // the entries and the descriptor ahead
+      __syncthreads();      // shared memory of this patch is free
+    }
   }
 }
 
@@ -1198,32 +1318,39 @@ cudaError_t raise_smem_limit(K kernel, size_t bytes) {
 
 // f(kernel) for the fan step's instantiation of a plan.
 template <int d, typename F>
-cudaError_t with_fan_kernel(bool lin, bool fext, bool persist, F f) {
-  if (lin)
-    return fext ? (persist ? f(k_fan_step<d, true, true, true>) : f(k_fan_step<d, true, true, false>))
-                : (persist ? f(k_fan_step<d, true, false, true>) : f(k_fan_step<d, true, false, false>));
-  return fext ? (persist ? f(k_fan_step<d, false, true, true>) : f(k_fan_step<d, false, true, false>))
-              : (persist ? f(k_fan_step<d, false, false, true>) : f(k_fan_step<d, false, false, false>));
+cudaError_t with_fan_kernel(bool lin, bool fext, F f) {
+  if (lin) return fext ? f(k_fan_step<d, true, true>) : f(k_fan_step<d, true, false>);
+  return fext ? f(k_fan_step<d, false, true>) : f(k_fan_step<d, false, false>);
 }
 
 template <int d>
 cudaError_t launch_fan(const DevModel& m, const DevPatches& p, double dt, bool fext, cudaStream_t s) {
-  const int grid = grid_of(p);
-  const size_t bytes = fan_layout(p, d).total;
-  return with_fan_kernel<d>(p.linear, fext, grid < p.npatch, [&](auto kernel) {
-    return launch_pdl(kernel, grid, kFanThreads, bytes, s, m, p, dt);
+  const size_t bytes = fan_layout(p, d, fext).total;
+  return with_fan_kernel<d>(p.linear, fext, [&](auto kernel) {
+    const int grid = p.grid > 0 ? p.grid : p.resident[fext];
+    return launch_pdl(kernel, std::min(grid, p.npatch), FanThreads<d>::value, bytes, s, m, p, dt);
   });
 }
 
+// Raises the kernels' shared-memory limit; resident: CTAs of the plan that are
+// on the device at the same time, without and with external forces.
 template <int d>
-cudaError_t configure_fan(const DevPatches& p) {
-  const size_t bytes = fan_layout(p, d).total;
+cudaError_t configure_fan(const DevPatches& p, int device, int* resident) {
+  int sms = 0, per_sm = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(g_attr_mutex);
-  for (int k = 0; k < 4; ++k) {
-    const cudaError_t e = with_fan_kernel<d>(p.linear, k & 1, k & 2, [&](auto kernel) {
-      return raise_smem_limit(kernel, bytes);
+  for (int k = 0; k < 2; ++k) {
+    const size_t bytes = fan_layout(p, d, k).total;
+    e = with_fan_kernel<d>(p.linear, k, [&](auto kernel) {
+      cudaError_t r = raise_smem_limit(kernel, bytes);
+      return r != cudaSuccess
+                 ? r
+                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel,
+                                                                 FanThreads<d>::value, bytes);
     });
     if (e != cudaSuccess) return e;
+    resident[k] = sms * per_sm;
   }
   return cudaSuccess;
 }
@@ -1245,8 +1372,13 @@ size_t patch_smem_bytes(const DevPatches& p, int dim, bool fp32, int nbuf) {
   return layout(p, dim, fp32 ? 4 : 8, nbuf).total;
 }
 
-size_t fan_smem_bytes(int max_nodes, int slots, int record_bytes, int dim) {
-  return fan_layout(max_nodes, slots, record_bytes, dim).total;
+size_t fan_smem_bytes(const PatchHost& p, int dim) {
+  return fan_layout(p.max_nodes, p.max_interior, p.max_shared, p.contrib_slots, p.chunk_bytes, dim,
+                    true).total;
+}
+
+cudaError_t fan_configure(const DevModel& m, const DevPatches& p, int device, int* resident) {
+  return m.dim == 2 ? configure_fan<2>(p, device, resident) : configure_fan<3>(p, device, resident);
 }
 
 int patch_buffers(const DevPatches& p, int type, bool fp32) {
@@ -1272,7 +1404,6 @@ int patch_buffers(const DevPatches& p, int type, bool fp32) {
 }
 
 cudaError_t patch_configure(const DevModel& m, const DevPatches& p, bool fp32) {
-  if (p.fans) return m.dim == 2 ? configure_fan<2>(p) : configure_fan<3>(p);
   switch (m.type) {
   case AKB_SEGMENT_2: return fp32 ? configure<AKB_SEGMENT_2, float>(p) : configure<AKB_SEGMENT_2, double>(p);
   case AKB_TRIANGLE_3: return fp32 ? configure<AKB_TRIANGLE_3, float>(p) : configure<AKB_TRIANGLE_3, double>(p);

@@ -85,15 +85,19 @@ inline int place_group(int dim) { return dim == 2 ? 8 : 16; }
 // writing one contribution per node, so that a fan of six tetrahedra loads 8
 // nodes and writes 8 contributions instead of 24 and 24. Contents (uint16,
 // every section on 16 bytes, offsets in uint16 units):
-//   header   nf, rows, o_row, o_node, o_info, o_ptr, o_idx, slots
-//   rowoff   rows + 1: first slot of row j (row j: node j of the fans that
+//   header   nf, rows, o_row, o_node, o_info, o_cnt, o_goff, slots
+//   rowoff   rows + 1: first entry of row j (row j: node j of the fans that
 //            have one, hinge first; fans by descending row count)
-//   node     slots: the position of the node of slot rowoff[j] + t (row j of
-//            fan t), which is also where its contribution goes
+//   node     per entry rowoff[j] + t (row j of fan t): its node's position, its
+//            contribution's slot
 //   info     per fan: elements | 0x8000 if the ring closes (the last element
 //            ends on r_0, whose contribution it adds to), first element of
 //            the fan within the patch
-//   ptr, idx per position its contribution slots idx[ptr[j] .. ptr[j + 1])
+//   cnt      per position the number of its contributions
+//   goff     per 32 positions, where their list starts in the record: entry q
+//            of position 32 g + l at goff[g] + 32 q + l
+// The slots are a colouring as the chunk records', 16 colours in 3D and 8 in 2D
+// (16-byte rows): scatter and sum are free of bank conflicts.
 // Partial slot of rank r of shared node s (ns shared nodes; over: the node's
 // first slot for ranks >= 2).
 __host__ __device__ inline uint32_t partial_slot(uint32_t ns, uint32_t s, uint32_t over,
@@ -150,8 +154,20 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
                         const uint8_t* force_shared = nullptr, int fan_cap = 0,
                         int max_fans = 0);
 
-// patch_mat of a patch with several materials
+// FanDesc::mat of a patch with several materials
 constexpr uint32_t kMixed = 0xffffffffu;
+
+// What k_fan_step needs to know to stage a patch, in one place (three 16-byte
+// loads).
+struct FanDesc {
+  int32_t ibeg, nint;    // interior nodes
+  int32_t s0, nsh;       // shared entries
+  uint32_t rec_off16, rec_bytes;
+  uint32_t mat;          // the patch's only material, or kMixed
+  uint32_t inst;         // batches: its instance
+  int32_t elem0;         // its first element in patch order
+  uint32_t pad[3];
+};
 
 // Device copy of a PatchHost.
 struct DevPatches {
@@ -159,8 +175,9 @@ struct DevPatches {
   int linear;  // fans: every material is small-strain elastic
   int npatch;
   int grid;  // 0: one CTA per patch; > 0: persistent grid of that many CTAs
+  int resident[2];  // fans, grid 0: CTAs on the device at once (without, with f_ext)
   int nbuf;  // chunk record buffers in shared memory (2: next chunk prefetched)
-  int max_nodes, max_shared, node_stride, contrib_slots, max_runs, chunk_bytes;
+  int max_nodes, max_interior, max_shared, node_stride, contrib_slots, max_runs, chunk_bytes;
   const int32_t* elem_ptr;
   const int32_t* ibeg;
   const int32_t* nint;
@@ -171,7 +188,8 @@ struct DevPatches {
   const uint2* chunks;     // ChunkDesc per chunk
   const uint16_t* cdata;   // chunk records (16-byte aligned)
   const uint32_t* emat;    // material of each patch-ordered element, or null
-  const uint32_t* patch_mat;  // fans: a patch's only material, kMixed, or null (one material)
+  const FanDesc* desc;     // fans: per patch
+  const uint2* entries;    // fans: per shared entry, its node and partial slot
   int* err;                // set when a bounded wait gave up
   double* partial;         // nslots x dim
   double* w;               // nn x dim predicted displacement
@@ -205,8 +223,10 @@ struct DevPatches {
 void assign_partial_slots(PatchHost& P, int64_t nn);
 
 size_t patch_smem_bytes(const DevPatches& p, int dim, bool fp32, int nbuf);
-// Shared memory of k_fan_step for a plan.
-size_t fan_smem_bytes(int max_nodes, int slots, int record_bytes, int dim);
+// Shared memory of k_fan_step for a plan; its configuration on the device
+// (resident[2]: its CTAs that run at the same time, without and with f_ext).
+size_t fan_smem_bytes(const PatchHost& p, int dim);
+cudaError_t fan_configure(const DevModel& m, const DevPatches& p, int device, int* resident);
 // Chunk record buffers (1 or 2) that keep the most CTAs per SM.
 int patch_buffers(const DevPatches& p, int type, bool fp32);
 cudaError_t patch_configure(const DevModel& m, const DevPatches& p, bool fp32);

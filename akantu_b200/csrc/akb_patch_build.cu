@@ -553,8 +553,15 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
           ++uses[v];
         }
       }
-      std::iota(first.begin(), first.end(), 0);
-      std::stable_sort(first.begin(), first.end(), [&](int32_t x, int32_t y) { return uses[x] > uses[y]; });
+      first.clear();
+      for (int j = 0; j < rows; ++j)  // in the order the groups of fans reach them
+        for (int t = 0; t < nf; ++t) {
+          const uint16_t v = lcl[(size_t)t * rows + j];
+          if (v == kNoNode || uses[v] < 0) continue;
+          first.push_back(v);
+          uses[v] = -uses[v];
+        }
+      std::stable_sort(first.begin(), first.end(), [&](int32_t x, int32_t y) { return uses[x] < uses[y]; });
       place_nodes(lcl, nf, rows, L, nint, GP, pos.data(), &first);
     } else {
       place_nodes(lcl, ne_p, nnpe, L, nint, GP, pos.data());
@@ -584,17 +591,55 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
         while (cnt < nf && lcl[(size_t)cnt * rows + j] != kNoNode) ++cnt;
         rowoff[j + 1] = rowoff[j] + cnt;
       }
-      const int slots = rowoff[rows];
+      const int entries = rowoff[rows];
+      if (entries > 65535) throw std::length_error("fan record above 128 KB");
       auto up8 = [](int x) { return (x + 7) / 8 * 8; };
-      const int o_row = 8, o_node = o_row + up8(rows + 1), o_info = o_node + up8(slots);
-      const int o_ptr = o_info + up8(2 * nf), o_idx = o_ptr + up8(L + 1), o_end = o_idx + up8(slots);
+      // the entries (row j of fan t) of each position, in ascending order
+      std::vector<std::vector<uint16_t>> of(L);
+      for (int j = 0; j < rows; ++j)
+        for (int t = 0; t < rowoff[j + 1] - rowoff[j]; ++t)
+          of[pos[lcl[(size_t)t * rows + j]]].push_back((uint16_t)(rowoff[j] + t));
+      const int ng = (L + 31) / 32;
+      gbase.assign(ng + 1, 0);
+      int most = 0;
+      for (int g = 0; g < ng; ++g) {
+        size_t n = 0;
+        for (int j = 32 * g; j < std::min(L, 32 * g + 32); ++j) n = std::max(n, of[j].size());
+        gbase[g + 1] = gbase[g] + 32 * (int)n;
+        most = std::max(most, (int)n);
+      }
+      // the entries' contribution slots: the colours of the graph of scatter
+      // instructions (row j of GP fans) and sum instructions (entry q of GP
+      // positions), as for the chunk records, so that both hit GP banks
+      const int nsg = (nf + GP - 1) / GP;
+      BipartiteColouring bc(nsg * rows, std::max((L + GP - 1) / GP * most, 1), GP);
+      eslot.assign(entries, 0);
+      cls.assign(GP, 0);
+      {
+        std::vector<int32_t> edge_of(entries);
+        int ne_ = 0, j = 0;
+        for (int k = 0; k < L; ++k)
+          for (size_t q = 0; q < of[k].size(); ++q) {
+            const int e = of[k][q];
+            for (j = 0; e >= rowoff[j + 1];) ++j;
+            bc.add(j * nsg + (e - rowoff[j]) / GP, k / GP * most + (int)q);
+            edge_of[e] = ne_++;
+          }
+        for (int e = 0; e < entries; ++e) {
+          const int c = bc.colour(edge_of[e]);
+          eslot[e] = c + GP * cls[c]++;
+        }
+      }
+      const int slots = GP * *std::max_element(cls.begin(), cls.end());
+      const int o_row = 8, o_node = o_row + up8(rows + 1), o_info = o_node + up8(2 * entries);
+      const int o_cnt = o_info + up8(2 * nf), o_goff = o_cnt + up8(L), o_idx = o_goff + up8(ng);
+      const int64_t o_end = o_idx + up8(gbase[ng]);
       if (o_end > 65535 || slots > 65535 || L > 65534)
         throw std::length_error("fan record above 128 KB");
       rec.assign(o_end, 0);
-      const int hdr[8] = {nf, rows, o_row, o_node, o_info, o_ptr, o_idx, slots};
+      const int hdr[8] = {nf, rows, o_row, o_node, o_info, o_cnt, o_goff, slots};
       for (int k = 0; k < 8; ++k) rec[k] = (uint16_t)hdr[k];
       for (int j = 0; j <= rows; ++j) rec[o_row + j] = (uint16_t)rowoff[j];
-      gbase.assign(L + 1, 0);
       int32_t ebase = 0;
       for (int t = 0; t < nf; ++t) {
         const uint32_t f = unit_order[unit_ptr[p] + t];
@@ -602,15 +647,16 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
         rec[o_info + 2 * t + 1] = (uint16_t)ebase;
         ebase += F.elems((int)f);
         for (int j = 0; j < F.rows((int)f); ++j) {
-          const uint16_t at = pos[lcl[(size_t)t * rows + j]];
-          rec[o_node + rowoff[j] + t] = at;
-          ++gbase[at + 1];
+          rec[o_node + 2 * (rowoff[j] + t)] = pos[lcl[(size_t)t * rows + j]];
+          rec[o_node + 2 * (rowoff[j] + t) + 1] = (uint16_t)eslot[rowoff[j] + t];
         }
       }
-      for (int j = 0; j < L; ++j) gbase[j + 1] += gbase[j];
-      for (int j = 0; j <= L; ++j) rec[o_ptr + j] = (uint16_t)gbase[j];
-      for (int k = 0; k < slots; ++k)  // a node's contributions by ascending slot
-        rec[o_idx + gbase[rec[o_node + k]]++] = (uint16_t)k;
+      for (int j = 0; j < L; ++j) {
+        rec[o_cnt + j] = (uint16_t)of[j].size();
+        for (size_t q = 0; q < of[j].size(); ++q)
+          rec[o_idx + gbase[j / 32] + 32 * q + j % 32] = (uint16_t)eslot[of[j][q]];
+      }
+      for (int g = 0; g < ng; ++g) rec[o_goff + g] = (uint16_t)(o_idx + gbase[g]);
       P.contrib_slots = std::max(P.contrib_slots, slots);
       ChunkDesc cd;
       cd.off16 = (uint32_t)(P.cdata.size() / 8);

@@ -117,15 +117,16 @@ void check(const char* name, const Mesh& m, int target, int maxn, int cap, int m
     CHECK((size_t)cd.off16 * 8 + cd.bytes / 2 <= P.cdata.size());
     const uint16_t* rec = &P.cdata[(size_t)cd.off16 * 8];
     const int end = (int)cd.bytes / 2, nf = rec[0], rows = rec[1], slots = rec[7];
-    const uint16_t *ro = rec + rec[2], *node = rec + rec[3], *info = rec + rec[4], *ptr = rec + rec[5],
-                   *idx = rec + rec[6];
-    CHECK(rec[2] >= 8 && rec[2] + rows + 1 <= rec[3] && rec[3] + slots <= rec[4]);
-    CHECK(rec[4] + 2 * nf <= rec[5] && rec[5] + L + 1 <= rec[6] && rec[6] + slots <= end);
-    CHECK(slots <= P.contrib_slots && rows <= H + 1 + cap && ro[0] == 0 && ro[rows] == slots);
-    CHECK(rec[4] % 2 == 0);  // info is read as 32-bit words
+    const uint16_t *ro = rec + rec[2], *node = rec + rec[3], *info = rec + rec[4], *cnt = rec + rec[5],
+                   *goff = rec + rec[6];
+    const int entries = ro[rows];
+    CHECK(rec[2] >= 8 && rec[2] + rows + 1 <= rec[3] && rec[3] + 2 * entries <= rec[4]);
+    CHECK(rec[4] + 2 * nf <= rec[5] && rec[5] + L <= rec[6] && rec[6] + (L + 31) / 32 <= end);
+    CHECK(slots <= P.contrib_slots && rows <= H + 1 + cap && ro[0] == 0 && entries <= slots);
+    CHECK(rec[3] % 2 == 0 && rec[4] % 2 == 0);  // read as 32-bit words
     CHECK(nf <= max_fans || nf == 1);
     nfans += nf;
-    std::vector<int> written(slots, 0);
+    std::vector<int> written(slots, -1);  // the position each slot belongs to
     int next = 0;
     for (int t = 0; t < nf; ++t) {
       const int k = info[2 * t] & 0x7fff, closed = info[2 * t] >> 15;
@@ -136,10 +137,10 @@ void check(const char* name, const Mesh& m, int target, int maxn, int cap, int m
       std::vector<int64_t> id(r);
       for (int j = 0; j < r; ++j) {
         CHECK(t < ro[j + 1] - ro[j]);
-        const int s = ro[j] + t;
-        CHECK(s < slots && node[s] < L);
-        written[s]++;
-        id[j] = node[s] < nint ? (int64_t)P.ibeg[p] + node[s] : (int64_t)P.sgid[s0 + node[s] - nint];
+        const int e = ro[j] + t, at = node[2 * e], s = node[2 * e + 1];
+        CHECK(e < entries && s < slots && at < L && written[s] < 0);
+        if (s < slots) written[s] = at;
+        id[j] = at < nint ? (int64_t)P.ibeg[p] + at : (int64_t)P.sgid[s0 + at - nint];
       }
       for (int s = 0; s < k; ++s) {  // the element: an even permutation of its own nodes
         const uint32_t e = P.elem_order[eb + info[2 * t + 1] + s];
@@ -162,17 +163,19 @@ void check(const char* name, const Mesh& m, int target, int maxn, int cap, int m
       }
     }
     CHECK(next == nep);
-    for (int s = 0; s < slots; ++s) CHECK(written[s] == 1);
     std::vector<int> read(slots, 0);
-    CHECK(ptr[0] == 0 && ptr[L] == slots);
-    for (int j = 0; j < L; ++j) {
-      CHECK(ptr[j] <= ptr[j + 1]);
-      for (int q = ptr[j]; q < ptr[j + 1]; ++q) {
-        CHECK(idx[q] < slots && node[idx[q]] == j);
-        if (idx[q] < slots) read[idx[q]]++;
+    for (int j = 0; j < L; ++j)
+      for (int q = 0; q < cnt[j]; ++q) {
+        const int at = goff[j / 32] + 32 * q + j % 32;
+        CHECK(at >= rec[6] + (L + 31) / 32 && at < end);
+        if (at >= end) continue;
+        CHECK(rec[at] < slots);
+        if (rec[at] < slots) {
+          CHECK(written[rec[at]] == j);
+          read[rec[at]]++;
+        }
       }
-    }
-    for (int s = 0; s < slots; ++s) CHECK(read[s] == 1);
+    for (int s = 0; s < slots; ++s) CHECK(read[s] == (written[s] >= 0));
   }
   p = -1;
   for (int64_t e = 0; e < ne; ++e) CHECK(seen[e] == 1);
