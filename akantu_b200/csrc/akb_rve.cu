@@ -25,6 +25,7 @@
 #include <cmath>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/akb_fe2.h"
@@ -176,6 +177,113 @@ __device__ inline void voxel_stress(const MatParams& mp, const S* g, S* P) {
     }
 }
 
+// The same in FP32 with every rounding spelled out (which product of a sum of
+// products is fused is the compiler's choice otherwise, and differs from kernel
+// to kernel): all kernels that relax FP32 RVEs agree bit for bit.
+__device__ __forceinline__ void voxel_stress_f32(const MatParams& mp, const float* g, float* P) {
+  const float lam = float(mp.lambda), mu = float(mp.mu);
+  if (mp.kind != AKB_MATERIAL_NEOHOOKEAN) {
+    const float lt = __fmul_rn(lam, g[0] + g[4] + g[8]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        P[i * 3 + j] = __fmaf_rn(mu, g[i * 3 + j] + g[j * 3 + i], i == j ? lt : 0.0f);
+    return;
+  }
+  float gg[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const float x = __fmaf_rn(g[i * 3], g[j], __fmul_rn(g[i * 3 + 1], g[3 + j]));
+      // (the last products of entries 3 and 4 are those of det g below)
+      gg[i * 3 + j] = i == 1 && j < 2 ? __fadd_rn(x, __fmul_rn(g[i * 3 + 2], g[6 + j]))
+                                      : __fmaf_rn(g[i * 3 + 2], g[6 + j], x);
+    }
+  const float t = g[0] + g[4] + g[8];
+  const float I2 = 0.5f * __fmaf_rn(t, t, -(gg[0] + gg[4] + gg[8]));
+  const float d0 = __fmaf_rn(g[4], g[8], -__fmul_rn(g[5], g[7]));
+  const float d1 = __fmaf_rn(g[3], g[8], -__fmul_rn(g[5], g[6]));
+  const float d2 = __fmaf_rn(-g[4], g[6], __fmul_rn(g[3], g[7]));
+  const float dg = __fmaf_rn(g[2], d2, __fmaf_rn(g[0], d0, -__fmul_rn(g[1], d1)));
+  const float jm1 = __fadd_rn(__fadd_rn(t, I2), dg);
+  const float iJ = 1.0f / __fadd_rn(1.0f, jm1);
+  const float a = __fmul_rn(mu, iJ), b = __fmul_rn(__fmul_rn(lam, log1pf(jm1)), iJ), c = 1.0f + t;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const float gt = g[j * 3 + i], ggt = gg[j * 3 + i];
+      float adjT, dev;
+      if (i == j) {
+        adjT = __fadd_rn(__fmaf_rn(-c, gt, __fadd_rn(c, I2)), ggt);
+        dev = __fadd_rn(__fmaf_rn(c, gt, dg), -ggt);
+      } else {
+        const float cg = __fmul_rn(c, gt);
+        adjT = __fadd_rn(ggt, -cg);
+        dev = __fadd_rn(cg, -ggt);
+      }
+      P[i * 3 + j] = __fmaf_rn(b, adjT, __fmaf_rn(mu, g[i * 3 + j], __fmul_rn(a, dev)));
+    }
+}
+
+// Edge sums T_j[e] = sum_q W[q][j][e] w_q P[:, j] of a voxel from its edge
+// differences D (see voxel_forces); PSUM adds sum_q w_q P to psum.
+template <typename S, bool PSUM>
+__device__ __forceinline__ void voxel_edge_sums(const S* B, const MatParams& mp,
+                                                const S (&D)[3][4][3], S wq, S (&T)[3][4][3],
+                                                double* psum) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) T[j][e][i] = 0;
+#pragma unroll 1
+  for (int q = 0; q < 8; ++q) {
+    const S* Wq = B + q * 12;  // [direction][edge]
+    S g[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        S c;
+        if constexpr (sizeof(S) == 4) {
+          c = __fmaf_rn(Wq[j * 4], D[j][0][i], __fmul_rn(Wq[j * 4 + 1], D[j][1][i]));
+          c = __fmaf_rn(Wq[j * 4 + 2], D[j][2][i], c);
+          c = __fmaf_rn(Wq[j * 4 + 3], D[j][3][i], c);
+        } else {
+          c = Wq[j * 4] * D[j][0][i];
+#pragma unroll
+          for (int e = 1; e < 4; ++e) c += Wq[j * 4 + e] * D[j][e][i];
+        }
+        g[i * 3 + j] = c;
+      }
+    S P[9];
+    if constexpr (sizeof(S) == 4)
+      voxel_stress_f32(mp, g, P);
+    else
+      voxel_stress<S>(mp, g, P);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) P[k] *= wq;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          if constexpr (sizeof(S) == 4)
+            T[j][e][i] = __fmaf_rn(Wq[j * 4 + e], P[i * 3 + j], T[j][e][i]);
+          else
+            T[j][e][i] += Wq[j * 4 + e] * P[i * 3 + j];
+        }
+    if (PSUM)
+#pragma unroll
+      for (int k = 0; k < 9; ++k) psum[k] += double(P[k]);
+  }
+}
+
 // f -= element forces of every voxel (8 colours); PSUM also adds
 // sum_q w_q P (row-major) of this thread's voxels to psum.
 //
@@ -220,39 +328,7 @@ __device__ void voxel_forces(const RveArgs& R, const RveSmem<S>& s, const S* hH,
       }
       const MatParams& mp = mats[s.mat[pidx(ex, ey, ez, n)]];
       S T[3][4][3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-          for (int i = 0; i < 3; ++i) T[j][e][i] = 0;
-#pragma unroll 1
-      for (int q = 0; q < 8; ++q) {
-        const S* Wq = s.B + q * 12;  // [direction][edge]
-        S g[9];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            S c = Wq[j * 4] * D[j][0][i];
-#pragma unroll
-            for (int e = 1; e < 4; ++e) c += Wq[j * 4 + e] * D[j][e][i];
-            g[i * 3 + j] = c;
-          }
-        S P[9];
-        voxel_stress<S>(mp, g, P);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) P[k] *= wq;
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int i = 0; i < 3; ++i) T[j][e][i] += Wq[j * 4 + e] * P[i * 3 + j];
-        if (PSUM)
-#pragma unroll
-          for (int k = 0; k < 9; ++k) psum[k] += double(P[k]);
-      }
+      voxel_edge_sums<S, PSUM>(s.B, mp, D, wq, T, psum);
 #pragma unroll
       for (int o = 0; o < 8; ++o) {
         const int ox = o & 1, oy = (o >> 1) & 1, oz = o >> 2;
@@ -279,6 +355,54 @@ __device__ inline double warp_sum(double x) {
   return x;
 }
 
+// Time-step scale, damping and residual scale of an instance.
+__device__ __noinline__ void instance_scales(const RveArgs& R, const double* Hd, double* par) {
+  double F[9], C[9];
+  for (int k = 0; k < 9; ++k) F[k] = Hd[k] + (k % 4 == 0 ? 1.0 : 0.0);
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) {
+      double c = 0;
+      for (int k = 0; k < 3; ++k) c += F[k * 3 + i] * F[k * 3 + j];
+      C[i * 3 + j] = c;
+    }
+  const double J = det3d(F);
+  const double smin = sqrt(fmax(smallest_eigenvalue(C), 0.0));
+  const double stiff = J > 0 ? fmax(0.0, -log(J)) : 0.0;
+  double c2 = 0.0, cs = 1e300, mumax = 0.0, hmax = 0.0;
+  for (int m = 0; m < R.nmat; ++m) {
+    const double m2 = R.lam[m] + 2.0 * R.mu[m];
+    const double t = R.kind[m] == AKB_MATERIAL_NEOHOOKEAN ? (m2 + 2.0 * R.lam[m] * stiff) / m2 : 1.0;
+    c2 = fmax(c2, t);
+    cs = fmin(cs, sqrt(R.mu[m] / m2));
+    mumax = fmax(mumax, R.mu[m]);
+  }
+  for (int k = 0; k < 9; ++k) hmax = fmax(hmax, fabs(Hd[k]));
+  par[0] = R.h * smin / sqrt(c2);
+  par[1] = R.dampf * 2.0 * (2.0 * M_PI / R.L) * cs;
+  par[2] = R.h * R.h * mumax * fmax(hmax, 1e-6);
+}
+
+// Edge weight W[q][direction][edge] (see voxel_forces), t = 12 q + 4 direction + edge.
+template <typename S>
+__device__ inline S edge_weight(const RveArgs& R, int t) {
+  const int q = t / 12, j = (t / 4) % 3, e = t % 4;
+  const double gp = 1.0 / sqrt(3.0);
+  const double c[3] = {(q & 1) ? gp : -gp, (q & 2) ? gp : -gp, (q & 4) ? gp : -gp};
+  const int d1 = j == 0 ? 1 : 0, d2 = j == 2 ? 1 : 2;  // the two other directions
+  const double s1 = 2.0 * (e & 1) - 1.0, s2 = 2.0 * (e >> 1) - 1.0;
+  return S((1.0 + s1 * c[d1]) * (1.0 + s2 * c[d2]) / (4.0 * R.h));
+}
+
+__device__ inline MatParams instance_material(const RveArgs& R, int k) {
+  MatParams mp{};
+  mp.kind = R.kind[k];
+  mp.finite = R.kind[k] == AKB_MATERIAL_NEOHOOKEAN;
+  mp.lambda = R.lam[k];
+  mp.mu = R.mu[k];
+  mp.E = 1.0;
+  return mp;
+}
+
 // One RVE instance, by the whole CTA: relaxation from the instance's
 // fluctuation (or zero), homogenised stress, state written back.
 template <typename S>
@@ -299,23 +423,8 @@ __device__ __forceinline__ void rve_instance(const RveArgs& R, int64_t inst,
     s.im[q] = im_g[k];
     s.mat[q] = R.vmat[k];
   }
-  if (tid < 96) {  // edge weights W[q][direction][edge] (see voxel_forces)
-    const int q = tid / 12, j = (tid / 4) % 3, e = tid % 4;
-    const double gp = 1.0 / sqrt(3.0);
-    const double c[3] = {(q & 1) ? gp : -gp, (q & 2) ? gp : -gp, (q & 4) ? gp : -gp};
-    const int d1 = j == 0 ? 1 : 0, d2 = j == 2 ? 1 : 2;  // the two other directions
-    const double s1 = 2.0 * (e & 1) - 1.0, s2 = 2.0 * (e >> 1) - 1.0;
-    s.B[tid] = S((1.0 + s1 * c[d1]) * (1.0 + s2 * c[d2]) / (4.0 * R.h));
-  }
-  if (tid < R.nmat) {
-    MatParams mp{};
-    mp.kind = R.kind[tid];
-    mp.finite = R.kind[tid] == AKB_MATERIAL_NEOHOOKEAN;
-    mp.lambda = R.lam[tid];
-    mp.mu = R.mu[tid];
-    mp.E = 1.0;
-    mats[tid] = mp;
-  }
+  if (tid < 96) s.B[tid] = edge_weight<S>(R, tid);
+  if (tid < R.nmat) mats[tid] = instance_material(R, tid);
   __shared__ S hH[9];  // h H, row-major
   double Hd[9];
 #pragma unroll
@@ -324,30 +433,7 @@ __device__ __forceinline__ void rve_instance(const RveArgs& R, int64_t inst,
     for (int j = 0; j < 3; ++j) Hd[i * 3 + j] = grad_u[inst * 9 + i + 3 * j];
   if (tid < 9) hH[tid] = S(R.h * Hd[tid]);
   if (tid == 0) {
-    // time-step scale, damping and residual scale of this instance
-    double F[9], C[9];
-    for (int k = 0; k < 9; ++k) F[k] = Hd[k] + (k % 4 == 0 ? 1.0 : 0.0);
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) {
-        double c = 0;
-        for (int k = 0; k < 3; ++k) c += F[k * 3 + i] * F[k * 3 + j];
-        C[i * 3 + j] = c;
-      }
-    const double J = det3d(F);
-    const double smin = sqrt(fmax(smallest_eigenvalue(C), 0.0));
-    const double stiff = J > 0 ? fmax(0.0, -log(J)) : 0.0;
-    double c2 = 0.0, cs = 1e300, mumax = 0.0, hmax = 0.0;
-    for (int m = 0; m < R.nmat; ++m) {
-      const double m2 = R.lam[m] + 2.0 * R.mu[m];
-      const double t = R.kind[m] == AKB_MATERIAL_NEOHOOKEAN ? (m2 + 2.0 * R.lam[m] * stiff) / m2 : 1.0;
-      c2 = fmax(c2, t);
-      cs = fmin(cs, sqrt(R.mu[m] / m2));
-      mumax = fmax(mumax, R.mu[m]);
-    }
-    for (int k = 0; k < 9; ++k) hmax = fmax(hmax, fabs(Hd[k]));
-    s.par[0] = R.h * smin / sqrt(c2);
-    s.par[1] = R.dampf * 2.0 * (2.0 * M_PI / R.L) * cs;
-    s.par[2] = R.h * R.h * mumax * fmax(hmax, 1e-6);
+    instance_scales(R, Hd, s.par);
   }
   __syncthreads();
   const double fscale = s.par[2];
@@ -461,6 +547,347 @@ __global__ void __launch_bounds__(kRveThreads, 1)
   }
 }
 
+// ------------------------------------------------------- one RVE per cluster
+// FP32 RVEs are relaxed by a cluster of C CTAs, each owning n / C planes of
+// voxels and nodes (C = 1, 2 or 4: at most 1024 voxels a CTA). Bound by FP32
+// issue, and for small batches by the slowest instance (of 512 random
+// gradients it takes 1500-2200 updates against 260 on average), so an update
+// has to be short as well as cheap. Two changes against one CTA per RVE:
+//  - the corner forces of every voxel go to shared memory (96 bytes a voxel)
+//    and each node then adds its 8 voxels' in colour order, the order in which
+//    the coloured scatter added them (the same sums bit for bit), so that a
+//    step is two cluster barriers instead of ten CTA barriers and all voxels
+//    are computed at once: 16 warps of 128 registers instead of 8 of 213;
+//  - the planes are spread over C SMs. A CTA reads the forces of the layer
+//    below its first plane, and writes the displacements of that plane, in the
+//    neighbour's shared memory.
+constexpr int kClusterThreads = 512;
+constexpr int kClusterVoxels = 1024;
+
+// CTAs per RVE of n^3 cells, 0: not this way.
+inline int cluster_of(int n) {
+  for (int c = 1; c <= 4; c *= 2)
+    if (n % c == 0 && (n / c) % 2 == 0 && (int64_t)n * n * n / c <= kClusterVoxels) return c;
+  return 0;
+}
+
+struct ClusterLayout {
+  int u, v, im, B, F, mat, red, total;  // byte offsets
+};
+__host__ __device__ inline ClusterLayout cluster_layout(int n, int C) {
+  const int nl = n * n * n / C, halo = C > 1 ? n * n : 0;
+  ClusterLayout s;
+  s.u = 0;
+  s.v = s.u + 4 * 3 * (nl + halo);
+  s.im = s.v + 4 * 3 * nl;
+  s.B = s.im + 4 * nl;
+  s.F = s.B + 4 * 96;
+  s.mat = s.F + 4 * 24 * nl;
+  s.red = (s.mat + nl + 15) & ~15;
+  // 16 warps x 9, the CTAs' sums (4 x 9) and maxima (2 x 4), 3 scales
+  s.total = s.red + 8 * (16 * 9 + 4 * 9 + 8 + 4);
+  return s;
+}
+
+template <int C>
+__device__ inline void cluster_sync() {
+  if constexpr (C == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+// The address of this CTA's shared-memory address a in CTA `rank` of the cluster.
+__device__ inline uint32_t remote(uint32_t a, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ inline float ld_remote(uint32_t a) {
+  float x;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(a) : "memory");
+  return x;
+}
+__device__ inline void st_remote(uint32_t a, float x) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory");
+}
+__device__ inline void st_remote(uint32_t a, double x) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(x) : "memory");
+}
+
+// One instance, by the whole cluster.
+template <int C>
+__device__ __forceinline__ void rve_cluster_instance(const RveArgs& R, int rank, int64_t inst,
+                                                     const double* __restrict__ grad_u, float* fluct,
+                                                     double* __restrict__ stress,
+                                                     int32_t* iterations, double* residual,
+                                                     double* internal_force) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ MatParams mats[8];
+  __shared__ float hH[9];
+  const int n = R.n, nn = R.nn, hn = n >> 1, plane = n * n, nl = nn / C, Zs = n / C;
+  const int z0 = rank * Zs, cls = nl >> 3, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const ClusterLayout lay = cluster_layout(n, C);
+  float* u = reinterpret_cast<float*>(smem + lay.u);  // [3][nl + halo]
+  float* v = reinterpret_cast<float*>(smem + lay.v);  // [3][nl]
+  float* im = reinterpret_cast<float*>(smem + lay.im);
+  float* B = reinterpret_cast<float*>(smem + lay.B);
+  float* F = reinterpret_cast<float*>(smem + lay.F);  // [corner][component][nl]
+  uint8_t* mat = smem + lay.mat;
+  double* red = reinterpret_cast<double*>(smem + lay.red);
+  double *csum = red + 16 * 9, *cmax = csum + 4 * 9, *par = cmax + 8;
+  const int US = nl + (C > 1 ? plane : 0);
+  const int below = (rank + C - 1) % C;
+  // position of node (or voxel) (x, y, z0 + z): by parity class as pidx; the
+  // plane above the CTA's (the next CTA's first) follows
+  auto at = [&](int x, int y, int z) {
+    if (C > 1 && z == Zs) return nl + ((x & 1) | ((y & 1) << 1)) * (hn * hn) + (x >> 1) + hn * (y >> 1);
+    return ((x & 1) | ((y & 1) << 1) | ((z & 1) << 2)) * cls + (x >> 1) + hn * ((y >> 1) + hn * (z >> 1));
+  };
+  // this thread's voxels and nodes: positions tid + m kClusterThreads < nl, and
+  // their (x, y, z), packed
+  constexpr int kNodes = (kClusterVoxels + kClusterThreads - 1) / kClusterThreads;
+  int xyz[kNodes];
+#pragma unroll
+  for (int m = 0; m < kNodes; ++m) {
+    const int k = tid + m * kClusterThreads, c = k / cls, t = k - c * cls;
+    xyz[m] = (2 * (t % hn) + (c & 1)) | (2 * ((t / hn) % hn) + ((c >> 1) & 1)) << 8 |
+             (2 * (t / (hn * hn)) + (c >> 2)) << 16;
+  }
+
+  for (int k = tid; k < nl; k += kClusterThreads) {
+    const int x = k % n, y = (k / n) % n, z = k / plane, g = k + z0 * plane;
+    im[at(x, y, z)] = static_cast<const float*>(R.inv_mass)[g];
+    mat[at(x, y, z)] = R.vmat[g];
+  }
+  if (tid < 96) B[tid] = edge_weight<float>(R, tid);
+  if (tid < R.nmat) mats[tid] = instance_material(R, tid);
+  double Hd[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) Hd[i * 3 + j] = grad_u[inst * 9 + i + 3 * j];
+  if (tid < 9) hH[tid] = float(R.h * grad_u[inst * 9 + tid / 3 + 3 * (tid % 3)]);
+  if (tid == 0) instance_scales(R, Hd, par);
+  __syncthreads();
+  const double fscale = par[2];
+  const float wq = float(R.h * R.h * R.h / 8.0);
+
+  // corner forces of the CTA's voxels into F
+  auto voxels = [&](auto psum_tag, double* psum) {
+    constexpr bool PSUM = decltype(psum_tag)::value;
+#pragma unroll 1
+    for (int m = 0; m < kNodes; ++m) {
+      const int k = tid + m * kClusterThreads;
+      if (k >= nl) break;
+      int pk = xyz[0];
+#pragma unroll
+      for (int j = 1; j < kNodes; ++j) pk = m == j ? xyz[j] : pk;
+      const int ex = pk & 255, ey = (pk >> 8) & 255, ez = pk >> 16;
+      const int x1 = ex + 1 == n ? 0 : ex + 1, y1 = ey + 1 == n ? 0 : ey + 1,
+                z1 = C == 1 && ez + 1 == n ? 0 : ez + 1;
+      int nd[8];
+#pragma unroll
+      for (int o = 0; o < 8; ++o) nd[o] = at((o & 1) ? x1 : ex, (o & 2) ? y1 : ey, (o & 4) ? z1 : ez);
+      float D[3][4][3];  // edge differences [direction][edge][component]
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        float uc[8];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) uc[o] = u[i * US + nd[o]];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int b0 = e & 1, b1 = e >> 1;
+          D[0][e][i] = (uc[1 + 2 * b0 + 4 * b1] - uc[2 * b0 + 4 * b1]) + hH[i * 3 + 0];
+          D[1][e][i] = (uc[b0 + 2 + 4 * b1] - uc[b0 + 4 * b1]) + hH[i * 3 + 1];
+          D[2][e][i] = (uc[b0 + 2 * b1 + 4] - uc[b0 + 2 * b1]) + hH[i * 3 + 2];
+        }
+      }
+      float T[3][4][3];
+      voxel_edge_sums<float, PSUM>(B, mats[mat[k]], D, wq, T, psum);
+#pragma unroll
+      for (int o = 0; o < 8; ++o) {
+        const int ox = o & 1, oy = (o >> 1) & 1, oz = o >> 2;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const float tx = T[0][oy + 2 * oz][i], ty = T[1][ox + 2 * oz][i], tz = T[2][ox + 2 * oy][i];
+          F[(o * 3 + i) * nl + k] = (ox ? tx : -tx) + (oy ? ty : -ty) + (oz ? tz : -tz);
+        }
+      }
+    }
+  };
+  // the force of the CTA's node at position k: its voxels' in colour order
+  const uint32_t F_below = C > 1 ? remote((uint32_t)__cvta_generic_to_shared(F), below) : 0;
+  auto force = [&](int x, int y, int z, float* f) {
+    f[0] = f[1] = f[2] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const bool hx = (x & 1) != (c & 1), hy = (y & 1) != ((c >> 1) & 1), hz = (z & 1) != (c >> 2);
+      const int vx = hx ? (x == 0 ? n - 1 : x - 1) : x, vy = hy ? (y == 0 ? n - 1 : y - 1) : y;
+      const int vz = hz ? (z == 0 ? Zs - 1 : z - 1) : z;
+      const int o = (hx ? 1 : 0) + (hy ? 2 : 0) + (hz ? 4 : 0);
+      const int w = o * 3 * nl + at(vx, vy, vz);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        f[i] -= C > 1 && hz && z == 0 ? ld_remote(F_below + 4 * (w + i * nl)) : F[w + i * nl];
+    }
+  };
+
+  int total = 0, k = 0;
+  double r = 0.0, tsf = R.tsf;
+  for (int attempt = 0;; ++attempt, tsf *= kRestartFactor) {
+    for (int idx = tid; idx < 3 * US; idx += kClusterThreads) {
+      const int node = idx / 3, i = idx - 3 * node;
+      const int x = node % n, y = (node / n) % n, z = node / plane;
+      const int64_t g = (int64_t)((z0 + z) % n) * plane + node % plane;
+      u[i * US + at(x, y, z)] = fluct ? fluct[inst * 3 * nn + 3 * g + i] : 0.0f;
+      if (z < Zs) v[idx] = 0.0f;
+    }
+    const double dtd = tsf * par[0];
+    const float dt = float(dtd);
+    const float a1 = float(1.0 - 0.5 * par[1] * dtd), a2 = float(1.0 + 0.5 * par[1] * dtd);
+    __syncthreads();
+    bool diverged = false;
+    for (k = 0;; ++k) {
+      voxels(std::false_type{}, nullptr);
+      cluster_sync<C>();  // every corner force is written
+      float f[kNodes][3];
+#pragma unroll
+      for (int m = 0; m < kNodes; ++m) {
+        const int q = tid + m * kClusterThreads;
+        if (q < nl) {
+          force(xyz[m] & 255, (xyz[m] >> 8) & 255, xyz[m] >> 16, f[m]);
+        }
+      }
+      const bool last = k >= R.max_it;
+      if (last || (R.check > 0 && k % R.check == 0)) {
+        double lm = 0.0;
+#pragma unroll
+        for (int m = 0; m < kNodes; ++m)
+          if (tid + m * kClusterThreads < nl)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              const double x = double(f[m][i]);
+              lm = isfinite(x) ? fmax(lm, fabs(x)) : INFINITY;
+            }
+        lm = warp_max(lm);
+        if (lane == 0) red[warp] = lm;
+        __syncthreads();
+        if (tid < C) {
+          double m = 0.0;
+          for (int w = 0; w < kClusterThreads / 32; ++w) m = fmax(m, red[w]);
+          if constexpr (C == 1)
+            cmax[0] = m;
+          else
+            st_remote(remote((uint32_t)__cvta_generic_to_shared(cmax + rank), tid), m);
+        }
+        cluster_sync<C>();
+        double m = 0.0;
+        for (int w = 0; w < C; ++w) m = fmax(m, cmax[w]);
+        r = isfinite(m) ? m / fscale : INFINITY;
+        diverged = !(r <= kDivergence);
+        if (last || diverged || (R.tol >= 0 && r <= R.tol)) break;
+      }
+#pragma unroll
+      for (int m = 0; m < kNodes; ++m) {
+        const int q = tid + m * kClusterThreads;
+        if (q < nl) {
+          const float imq = im[q];
+          const int x = xyz[m] & 255, y = (xyz[m] >> 8) & 255, z = xyz[m] >> 16;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const float vv =
+                __fmaf_rn(a1, v[i * nl + q], __fmul_rn(__fmul_rn(dt, f[m][i]), imq)) / a2;
+            v[i * nl + q] = vv;
+            const float un = __fmaf_rn(dt, vv, u[i * US + q]);
+            u[i * US + q] = un;
+            if (C > 1 && z == 0)  // the plane above the CTA below
+              st_remote(remote((uint32_t)__cvta_generic_to_shared(u + i * US + at(x, y, Zs)), below), un);
+          }
+        }
+      }
+      cluster_sync<C>();  // every displacement is written
+    }
+    total += k;
+    if (!diverged || attempt >= kMaxRestarts) break;
+    cluster_sync<C>();
+  }
+
+  // homogenised stress (and force) of the final state
+  double ps[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) ps[q] = 0.0;
+  cluster_sync<C>();  // the forces of the last update are read
+  voxels(std::true_type{}, ps);
+#pragma unroll
+  for (int q = 0; q < 9; ++q) {
+    const double x = warp_sum(ps[q]);
+    if (lane == 0) red[warp * 9 + q] = x;
+  }
+  __syncthreads();
+  if (tid < 9) {
+    double t = 0.0;
+    for (int w = 0; w < kClusterThreads / 32; ++w) t += red[w * 9 + tid];
+    if constexpr (C == 1)
+      csum[tid] = t;
+    else
+      st_remote(remote((uint32_t)__cvta_generic_to_shared(csum + rank * 9 + tid), 0), t);
+  }
+  cluster_sync<C>();
+  if (rank == 0 && tid < 9) {
+    double t = 0.0;
+    for (int w = 0; w < C; ++w) t += csum[w * 9 + tid];
+    const int i = tid / 3, j = tid % 3;
+    stress[inst * 9 + i + 3 * j] = t / (R.L * R.L * R.L);
+  }
+  if (rank == 0 && tid == 0) {
+    if (iterations) iterations[inst] = total;
+    if (residual) residual[inst] = r;
+  }
+#pragma unroll
+  for (int m = 0; m < kNodes; ++m) {
+    const int q = tid + m * kClusterThreads;
+    if (q >= nl) break;
+    const int x = xyz[m] & 255, y = (xyz[m] >> 8) & 255, z = xyz[m] >> 16;
+    const int64_t g = inst * 3 * nn + 3 * ((int64_t)(z0 + z) * plane + y * n + x);
+    if (fluct && R.write_fluct)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) fluct[g + i] = u[i * US + q];
+    if (internal_force) {
+      float f[3];
+      force(x, y, z, f);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) internal_force[g + i] = double(f[i]);
+    }
+  }
+  cluster_sync<C>();  // no CTA leaves (or reuses its memory) while another reads it
+}
+
+__device__ inline int cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return (int)r;
+}
+
+// The instances [0, nb), or with INDEXED index[0 .. min(*count, nb)), the count
+// read on the device: clusters stride over them.
+template <int C, bool INDEXED>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    k_rve_cluster(RveArgs R, int64_t nb, const int32_t* __restrict__ index,
+                  const int32_t* __restrict__ count, const double* __restrict__ grad_u,
+                  float* fluct, double* __restrict__ stress, int32_t* iterations, double* residual,
+                  double* internal_force) {
+  const int rank = C == 1 ? 0 : cluster_rank();
+  grid_wait();  // whatever the stream did before has completed
+  const int64_t n = INDEXED ? min((int64_t)*count, nb) : nb;
+  for (int64_t b = blockIdx.x / C; b < n; b += gridDim.x / C) {
+    const int64_t inst = INDEXED ? index[b] : b;
+    if (inst < 0 || inst >= nb) continue;  // uniform over the cluster
+    rve_cluster_instance<C>(R, rank, inst, grad_u, fluct, stress, iterations, residual,
+                            internal_force);
+  }
+}
+
 std::mutex g_rve_attr_mutex;
 
 template <typename S>
@@ -474,6 +901,68 @@ cudaError_t raise_limit(size_t bytes) {
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(k_rve_indexed<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)bytes);
+}
+
+template <int C>
+cudaError_t configure_cluster(int n) {
+  std::lock_guard<std::mutex> lock(g_rve_attr_mutex);
+  const int bytes = cluster_layout(n, C).total;
+  const void* kernels[2] = {(const void*)k_rve_cluster<C, false>, (const void*)k_rve_cluster<C, true>};
+  for (const void* k : kernels) {
+    cudaFuncAttributes attr;
+    cudaError_t e = cudaFuncGetAttributes(&attr, k);
+    if (e == cudaSuccess && attr.maxDynamicSharedSizeBytes < bytes)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+cudaError_t configure_cluster(int n) {
+  switch (cluster_of(n)) {
+  case 1: return configure_cluster<1>(n);
+  case 2: return configure_cluster<2>(n);
+  case 4: return configure_cluster<4>(n);
+  default: return cudaSuccess;
+  }
+}
+
+// `clusters` clusters over nb instances (or the listed ones of them).
+template <int C, bool INDEXED>
+cudaError_t launch_cluster(const RveArgs& a, int64_t clusters, int64_t nb, const int32_t* index,
+                           const int32_t* count, const double* grad_u, float* fluct, double* stress,
+                           int32_t* iterations, double* residual, double* force, cudaStream_t s) {
+  clusters = std::min<int64_t>(clusters, INT32_MAX / C);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(clusters * C));
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = cluster_layout(a.n, C).total;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  // the launch itself overlaps the kernel before it: most lists are empty
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, k_rve_cluster<C, INDEXED>, a, nb, index, count, grad_u, fluct,
+                            stress, iterations, residual, force);
+}
+template <bool INDEXED>
+cudaError_t launch_cluster(int C, const RveArgs& a, int64_t clusters, int64_t nb,
+                           const int32_t* index, const int32_t* count, const double* grad_u,
+                           void* fluct, double* stress, int32_t* iterations, double* residual,
+                           double* force, cudaStream_t s) {
+  float* w = static_cast<float*>(fluct);
+  switch (C) {
+  case 1: return launch_cluster<1, INDEXED>(a, clusters, nb, index, count, grad_u, w, stress,
+                                            iterations, residual, force, s);
+  case 2: return launch_cluster<2, INDEXED>(a, clusters, nb, index, count, grad_u, w, stress,
+                                            iterations, residual, force, s);
+  default: return launch_cluster<4, INDEXED>(a, clusters, nb, index, count, grad_u, w, stress,
+                                             iterations, residual, force, s);
+  }
 }
 
 RveArgs args_of(const akb_rve* r, int max_it) {
@@ -513,6 +1002,9 @@ akb_status launch(akb_rve* r, int max_it, int64_t nb, const double* grad_u, void
   if (r->mode == AKB_MODE_FP64)
     k_rve<double><<<(unsigned)nb, kRveThreads, r->smem, s>>>(
         a, nb, grad_u, static_cast<double*>(fluct), stress, iterations, residual, force);
+  else if (const int C = cluster_of(r->n))
+    AKB_CUDA_TRY(launch_cluster<false>(C, a, nb, nb, nullptr, nullptr, grad_u, fluct, stress,
+                                       iterations, residual, force, s));
   else
     k_rve<float><<<(unsigned)nb, kRveThreads, r->smem, s>>>(
         a, nb, grad_u, static_cast<float*>(fluct), stress, iterations, residual, force);
@@ -604,6 +1096,7 @@ akb_status akb_rve_create(const akb_rve_desc* desc, const akb_rve_options* optio
     AKB_CUDA_TRY(cudaMalloc(&r->d_inv_mass, nn * sizeof(float)));
     AKB_CUDA_TRY(cudaMemcpy(r->d_inv_mass, im.data(), nn * sizeof(float), cudaMemcpyHostToDevice));
     AKB_CUDA_TRY(raise_limit<float>(r->smem));
+    AKB_CUDA_TRY(configure_cluster(n));
   }
   *out = r.release();
   return AKB_OK;
@@ -656,6 +1149,10 @@ akb_status akb_rve_solve_indexed(akb_rve* r, int64_t capacity, const int32_t* in
     k_rve_indexed<double><<<grid, kRveThreads, r->smem, s>>>(
         a, capacity, index, count, grad_u, static_cast<double*>(fluctuation), stress, iterations,
         residual);
+  else if (const int C = cluster_of(r->n))
+    AKB_CUDA_TRY(launch_cluster<true>(C, a, std::max<int64_t>(1, std::min<int64_t>(capacity, sms / C)),
+                                      capacity, index, count, grad_u, fluctuation, stress,
+                                      iterations, residual, nullptr, s));
   else
     k_rve_indexed<float><<<grid, kRveThreads, r->smem, s>>>(
         a, capacity, index, count, grad_u, static_cast<float*>(fluctuation), stress, iterations,
