@@ -385,6 +385,153 @@ __device__ inline void hex_parallelepiped_force(const MatParams& p, const double
     }
 }
 
+// Signed corner sums of v (v_0 = 0) that give the trilinear derivatives at the
+// Gauss points (hex_parallelepiped_force): E0[k] (s_k), Fp[pair] (s_k s_m, times
+// 1/sqrt(3)), F3 (s_x s_y s_z, times 1/3), all times 1/8.
+__device__ inline void hex_sums(const double* v, double (*E0)[3], double (*Fp)[3], double* F3) {
+  const int sg[3][8] = {{-1, 1, 1, -1, -1, 1, 1, -1},
+                        {-1, -1, 1, 1, -1, -1, 1, 1},
+                        {-1, -1, -1, -1, 1, 1, 1, 1}};
+  const double g8 = 0.125 * 0.57735026918962576451, t8 = 0.125 / 3.0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    double e0x = 0, e0y = 0, e0z = 0, exy = 0, exz = 0, eyz = 0, exyz = 0;
+#pragma unroll
+    for (int a = 1; a < 8; ++a) {
+      const double x = v[a * 3 + i];
+      e0x += sg[0][a] * x;
+      e0y += sg[1][a] * x;
+      e0z += sg[2][a] * x;
+      exy += (sg[0][a] * sg[1][a]) * x;
+      exz += (sg[0][a] * sg[2][a]) * x;
+      eyz += (sg[1][a] * sg[2][a]) * x;
+      exyz += (sg[0][a] * sg[1][a] * sg[2][a]) * x;
+    }
+    E0[0][i] = 0.125 * e0x;
+    E0[1][i] = 0.125 * e0y;
+    E0[2][i] = 0.125 * e0z;
+    Fp[0][i] = g8 * exy;
+    Fp[1][i] = g8 * exz;
+    Fp[2][i] = g8 * eyz;
+    F3[i] = t8 * exyz;
+  }
+}
+// dv_i/dxi_k at the Gauss point of signs s from the sums.
+__device__ inline double hex_derivative(const double (*E0)[3], const double (*Fp)[3],
+                                        const double* F3, const double* s, int i, int k) {
+  const int m = k == 0 ? 1 : 0, n = k == 2 ? 1 : 2;
+  return E0[k][i] + s[m] * Fp[k + m - 1][i] + s[n] * Fp[k + n - 1][i] + (s[m] * s[n]) * F3[i];
+}
+
+// FP64 hexahedron force by the signed sums (hex_parallelepiped_force, whose
+// accuracy notes concern FP32): with PAR the element map is affine, one
+// Jacobian for all points and 1 / det J folded into it; otherwise the Jacobian
+// of each point comes from the coordinates' sums, at 27 operations instead of
+// the 63 of the shape derivatives, and so do the displacement derivatives and
+// the corner forces (36 instead of 72).
+template <bool PAR>
+__device__ inline void hex_force_f64(const MatParams& p, const double* dX, const double* du,
+                                     double* fe) {
+  constexpr int d = 3;
+  const int sg[3][8] = {{-1, 1, 1, -1, -1, 1, 1, -1},
+                        {-1, -1, 1, 1, -1, -1, 1, 1},
+                        {-1, -1, -1, -1, 1, 1, 1, 1}};
+  double X0[3][3], Xp[3][3], X3[3], E0[3][3], Fp[3][3], F3[3], A[9], Ai[9];
+  hex_sums(dX, X0, Xp, X3);
+  hex_sums(du, E0, Fp, F3);
+  if (PAR) {
+    double J[9];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) J[k * 3 + j] = X0[k][j];
+    const double idet = 1.0 / adjugate<3, double>(J, A);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Ai[k] = A[k] * idet;
+  }
+  double T0[9], Tm[9], Tn[9], Tmn[9];
+#pragma unroll
+  for (int t = 0; t < 9; ++t) T0[t] = Tm[t] = Tn[t] = Tmn[t] = 0;
+#pragma unroll 1  // (two points in flight gain nothing at 255 registers: 80.0 against 79.5 us)
+  for (int q = 0; q < 8; ++q) {
+    const double s[3] = {(q & 1) ? 1. : -1., (q & 2) ? 1. : -1., (q & 4) ? 1. : -1.};
+    if (!PAR) {
+      double J[9];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) J[k * 3 + j] = hex_derivative(X0, Xp, X3, s, j, k);
+      const double idet = 1.0 / adjugate<3, double>(J, A);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) Ai[k] = A[k] * idet;
+    }
+    double g[9], P[9];
+#pragma unroll
+    for (int i = 0; i < d; ++i) {
+      double H[3];
+#pragma unroll
+      for (int k = 0; k < d; ++k) H[k] = hex_derivative(E0, Fp, F3, s, i, k);
+#pragma unroll
+      for (int j = 0; j < d; ++j)
+        g[i * 3 + j] = H[0] * Ai[j * 3] + H[1] * Ai[j * 3 + 1] + H[2] * Ai[j * 3 + 2];
+    }
+    stress_P<3, double>(p, g, P);
+#pragma unroll
+    for (int i = 0; i < d; ++i)
+#pragma unroll
+      for (int k = 0; k < d; ++k) {
+        const int m = k == 0 ? 1 : 0, n = k == 2 ? 1 : 2, t = i * d + k;
+        const double Q = P[i * 3] * A[k] + P[i * 3 + 1] * A[3 + k] + P[i * 3 + 2] * A[6 + k];
+        T0[t] += Q;
+        Tm[t] += s[m] * Q;
+        Tn[t] += s[n] * Q;
+        Tmn[t] += (s[m] * s[n]) * Q;
+      }
+  }
+#pragma unroll
+  for (int t = 0; t < 9; ++t) {
+    T0[t] *= 0.125;
+    Tm[t] *= 0.125 * 0.57735026918962576451;
+    Tn[t] *= 0.125 * 0.57735026918962576451;
+    Tmn[t] *= 0.125 / 3.0;
+  }
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int i = 0; i < d; ++i) {
+      double f = 0;
+#pragma unroll
+      for (int k = 0; k < d; ++k) {
+        const int m = k == 0 ? 1 : 0, n = k == 2 ? 1 : 2, t = i * d + k;
+        const double sm = sg[m][a], sn = sg[n][a];
+        f += sg[k][a] * (T0[t] + sm * Tm[t] + sn * Tn[t] + (sm * sn) * Tmn[t]);
+      }
+      fe[a * d + i] = f;
+    }
+}
+
+// Whether a hexahedron's trilinear terms vanish to 1e-12 of its extent (dX:
+// corner differences to the first).
+__host__ __device__ inline bool hex_is_parallelepiped(const double* dX) {
+  const int sx[8] = {-1, 1, 1, -1, -1, 1, 1, -1};
+  const int sy[8] = {-1, -1, 1, 1, -1, -1, 1, 1};
+  const int sz[8] = {-1, -1, -1, -1, 1, 1, 1, 1};
+  double ext = 0, bend = 0;
+  for (int j = 0; j < 3; ++j) {
+    double c[4] = {0, 0, 0, 0};
+    for (int a = 1; a < 8; ++a) {
+      const double x = dX[a * 3 + j];
+      c[0] += sx[a] * sy[a] * x;
+      c[1] += sx[a] * sz[a] * x;
+      c[2] += sy[a] * sz[a] * x;
+      c[3] += sx[a] * sy[a] * sz[a] * x;
+      ext = fmax(ext, fabs(x));
+    }
+    for (int k = 0; k < 4; ++k) bend = fmax(bend, fabs(c[k]));
+  }
+  return bend <= 1e-12 * ext;
+}
+
 // Simplex (triangle_3, tetrahedron_4) internal force. The natural
 // derivatives are constant (dN_a/dxi_k = delta(a, k+1) - delta(a, 0)), so the
 // rows of J are X_a - X_0 (a >= 1) and w det J grad N_a = w adj(J)[:, a-1]:

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/akb_fe2.h"
+#include "akb_fastmath.cuh"
 #include "akb_internal.cuh"
 #include "akb_patch.cuh"
 
@@ -47,7 +48,7 @@ struct akb_model {
   bool stresses_valid = false;
   // user materials: stresses come from the caller between step_begin/end
   bool user = false;
-  bool linear = false;  // every material small-strain elastic
+  bool linear = false;  // DevPatches::linear
   bool in_step = false;
   double* d_scratch = nullptr;  // reduction partials
   int scratch_len = 0;
@@ -245,17 +246,21 @@ template <typename T>
 akb_status upload(akb_model* m, const std::vector<T>& v, const T** out);
 
 // The same for fan records: patches of at most max_fans fans of at most
-// fan_cap elements.
+// fan_cap elements (triangles and tetrahedra: a fan per thread of the CTA,
+// FanBuild), or of single elements.
 void fan_params(int type, int* target, int* max_nodes, int* fan_cap, int* max_fans) {
-  *fan_cap = 8;
-  if (type == AKB_TRIANGLE_3) {  // a fan per thread of the CTA (FanThreads)
+  *fan_cap = type == AKB_HEXAHEDRON_8 ? kSingles : 8;
+  if (type == AKB_TRIANGLE_3) {
     *max_fans = 128;
     *target = 768;
     *max_nodes = 500;
-  } else {
+  } else if (type == AKB_TETRAHEDRON_4) {
     *max_fans = 256;
     *target = 1536;
     *max_nodes = 640;
+  } else {
+    *max_fans = *target = 128;
+    *max_nodes = 400;
   }
 }
 
@@ -788,10 +793,20 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
   const double* mesh_X = mesh->nodes;
   const uint32_t* mesh_C = mesh->connectivity;
   if (patched) {
-    // FP64 triangles and tetrahedra step on fan records; a plan whose record or
-    // contributions do not fit an SM (patch sizes far above the defaults)
-    // steps chunk by chunk
-    bool fans = m->mode == AKB_MODE_FP64 && (type == AKB_TRIANGLE_3 || type == AKB_TETRAHEDRON_4);
+    // FP64 steps run on fan records, but for segments; a plan whose record or
+    // contributions do not fit an SM (patch sizes far above the defaults) steps
+    // chunk by chunk, as do FP32 steps, whose roundings go with that kernel
+    bool fans = m->mode == AKB_MODE_FP64 && type != AKB_SEGMENT_2;
+    if (fans && type == AKB_HEXAHEDRON_8) {
+      m->linear = true;
+      for (int64_t e = 0; e < ne && m->linear; ++e) {
+        double dX[24];
+        for (int k = 0; k < 24; ++k)
+          dX[k] = mesh->nodes[(int64_t)mesh->connectivity[e * 8 + k / 3] * 3 + k % 3] -
+                  mesh->nodes[(int64_t)mesh->connectivity[e * 8] * 3 + k % 3];
+        m->linear = fast::hex_is_parallelepiped(dX);
+      }
+    }
     if (fans) {
       st = plan_patches(m.get(), mesh, batch, part, true, plan, patch_inst, orphan_inst);
       fans = st == AKB_OK && fan_smem_bytes(plan, d) <= 227 * 1024;

@@ -644,8 +644,24 @@ __host__ __device__ inline FanLayout fan_layout(const DevPatches& p, int d, bool
 // Tetrahedra at 128 registers (16 warps an SM either way; more spill): 256
 // threads 140.6 us a step on the 6 M-element cube, 128 threads 145.3, 192
 // threads 148.7. Triangles (512 plates): 128 threads 47.9 us, 256 threads 48.4.
-template <int D> struct FanThreads { static constexpr int value = D == 3 ? 256 : 128; };
-template <int D, bool LIN> struct FanOccupancy { static constexpr int value = D == 3 ? 2 : LIN ? 6 : 5; };
+// LIN: every material small-strain elastic (simplices), every element a
+// parallelepiped (hexahedra).
+template <int TY, bool LIN> struct FanBuild;
+template <bool LIN> struct FanBuild<AKB_TETRAHEDRON_4, LIN> {
+  static constexpr int threads = 256, ctas = 2;
+};
+template <bool LIN> struct FanBuild<AKB_TRIANGLE_3, LIN> {
+  static constexpr int threads = 128, ctas = LIN ? 6 : 5;
+};
+// Hexahedra: FP64 issue bound, 255 registers for the signed sums and the 36
+// accumulators, so 8 warps an SM; 128-thread CTAs (a 128-element patch each)
+// overlap one patch's staging and finish with the other's elements. 64^3
+// neo-Hookean block: 79.5 us a step (256-element chunks in one 256-thread CTA
+// 95.1; 4 x 64 threads 81.4; 1 x 256 threads 126; 3 x 128 at 168 registers,
+// spilling, 86.8); 37 x 31 x 33 distorted 17.0 against 31.3.
+template <bool PAR> struct FanBuild<AKB_HEXAHEDRON_8, PAR> {
+  static constexpr int threads = 128, ctas = 2;
+};
 
 // w P of one element from G = det * grad u (row-major), P the Cauchy (small
 // strain) or first Piola stress, w the reference volume of the simplex.
@@ -806,6 +822,32 @@ __device__ __forceinline__ void fan_forces(const uint16_t* rec, int t, const dou
   if constexpr (d == 3) store((int)(node[ro[1] + t] >> 16), fb);
 }
 
+// Contributions of hexahedron t of a staged patch (fan records of single
+// elements, row a its corner a).
+template <bool PAR>
+__device__ __forceinline__ void hex_forces(const uint16_t* rec, int t, const double* xs,
+                                           const double* ws, double* C, const MatParams& mp0,
+                                           const MatParams* table, const uint32_t* emat) {
+  constexpr int d = 3, n = 8;
+  const int nf = rec[0];
+  const uint32_t* node = reinterpret_cast<const uint32_t*>(rec + rec[3]) + t;
+  const MatParams& mp = emat ? table[emat[t]] : mp0;
+  double dX[d * n], du[d * n], fe[d * n];
+  {
+    int lc[n];
+#pragma unroll
+    for (int a = 0; a < n; ++a) lc[a] = (int)(node[a * nf] & 0xffff);
+    gather_differences<d, n, double>(xs, ws, lc, dX, du);
+  }
+  fast::hex_force_f64<PAR>(mp, dX, du, fe);
+#pragma unroll
+  for (int a = 0; a < n; ++a) {
+    const int s = (int)(node[a * nf] >> 16);
+#pragma unroll
+    for (int i = 0; i < d; ++i) C[d * s + i] = fe[a * d + i];
+  }
+}
+
 // A node's d values at position j of a row-major array.
 template <int d>
 __device__ inline void get_row(const double* p, int j, double* x) {
@@ -835,11 +877,11 @@ __device__ inline void put_row(double* p, int j, const double* x) {
 // and record are prefetched into L2. What does not change between steps (X,
 // record, entries of the CTA's first patch) is staged before the previous
 // grid in the stream has finished.
-template <int d, bool LIN, bool FEXT>
-__global__ void __launch_bounds__(FanThreads<d>::value, (FanOccupancy<d, LIN>::value))
+template <int TY, bool LIN, bool FEXT>
+__global__ void __launch_bounds__(FanBuild<TY, LIN>::threads, (FanBuild<TY, LIN>::ctas))
     k_fan_step(DevModel m, DevPatches P, double dt0) {
   extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int T = FanThreads<d>::value;
+  constexpr int d = ET<TY>::dim, T = FanBuild<TY, LIN>::threads;
   __shared__ double warp_sums[T / 32];
   const FanLayout lay = fan_layout(P, d, FEXT);
   const int tid = threadIdx.x, G = gridDim.x;
@@ -961,15 +1003,19 @@ __global__ void __launch_bounds__(FanThreads<d>::value, (FanOccupancy<d, LIN>::v
       }
       fetch_desc(p + 2 * G, cur == 0 ? 2 : cur - 1);
     }
-    {  // 2. element forces, one thread per fan
+    {  // 2. element forces, one thread per fan (or element)
       const FanDesc& D = descs[cur];
       const bool mixed = D.mat == kMixed;
       const MatParams& mp = P.emat && !mixed ? m.mat_table[D.mat] : m.mats[0];
       const uint32_t* emat = mixed ? P.emat + D.elem0 : nullptr;
       const double *xs = nodes(lay.xs, D.ibeg), *ws = nodes(lay.ws, D.ibeg);
       const int nf = rec[0];
-      for (int t = tid; t < nf; t += T)
-        fan_forces<d, LIN>(rec, t, xs, ws, C, mp, m.mat_table, emat);
+      for (int t = tid; t < nf; t += T) {
+        if constexpr (TY == AKB_HEXAHEDRON_8)
+          hex_forces<LIN>(rec, t, xs, ws, C, mp, m.mat_table, emat);
+        else
+          fan_forces<d, LIN>(rec, t, xs, ws, C, mp, m.mat_table, emat);
+      }
     }
     {
       const bool ok = mbar_wait(mb + 8, it & 1);  // finishing inputs
@@ -1316,43 +1362,34 @@ cudaError_t raise_smem_limit(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// f(kernel) for the fan step's instantiation of a plan.
-template <int d, typename F>
-cudaError_t with_fan_kernel(bool lin, bool fext, F f) {
-  if (lin) return fext ? f(k_fan_step<d, true, true>) : f(k_fan_step<d, true, false>);
-  return fext ? f(k_fan_step<d, false, true>) : f(k_fan_step<d, false, false>);
+// f(kernel, threads) for the fan step's instantiation of a plan.
+template <int TY, bool LIN, typename F>
+cudaError_t with_fan_kernel(bool fext, F f) {
+  constexpr int threads = FanBuild<TY, LIN>::threads;
+  return fext ? f(k_fan_step<TY, LIN, true>, threads) : f(k_fan_step<TY, LIN, false>, threads);
 }
-
-template <int d>
-cudaError_t launch_fan(const DevModel& m, const DevPatches& p, double dt, bool fext, cudaStream_t s) {
-  const size_t bytes = fan_layout(p, d, fext).total;
-  return with_fan_kernel<d>(p.linear, fext, [&](auto kernel) {
-    const int grid = p.grid > 0 ? p.grid : p.resident[fext];
-    return launch_pdl(kernel, std::min(grid, p.npatch), FanThreads<d>::value, bytes, s, m, p, dt);
-  });
-}
-
-// Raises the kernels' shared-memory limit; resident: CTAs of the plan that are
-// on the device at the same time, without and with external forces.
-template <int d>
-cudaError_t configure_fan(const DevPatches& p, int device, int* resident) {
-  int sms = 0, per_sm = 0;
-  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lock(g_attr_mutex);
-  for (int k = 0; k < 2; ++k) {
-    const size_t bytes = fan_layout(p, d, k).total;
-    e = with_fan_kernel<d>(p.linear, k, [&](auto kernel) {
-      cudaError_t r = raise_smem_limit(kernel, bytes);
-      return r != cudaSuccess
-                 ? r
-                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel,
-                                                                 FanThreads<d>::value, bytes);
-    });
-    if (e != cudaSuccess) return e;
-    resident[k] = sms * per_sm;
+template <typename F>
+cudaError_t with_fan_kernel(int type, bool lin, bool fext, F f) {
+  switch (type) {
+  case AKB_TRIANGLE_3:
+    return lin ? with_fan_kernel<AKB_TRIANGLE_3, true>(fext, f)
+               : with_fan_kernel<AKB_TRIANGLE_3, false>(fext, f);
+  case AKB_TETRAHEDRON_4:
+    return lin ? with_fan_kernel<AKB_TETRAHEDRON_4, true>(fext, f)
+               : with_fan_kernel<AKB_TETRAHEDRON_4, false>(fext, f);
+  default:
+    return lin ? with_fan_kernel<AKB_HEXAHEDRON_8, true>(fext, f)
+               : with_fan_kernel<AKB_HEXAHEDRON_8, false>(fext, f);
   }
-  return cudaSuccess;
+}
+
+cudaError_t launch_fan(const DevModel& m, const DevPatches& p, double dt, bool fext,
+                       cudaStream_t s) {
+  const size_t bytes = fan_layout(p, m.dim, fext).total;
+  return with_fan_kernel(m.type, p.linear, fext, [&](auto kernel, int threads) {
+    const int grid = p.grid > 0 ? p.grid : p.resident[fext];
+    return launch_pdl(kernel, std::min(grid, p.npatch), threads, bytes, s, m, p, dt);
+  });
 }
 
 template <int T, typename S>
@@ -1378,7 +1415,22 @@ size_t fan_smem_bytes(const PatchHost& p, int dim) {
 }
 
 cudaError_t fan_configure(const DevModel& m, const DevPatches& p, int device, int* resident) {
-  return m.dim == 2 ? configure_fan<2>(p, device, resident) : configure_fan<3>(p, device, resident);
+  int sms = 0, per_sm = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(g_attr_mutex);
+  for (int k = 0; k < 2; ++k) {
+    const size_t bytes = fan_layout(p, m.dim, k).total;
+    e = with_fan_kernel(m.type, p.linear, k, [&](auto kernel, int threads) {
+      const cudaError_t r = raise_smem_limit(kernel, bytes);
+      return r != cudaSuccess
+                 ? r
+                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes);
+    });
+    if (e != cudaSuccess) return e;
+    resident[k] = sms * per_sm;
+  }
+  return cudaSuccess;
 }
 
 int patch_buffers(const DevPatches& p, int type, bool fp32) {
@@ -1415,7 +1467,7 @@ cudaError_t patch_configure(const DevModel& m, const DevPatches& p, bool fp32) {
 cudaError_t patch_step(const DevModel& m, const DevPatches& p, double dt, bool fp32,
                        bool fext, cudaStream_t s) {
   if (p.npatch == 0) return cudaSuccess;
-  if (p.fans) return m.dim == 2 ? launch_fan<2>(m, p, dt, fext, s) : launch_fan<3>(m, p, dt, fext, s);
+  if (p.fans) return launch_fan(m, p, dt, fext, s);
   switch (m.type) {
   case AKB_SEGMENT_2:
     return fp32 ? launch_patch<AKB_SEGMENT_2, float>(m, p, dt, fext, s)

@@ -78,7 +78,7 @@ inline int place_group(int dim) { return dim == 2 ? 8 : 16; }
 // runs (one sum instruction) hit G different banks (G = 16 for 8-byte
 // contributions, 32 for 4-byte ones), and the runs of a group have their
 // nodes at distinct positions mod 16 where the build could arrange it.
-// Fan record (FP64 triangles and tetrahedra): one per patch, staged by one
+// Fan record (FP64 steps but segments): one per patch, staged by one
 // bulk copy. A fan is a row of elements around a hinge (a node of triangles, an
 // edge of tetrahedra), element t having the hinge and the ring nodes r_t and
 // r_{t+1}; one thread computes a fan, loading each of its nodes once and
@@ -96,8 +96,9 @@ inline int place_group(int dim) { return dim == 2 ? 8 : 16; }
 //   cnt      per position the number of its contributions
 //   goff     per 32 positions, where their list starts in the record: entry q
 //            of position 32 g + l at goff[g] + 32 q + l
-// The slots are a colouring as the chunk records', 16 colours in 3D and 8 in 2D
-// (16-byte rows): scatter and sum are free of bank conflicts.
+// Hexahedra: fans of one element, row j its corner j. The slots are a colouring
+// as the chunk records', 16 colours in 3D and 8 in 2D (16-byte rows): scatter
+// and sum are free of bank conflicts.
 // Partial slot of rank r of shared node s (ns shared nodes; over: the node's
 // first slot for ranks >= 2).
 __host__ __device__ inline uint32_t partial_slot(uint32_t ns, uint32_t s, uint32_t over,
@@ -141,6 +142,8 @@ struct PatchHost {
   int64_t nslots = 0;
 };
 
+constexpr int kSingles = -1;
+
 // Builds the patches and the internal node order. target_elems: elements per
 // patch; max_nodes: local node cap (<= 60000); contrib_bytes: element vector
 // precision (8: FP64, 4: FP32); force_shared (per node, or null): nodes treated as shared
@@ -148,7 +151,8 @@ struct PatchHost {
 // them (the interface nodes of a partitioned mesh). fan_cap > 0 (triangles,
 // tetrahedra): fans of at most fan_cap elements, at most max_fans of them in a
 // patch, with fan records (throws std::length_error when a record does not
-// fit).
+// fit); fan_cap = kSingles: fan records of single elements, their rows the
+// element's corners in their own order.
 PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64_t ne, int dim,
                         int nnpe, int target_elems, int max_nodes, int contrib_bytes,
                         const uint8_t* force_shared = nullptr, int fan_cap = 0,
@@ -172,7 +176,8 @@ struct FanDesc {
 // Device copy of a PatchHost.
 struct DevPatches {
   int fans;  // fan records: the step runs k_fan_step
-  int linear;  // fans: every material is small-strain elastic
+  int linear;  // fans: every material is small-strain elastic (hexahedra: every
+               // element a parallelepiped)
   int npatch;
   int grid;  // 0: one CTA per patch; > 0: persistent grid of that many CTAs
   int resident[2];  // fans, grid 0: CTAs on the device at once (without, with f_ext)

@@ -317,7 +317,7 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
                         int nnpe, int target_elems, int max_nodes, int contrib_bytes,
                         const uint8_t* force_shared, int fan_cap, int max_fans) {
   PatchHost P;
-  P.fans = fan_cap > 0;
+  P.fans = fan_cap != 0;
   // 1. element centroids and their Morton keys
   double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
   for (int64_t i = 0; i < nn; ++i)
@@ -366,7 +366,18 @@ PatchHost build_patches(const double* X, const uint32_t* conn, int64_t nn, int64
     if (!std::is_sorted(keyed.begin(), keyed.end())) std::sort(keyed.begin(), keyed.end());
     std::vector<uint32_t> by_key(ne);
     for (int64_t e = 0; e < ne; ++e) by_key[e] = keyed[e].second;
-    F = build_fans(X, conn, nn, ne, dim, std::min(fan_cap, std::max(target_elems, 1)), by_key);
+    if (fan_cap == kSingles) {
+      F.elem.swap(by_key);
+      F.node.reserve((size_t)ne * nnpe);
+      for (uint32_t e : F.elem) {
+        F.node.insert(F.node.end(), conn + (int64_t)e * nnpe, conn + (int64_t)(e + 1) * nnpe);
+        F.nptr.push_back((int32_t)F.node.size());
+        F.eptr.push_back((int32_t)F.eptr.size());
+      }
+      F.closed.assign(ne, 0);
+    } else {
+      F = build_fans(X, conn, nn, ne, dim, std::min(fan_cap, std::max(target_elems, 1)), by_key);
+    }
     nu = F.count();
     // a fan's centroid and key: those of its elements' mean, and of its first element
     std::vector<double> fcen((size_t)nu * 3, 0.0);

@@ -1,0 +1,98 @@
+"""The fan step's branches at the sizes where they can go wrong, against the
+CPU oracle: one element to a few patches, affine and distorted hexahedra in
+one mesh or apart, several materials in a patch, external forces (the finish
+with f_ext), a persistent grid of one CTA, and plans too large for an SM (the
+chunk records). Tolerance: FP64 <= 1e-10 of the field's maximum
+(test_gpu_patch_layout.py)."""
+import numpy as np
+import pytest
+
+from akantu_b200 import _abi, configs
+from akantu_b200.mesh import box_hexahedron8, box_tetrahedron4, plate_triangle3
+from oracle.oracle import OracleModel, material_desc
+from tests.golden_cases import OracleAdapter
+
+pytestmark = pytest.mark.gpu
+
+NEO = configs.neohookean_from_lame(1.0e6, 0.4e6, 1100.0)
+ELASTIC = dict(kind=_abi.MATERIAL_ELASTIC, rho=2700.0, E=70e9, nu=0.33)
+STIFF = dict(kind=_abi.MATERIAL_ELASTIC, rho=7800.0, E=210e9, nu=0.3)
+FINITE = dict(kind=_abi.MATERIAL_ELASTIC, rho=2700.0, E=70e9, nu=0.33, finite_deformation=True)
+
+
+def build(kind, n, jitter):
+    mesh = {"hex": lambda: box_hexahedron8(*n, *[0.1 * k for k in n]),
+            "tet": lambda: box_tetrahedron4(*n, *[0.1 * k for k in n]),
+            "tri": lambda: plate_triangle3(n[0], n[1], 0.1 * n[0], 0.1 * n[1])}[kind]()
+    if jitter:  # moves the nodes of the right half only: affine elements remain
+        x = mesh.nodes
+        rng = np.random.default_rng(1)
+        move = x[:, 0] > 0.05 * n[0]
+        x[move] += rng.uniform(-0.01, 0.01, x[move].shape)
+    return mesh
+
+
+CASES = [
+    ("hex", (1, 1, 1), NEO, 0, {}), ("hex", (3, 2, 1), NEO, 1, {}), ("hex", (9, 8, 7), NEO, 0, {}),
+    ("hex", (11, 7, 5), NEO, 1, {}), ("hex", (6, 5, 9), ELASTIC, 1, dict(patch_grid=1)),
+    ("hex", (8, 8, 8), NEO, 0, dict(patch_elements=512, patch_nodes=800)),
+    ("tet", (1, 1, 1), ELASTIC, 0, {}), ("tet", (7, 6, 5), [ELASTIC, STIFF], 1, {}),
+    ("tet", (9, 9, 4), FINITE, 0, dict(patch_grid=1)), ("tet", (10, 9, 8), ELASTIC, 1,
+                                                       dict(patch_elements=1, patch_nodes=8)),
+    ("tri", (1, 1), ELASTIC, 0, {}), ("tri", (40, 31), [STIFF, ELASTIC], 1, {}),
+    ("tri", (64, 3), FINITE, 1, dict(patch_elements=100, patch_nodes=90, patch_grid=1)),
+    ("tri", (60, 60), ELASTIC, 0, dict(patch_elements=8000, patch_nodes=6000)),
+]
+
+
+@pytest.mark.parametrize("load", [False, True], ids=["free", "loaded"])
+@pytest.mark.parametrize("kind,n,mats,jitter,patch", CASES)
+def test_against_oracle(kind, n, mats, jitter, patch, load):
+    from akantu_b200.model import SolidMechanicsModel, material_from_dict
+    mesh = build(kind, n, jitter)
+    mats = mats if isinstance(mats, list) else [mats]
+    em = None if len(mats) == 1 else (np.arange(mesh.getNbElement()) % 3 == 0).astype(np.uint32)
+    x = mesh.nodes
+    rng = np.random.default_rng(2)
+    blocked = np.zeros(x.shape, dtype=np.uint8)
+    blocked[np.isclose(x[:, 0], 0.0)] = 1
+    v0 = rng.normal(0.0, 0.05 if mats[0] is NEO else 1.0, x.shape)
+    v0[blocked != 0] = 0.0
+    fext = np.zeros(x.shape)
+    if load:
+        fext[np.isclose(x[:, 0], x[:, 0].max()), 0] = 1e-5 * mats[0]["E"] * 0.01
+    cpu = OracleAdapter(mesh, mats)
+    if em is not None:
+        cpu.m = OracleModel(mesh, [material_desc(**m) for m in mats], em)
+    dev = SolidMechanicsModel(mesh, [material_from_dict(m) for m in mats], element_material=em,
+                              precision=_abi.MODE_FP64, **patch)
+    dev.initFull()
+    dt = 0.5 * dev.getStableTimeStep()
+    dev.setBlockedDOFs(blocked)
+    dev.setField(_abi.FIELD_VELOCITY, v0)
+    dev.setField(_abi.FIELD_EXTERNAL_FORCE, fext)
+    dev.setTimeStep(dt)
+    cpu.set_blocked(blocked)
+    cpu.set(_abi.FIELD_VELOCITY, v0)
+    cpu.set(_abi.FIELD_EXTERNAL_FORCE, fext)
+    cpu.set_time_step(dt)
+    dev.solveSteps(40)
+    cpu.solve_steps(40)
+    for f in (_abi.FIELD_DISPLACEMENT, _abi.FIELD_VELOCITY):
+        a, b = np.array(dev.getField(f)), cpu.get(f)
+        assert np.abs(a - b).max() <= 1e-10 * np.abs(b).max(), f
+    v = np.array(dev.getVelocity())
+    m = np.array(dev.getMass())
+    assert dev.getEnergy("kinetic") == pytest.approx(0.5 * (m * v * v).sum(), rel=1e-12)
+    dev.close()
+
+
+def test_a_patch_above_an_sm_is_refused():
+    """4913 nodes in one patch: neither the fan record's staging nor the chunk
+    records' fits 227 KB."""
+    from akantu_b200._lib import AkbError
+    from akantu_b200.model import SolidMechanicsModel, material_from_dict
+    m = SolidMechanicsModel(box_hexahedron8(16, 16, 16, 1.6, 1.6, 1.6), [material_from_dict(NEO)],
+                            precision=_abi.MODE_FP64, patch_elements=4096, patch_nodes=6000)
+    with pytest.raises(AkbError, match="shared memory"):
+        m.initFull()
