@@ -46,7 +46,7 @@ SIGNATURES = {
     "akb_compute_stresses": (I32, [P]),
     "akb_get_energy": (I32, [P, I32, PD]),
     "akb_get_energy_async": (I32, [P, I32, P]),
-    "akb_apply_dirichlet": (I32, [P, PU32, I64, I32, PD]),
+    "akb_apply_dirichlet": (I32, [P, P, I64, I32, P]),
     "akb_time_kernels": (I32, [P, I64, PD, I32]),
     "akb_kernel_name": (C.c_char_p, [P, I32]),
     "akb_batch_create": (I32, [C.POINTER(_abi.BatchDesc), C.POINTER(_abi.ModelOptions),

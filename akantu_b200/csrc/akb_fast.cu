@@ -183,6 +183,16 @@ __global__ void k_qp_forces(DevModel m) {
   }
 }
 
+__device__ inline void set_dirichlet(const DevModel& m, uint32_t node, int c, double value,
+                                     const uint32_t* perm, double* w) {
+  if (node >= m.nn) return;  // out-of-range node ids are ignored
+  if (perm) node = perm[node];
+  const int64_t i = (int64_t)node * m.dim + c;
+  m.blocked[i] = 1;
+  m.u[i] = value;
+  if (w) w[i] = value;  // a blocked DOF's predicted displacement is its u
+}
+
 // comp >= 0: one thread per listed node, that component; comp < 0: one
 // thread per (listed node, component), values row per node. Launched with
 // programmatic serialization behind the step's last kernel, it waits for
@@ -195,14 +205,19 @@ __global__ void k_apply_dirichlet(DevModel m, const uint32_t* nodes, int64_t n, 
   const int ncomp = comp < 0 ? m.dim : 1;
   if (k >= n * ncomp) return;
   const int64_t q = k / ncomp;
-  const int c = comp < 0 ? (int)(k - q * ncomp) : comp;
-  uint32_t node = nodes[q];
-  if (node >= m.nn) return;  // out-of-range node ids are ignored
-  if (perm) node = perm[node];
-  const int64_t i = (int64_t)node * m.dim + c;
-  m.blocked[i] = 1;
-  m.u[i] = values[k];
-  if (w) w[i] = values[k];  // a blocked DOF's predicted displacement is its u
+  set_dirichlet(m, nodes[q], comp < 0 ? (int)(k - q * ncomp) : comp, values[k], perm, w);
+}
+
+// The same with the nodes and values in the kernel's parameters: a short list
+// (kInlineDirichlet values) needs no upload, no staging slot and no events.
+__global__ void k_apply_dirichlet_inline(DevModel m, InlineDirichlet list, int n, int comp,
+                                         const uint32_t* perm, double* w) {
+  grid_wait();
+  grid_launch_dependents();
+  const int k = threadIdx.x, ncomp = comp < 0 ? m.dim : 1;
+  if (k >= n * ncomp) return;
+  const int q = k / ncomp;
+  set_dirichlet(m, list.nodes[q], comp < 0 ? k - q * ncomp : comp, list.values[k], perm, w);
 }
 
 }  // namespace
@@ -212,6 +227,11 @@ cudaError_t apply_dirichlet(const DevModel& m, const uint32_t* nodes, int64_t n,
                             cudaStream_t s) {
   return launch_pdl(k_apply_dirichlet, blocks_for(comp < 0 ? n * m.dim : n), kThreads, 0, s, m,
                     nodes, n, comp, values, perm, w);
+}
+
+cudaError_t apply_dirichlet_inline(const DevModel& m, const InlineDirichlet& list, int n, int comp,
+                                   const uint32_t* perm, double* w, cudaStream_t s) {
+  return launch_pdl(k_apply_dirichlet_inline, 1, kInlineDirichlet, 0, s, m, list, n, comp, perm, w);
 }
 
 cudaError_t user_qp_gradients(const DevModel& m, cudaStream_t s) {

@@ -118,6 +118,16 @@ cudaError_t apply_dirichlet(const DevModel& m, const uint32_t* nodes, int64_t n,
                             const double* values, const uint32_t* perm, double* w,
                             cudaStream_t s);
 
+// A list short enough for the kernel's parameters (the model takes about 0.7 of
+// their 4 KB): at most kInlineDirichlet values.
+constexpr int kInlineDirichlet = 192;
+struct InlineDirichlet {
+  double values[kInlineDirichlet];
+  uint32_t nodes[kInlineDirichlet];
+};
+cudaError_t apply_dirichlet_inline(const DevModel& m, const InlineDirichlet& list, int n, int comp,
+                                   const uint32_t* perm, double* w, cudaStream_t s);
+
 // Reductions (akb_reduce.cu). Scratch holds per-block partial results.
 cudaError_t stable_dt(const DevModel& m, double* d_scratch, int scratch_len,
                       double* d_out, cudaStream_t s);

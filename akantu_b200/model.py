@@ -524,10 +524,11 @@ class SolidMechanicsModel:
         self._sync_in()
         n = np.ascontiguousarray(nodes, dtype=np.uint32)
         shape = n.shape + ((self.dim,) if component == _abi.ALL_COMPONENTS else ())
-        v = np.ascontiguousarray(np.broadcast_to(values, shape), dtype=np.float64)
-        check(lib().akb_apply_dirichlet(self.handle, n.ctypes.data_as(C.POINTER(C.c_uint32)),
-                                        n.size, int(component),
-                                        v.ctypes.data_as(C.POINTER(C.c_double))))
+        if getattr(values, "shape", None) != shape:
+            values = np.broadcast_to(values, shape)
+        v = np.ascontiguousarray(values, dtype=np.float64)
+        check(lib().akb_apply_dirichlet(self.handle, n.ctypes.data, n.size, int(component),
+                                        v.ctypes.data))
 
     def applyBC(self, functor, group):
         """applyBC(functor, group) (py_solid_mechanics_model.cc:58-67,
