@@ -22,8 +22,8 @@
 //            A = dZ_l and B = H_{l-1} both MN-major (samples are K);
 //   Adam on FP32 master weights, then the BF16 copies are repacked.
 // Weights and activation tiles are staged by TMA bulk copies completing on an
-// mbarrier (no multicast); in the forward and backward passes the next
-// layer's weights are copied while the current layer's epilogue runs. Each
+// mbarrier (no multicast); in the forward and backward passes weights of the
+// next layer are copied while the current layer's epilogue runs. Each
 // wait (copy or MMA completion) is bounded: past the limit the kernel raises
 // the error flag, waits (bounded) for what is still in flight, frees its
 // tensor memory and returns.
@@ -54,7 +54,8 @@ struct Net {
   int nin, nout;                // real input / output counts
   int K[kMaxLayers], N[kMaxLayers];    // padded shapes (K[0] = N[nl-1] = 16)
   int Kr[kMaxLayers], Nr[kMaxLayers];  // real shapes
-  const __nv_bfloat16* W[kMaxLayers];  // packed N x K
+  int ks[kMaxLayers];                  // columns of a weight slice (slice_cols)
+  const __nv_bfloat16* W[kMaxLayers];  // packed N x K in slices (w_off)
   const __nv_bfloat16* Wt[kMaxLayers]; // packed K x N
   const float* b[kMaxLayers];          // N (zero past the real outputs)
   float in_shift[kIO], in_scale[kIO], out_shift[kIO], out_scale[kIO];
@@ -75,6 +76,18 @@ struct Bufs {
 
 __host__ __device__ inline size_t pk_off(int r, int c, int cols) {
   return ((size_t)(r >> 3) * (cols >> 3) + (c >> 3)) * 128 + (r & 7) * 16 + (c & 7) * 2;
+}
+
+// The forward pass's weights W (N x K) are packed in slices of KS columns (K
+// for the MMA), each a packed N x KS matrix of at most kSliceBytes: an MMA then
+// takes the layer's whole width, and a slice is one contiguous copy.
+constexpr size_t kSliceBytes = (size_t)32 * kMaxWidth * 2;
+__host__ __device__ inline int slice_cols(int N, int K) {  // a multiple of 16 that divides K
+  const int most = (int)(kSliceBytes / (2 * (size_t)N));
+  return K < most ? K : most;
+}
+__host__ __device__ inline size_t w_off(int r, int c, int N, int ks) {
+  return (size_t)(c / ks) * N * ks * 2 + pk_off(r, c % ks, ks);
 }
 
 // ------------------------------------------------------------ PTX wrappers
@@ -232,38 +245,48 @@ __device__ inline void gemm_kmajor(uint32_t tmem_d, uint32_t a, uint32_t b, int 
     mma(tmem_d, sdesc(a + s * 256, 128, 16 * K), sdesc(b + s * 256, 128, 16 * K), id, s > 0);
 }
 
+// The same for columns [k0, k0 + ks) of A and a packed N x ks slice of B,
+// added to tmem_d unless k0 is 0.
+__device__ inline void gemm_slice(uint32_t tmem_d, uint32_t a, uint32_t b, int K, int k0, int ks,
+                                  int N) {
+  const uint32_t id = idesc(kTile, N, false, false);
+  uint64_t da = sdesc(a + k0 * 16, 128, 16 * K), db = sdesc(b, 128, 16 * ks);
+  for (int s = 0; s < ks / 16; ++s, da += 16, db += 16)  // 256 bytes on
+    mma(tmem_d, da, db, id, k0 + s > 0);
+}
+
 struct Shared {
   unsigned char* act;  // 128 x 256 packed BF16 (64 KB)
   unsigned char* wgt;  // 256 x 256 packed BF16 (128 KB)
-  float* bias;         // forward: every layer's biases (kMaxWidth per layer); backward: 256
+  float* bias;         // 256 (the backward pass's loss reduction)
   uint64_t* mbar;      // [0] MMA completion, [1] weights landed
   uint32_t* tmem_holder;
-  double* hnorm;       // 128: |H| of each row (stress mode)
 };
 
 constexpr size_t kActBytes = (size_t)kTile * kMaxWidth * 2;
 constexpr size_t kWgtBytes = (size_t)kMaxWidth * kMaxWidth * 2;
-// The forward pass stages a layer's weights in slices of output rows (a
-// contiguous block of the packed N x K matrix; 64 rows of a 256-wide layer),
-// so that its shared memory (~97 KB) lets two CTAs share an SM: one CTA's
-// epilogue (TMEM -> bias -> SiLU -> BF16) runs while the other's MMAs use
-// the tensor cores.
-constexpr size_t kSliceBytes = (size_t)64 * kMaxWidth * 2;
-constexpr size_t kTail = kMaxLayers * kMaxWidth * 4 + 64 + kTile * 8;  // biases, barriers, |H|
-constexpr size_t kFwdSmem = kActBytes + kSliceBytes + kTail;
-constexpr size_t kBwdSmem = kActBytes + kWgtBytes + kTail;
+constexpr size_t kBwdSmem = kActBytes + kWgtBytes + kMaxWidth * 4 + 64;
 
-__device__ inline Shared carve(unsigned char* smem, size_t wgt_bytes) {
+__device__ inline Shared carve(unsigned char* smem) {
   Shared s;
   s.act = smem;
   s.wgt = smem + kActBytes;
-  unsigned char* t = smem + kActBytes + wgt_bytes;
+  unsigned char* t = s.wgt + kWgtBytes;
   s.bias = reinterpret_cast<float*>(t);
-  s.mbar = reinterpret_cast<uint64_t*>(t + kMaxLayers * kMaxWidth * 4);
+  s.mbar = reinterpret_cast<uint64_t*>(t + kMaxWidth * 4);
   s.tmem_holder = reinterpret_cast<uint32_t*>(s.mbar + 2);
-  s.hnorm = reinterpret_cast<double*>(t + kMaxLayers * kMaxWidth * 4 + 64);
   return s;
 }
+
+// The forward pass streams every layer's weights through a ring of slices
+// (w_off: 32 columns of a 256-wide layer), which one thread keeps full across
+// layers and under the epilogues. Activations, ring, barriers and the TMEM
+// address take 112.1 KB, so that two CTAs share an SM: one's epilogue (TMEM ->
+// bias -> SiLU -> BF16) runs beside the other's MMAs. (Slices twice as large
+// leave one CTA an SM: 1000 samples 24.9 us, but 262144 take 275 us.)
+constexpr int kRing = 3;
+constexpr size_t kFwdSmem = kActBytes + kRing * kSliceBytes + 128;
+static_assert(2 * (kFwdSmem + 1024) <= 228 * 1024, "two CTAs an SM");
 
 // Stress mode of the forward pass (MaterialFE2 with the surrogate): the
 // inputs are displacement gradients H ([nb][9], column-major per point), the
@@ -292,11 +315,11 @@ __device__ inline double det_i_plus(const double* H) {  // det(I + H), H column-
 // The normalised inputs of row r of a tile (columns 8 half .. 8 half + 7 of
 // 16) into the packed A tile `act`: x's columns, or in stress mode the
 // features (H / r, log r) of the row's displacement gradient, whose |H| goes
-// to hnorm[r] and whose envelope test (by the half-0 threads, whole warps)
+// to hnorm (half 0) and whose envelope test (by the half-0 threads, whole warps)
 // appends the row to the fallback list.
 template <bool STRESS>
 __device__ inline void stage_inputs(const Net& net, int64_t nb, const double* __restrict__ x,
-                                    unsigned char* act, double* hnorm, int r, int half,
+                                    unsigned char* act, double& hnorm, int r, int half,
                                     int64_t row, int tid, const StressArgs& sa, float* v) {
   if (STRESS) {
     double H[9], n2 = 0.0;
@@ -314,7 +337,7 @@ __device__ inline void stage_inputs(const Net& net, int64_t nb, const double* __
     }
     store8(act, r, 8 * half, 16, v);
     if (half == 0) {  // whole warps: one row per lane
-      hnorm[r] = hn;
+      hnorm = hn;
       if (sa.count) {
         double hmax = 0.0;
 #pragma unroll
@@ -339,99 +362,113 @@ __device__ inline void stage_inputs(const Net& net, int64_t nb, const double* __
   }
 }
 
-// Output rows per weight slice of layer l: as many as the buffer holds (a
-// multiple of 16: whole row groups, a valid MMA N), at most the layer's N.
-__device__ inline int slice_rows(const Net& net, int l) {
-  return min(net.N[l], (int)(kSliceBytes / (2 * (size_t)net.K[l])) & ~15);
-}
-// Rows of slice j of layer l, its bytes and its source (rows [rows0 j, ...)
-// of the packed N x K matrix are one contiguous block).
-__device__ inline int slice_n(const Net& net, int l, int j) {
-  return min(slice_rows(net, l), net.N[l] - slice_rows(net, l) * j);
-}
-__device__ inline uint32_t slice_bytes(const Net& net, int l, int j) {
-  return (uint32_t)(slice_n(net, l, j) * net.K[l] * 2);
-}
-__device__ inline const void* slice_src(const Net& net, int l, int j) {
-  return reinterpret_cast<const unsigned char*>(net.W[l]) +
-         (size_t)slice_rows(net, l) * j * net.K[l] * 2;
-}
-
-template <bool TRAIN, bool STRESS = false>
+// One CTA per tile of 128 samples, two per SM. Bound by the epilogues (one
+// special-function operation an element) and by the chain slice landed -> MMAs
+// issued -> slice free again. The time of an MMA hardly falls with its width
+// below 256 columns, so that a slice holds columns of the whole layer: 16 MMAs
+// for a 256-wide layer instead of 64 with slices of 64 rows. Thread 0 only
+// waits for slices and issues; the copies have a thread of another warp, whose
+// wait for a slice to be free holds up nobody (with one thread doing both, the
+// wait was 500 of a slice's 1300 cycles). Stress calls, 4 x 256 hidden: 1000
+// points 29.0 -> 22.9 us, 20000 33.3 -> 27.1, 262144 206 -> 164, 500000
+// 396 -> 314; a step of 32^3 macro elements 273 -> 231 us, of 8^3 77 -> 65.
+template <bool TRAIN, bool STRESS>
 __global__ void __launch_bounds__(kFwdThreads, 2)
     k_forward(Net net, int64_t nb, const double* __restrict__ x, double* __restrict__ y,
               Bufs bufs, StressArgs sa = StressArgs{}) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  Shared s = carve(smem, kSliceBytes);
+  unsigned char *act = smem, *ring = smem + kActBytes;
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(ring + kRing * kSliceBytes);
+  uint32_t* holder = reinterpret_cast<uint32_t*>(mbar + 2 * kRing + 1);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int r = tid & (kTile - 1), half = tid >> 7;  // row in the tile, column half
   const int64_t tile = blockIdx.x;
   const int64_t row = tile * kTile + r;
-  const uint32_t mb_mma = saddr(s.mbar), mb_w = saddr(s.mbar + 1);
-  if (warp == 0) tmem_alloc(saddr(s.tmem_holder), 256);
-  if (tid == 0) {
-    mbar_init(mb_mma);
-    mbar_init(mb_w);
-    bulk_load(saddr(s.wgt), slice_src(net, 0, 0), slice_bytes(net, 0, 0), mb_w);
+  double hnorm = 0.0;
+  auto full = [&](int s) { return saddr(mbar + s); };
+  auto empty = [&](int s) { return saddr(mbar + kRing + s); };
+  const uint32_t mb_done = saddr(mbar + 2 * kRing);
+  if (warp == 0) tmem_alloc(saddr(holder), 256);
+  // the ring: thread 32 loads slice after slice (ll, lj: the next one), thread 0
+  // consumes them
+  constexpr int kLoader = 32;
+  int loaded = 0, used = 0, ll = 0, lj = 0;
+  bool ok = true;
+  auto load_next = [&]() {
+    const int s = loaded % kRing, ks = net.ks[ll];
+    if (loaded >= kRing && !mbar_wait(empty(s), (loaded / kRing - 1) & 1)) {
+      ok = false;
+      return;
+    }
+    const uint32_t bytes = (uint32_t)(net.N[ll] * ks * 2);
+    bulk_load(saddr(ring + s * kSliceBytes),
+              reinterpret_cast<const unsigned char*>(net.W[ll]) + (size_t)lj * bytes, bytes, full(s));
+    ++loaded;
+    if (++lj * ks >= net.K[ll]) {
+      lj = 0;
+      ++ll;
+    }
+  };
+  if (tid == kLoader) {
+    for (int k = 0; k < 2 * kRing + 1; ++k) mbar_init(saddr(mbar + k));
+    for (int k = 0; k < kRing && ll < net.nl; ++k) load_next();
   }
-  // every layer's biases, once (the first barrier below publishes them)
-  for (int l = 0; l < net.nl; ++l)
-    for (int c = tid; c < net.N[l]; c += kFwdThreads) s.bias[l * kMaxWidth + c] = net.b[l][c];
   // inputs, normalised, padded to 16 columns (8 per thread)
   {
     float v[8];
-    stage_inputs<STRESS>(net, nb, x, s.act, s.hnorm, r, half, row, tid, sa, v);
+    stage_inputs<STRESS>(net, nb, x, act, hnorm, r, half, row, tid, sa, v);
     if (TRAIN) store8(bufs.act[0] + tile * (size_t)kTile * 16 * 2, r, 8 * half, 16, v);
   }
   fence_smem_async();  // the A tile, written by this thread, before the MMAs read it
   fence_before();
   __syncthreads();
   fence_after();
-  const uint32_t tmem = *s.tmem_holder;
-  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-  // A layer's weights arrive slice by slice (TMA bulk into one buffer):
-  // slice j's MMAs write accumulator columns [kSlice j, ...); the next slice
-  // (or the next layer's first, during this layer's epilogue) is copied as
-  // soon as they completed.
-  uint32_t pm = 0, pw = 0;
-  bool ok = true, w_pending = true, m_pending = false;
-  for (int l = 0; l < net.nl && ok; ++l) {
+  const uint32_t tmem = *holder;
+  const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  int l = 0;
+  for (; l < net.nl; ++l) {
     const int K = net.K[l], N = net.N[l];
-    const int rows0 = slice_rows(net, l);
-    const int nslices = (N + rows0 - 1) / rows0;
-    const float* bias = s.bias + l * kMaxWidth;
-    for (int j = 0; j < nslices && ok; ++j) {
-      ok = mbar_wait(mb_w, pw);
-      if (!ok) break;
-      pw ^= 1;
-      w_pending = false;
-      if (tid == 0) {
-        fence_after();
-        gemm_kmajor(tmem + rows0 * j, saddr(s.act), saddr(s.wgt), K, slice_n(net, l, j));
-        mma_commit(mb_mma);
-      }
-      m_pending = true;
-      ok = mbar_wait(mb_mma, pm);
-      if (!ok) break;
-      pm ^= 1;
-      m_pending = false;
+    if (tid == 0) {
       fence_after();
-      if (j + 1 < nslices) {
-        if (tid == 0) bulk_load(saddr(s.wgt), slice_src(net, l, j + 1), slice_bytes(net, l, j + 1), mb_w);
-        w_pending = true;
-      } else if (l + 1 < net.nl) {
-        if (tid == 0) bulk_load(saddr(s.wgt), slice_src(net, l + 1, 0), slice_bytes(net, l + 1, 0), mb_w);
-        w_pending = true;
+      const int ks = net.ks[l];
+      for (int k0 = 0; k0 < K && ok; k0 += ks) {
+        const int s = used % kRing;
+        ok = mbar_wait(full(s), (used / kRing) & 1);
+        if (!ok) break;
+        gemm_slice(tmem, saddr(act), saddr(ring + s * kSliceBytes), K, k0, ks, N);
+        mma_commit(empty(s));
+        ++used;
       }
+      if (ok) mma_commit(mb_done);
+    } else if (tid == kLoader) {
+      // this layer's slices and, into the places they leave, the next one's first
+      used += K / net.ks[l];
+      while (ok && ll < net.nl && loaded < used + kRing) load_next();
     }
-    if (!ok) break;
+    // lanes that waited on the barrier below while one of their warp still
+    // issues would suspend the warp, 3000 cycles at a time
+    __syncwarp();
+    // (a wait that gave up in one thread ends the layer loop in all)
+    if (ok) ok = mbar_wait(mb_done, l & 1);
+    if (__syncthreads_or(!ok)) {
+      ok = false;
+      break;
+    }
+    fence_after();
+    const float* __restrict__ bias = net.b[l];
     const bool last = l == net.nl - 1;
     if (!last) {
       for (int c0 = half * (N >> 1); c0 < (half + 1) * (N >> 1); c0 += 32) {
         float v[32];
-        tmem_ld32(tmem + lane_base + c0, v);
+        tmem_ld32(mine + c0, v);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] += bias[c0 + j];
+        for (int q = 0; q < 8; ++q) {
+          const float4 b4 = __ldg(reinterpret_cast<const float4*>(bias + c0) + q);
+          v[4 * q] += b4.x;
+          v[4 * q + 1] += b4.y;
+          v[4 * q + 2] += b4.z;
+          v[4 * q + 3] += b4.w;
+        }
         if (TRAIN && row < nb) {  // the pre-activations: eight 16-byte stores
           float4* z4 = reinterpret_cast<float4*>(bufs.z[l] + (size_t)row * N + c0);
 #pragma unroll
@@ -441,18 +478,18 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = silu(v[j]);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) store8(s.act, r, c0 + 8 * q, N, v + 8 * q);
+        for (int q = 0; q < 4; ++q) store8(act, r, c0 + 8 * q, N, v + 8 * q);
         if (TRAIN) {
           unsigned char* g = bufs.act[l + 1] + tile * (size_t)kTile * N * 2;
 #pragma unroll
           for (int q = 0; q < 4; ++q) store8(g, r, c0 + 8 * q, N, v + 8 * q);
         }
       }
-    } else if (half == 0) {  // warp-uniform: warps 0-3 read the 16 output columns
+    } else if (half == 0) {  // warp-uniform: warps 0-3 of a tile read the 16 output columns
       float v[16];
-      tmem_ld16(tmem + lane_base, v);
+      tmem_ld16(mine, v);
       if (row < nb) {
-        const double scale = STRESS ? s.hnorm[r] : 1.0;
+        const double scale = STRESS ? hnorm : 1.0;
         for (int j = 0; j < 16; ++j) {
           const float yy = v[j] + bias[j];
           if (TRAIN) bufs.ynorm[row * 16 + j] = yy;
@@ -465,11 +502,13 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
     fence_before();
     __syncthreads();  // TMEM read and activations written before the next MMA
   }
-  if (!ok) {  // drain the copy / MMA still in flight before leaving (bounded)
-    if (w_pending) mbar_wait(mb_w, pw);
-    if (m_pending) mbar_wait(mb_mma, pm);
-    if (tid == 0) atomicExch(net.error, 1);
+  // drain the copies and MMAs still in flight before leaving (bounded)
+  if (!ok && tid == 0) {
+    atomicExch(net.error, 1);
+    for (int k = max(0, used - kRing); k < used; ++k) mbar_wait(empty(k % kRing), (k / kRing) & 1);
   }
+  if (!ok && tid == kLoader)
+    for (int k = max(0, loaded - kRing); k < loaded; ++k) mbar_wait(full(k % kRing), (k / kRing) & 1);
   __syncthreads();
   if (warp == 0) tmem_free(tmem, 256);
 }
@@ -481,7 +520,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
 __global__ void __launch_bounds__(kFwdThreads, 1)
     k_backward(Net net, int64_t nb, const double* __restrict__ target, Bufs bufs) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  Shared s = carve(smem, kWgtBytes);
+  Shared s = carve(smem);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int r = tid & (kTile - 1), half = tid >> 7;  // row in the tile, column half
   const int64_t tile = blockIdx.x;
@@ -543,6 +582,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       gemm_kmajor(tmem, saddr(s.act), saddr(s.wgt), K, N);
       mma_commit(mb_mma);
     }
+    __syncwarp();  // (as in k_forward)
     m_pending = true;
     ok = mbar_wait(mb_mma, pm);
     if (!ok) break;
@@ -692,9 +732,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (tid == 0)
       bulk_load2(saddr(sa), A + t * (size_t)kTile * ca * 2, (uint32_t)(kTile * ca * 2), saddr(sb),
                  B + t * (size_t)kTile * cb * 2, (uint32_t)(kTile * cb * 2), mb_t);
+    __syncwarp();  // (as in k_forward: nobody waits before thread 0 has issued)
     t_pending = true;
-    ok = mbar_wait(mb_t, pt);
-    if (ok) {
+    ok = __all_sync(0xffffffffu, mbar_wait(mb_t, pt));
+    if (ok) {  // whole warps
       pt ^= 1;
       t_pending = false;
       if (tid == 0) {
@@ -706,6 +747,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 sdesc(saddr(sb) + s * 2 * 16 * cb, 16 * cb, 128), id, (t > t0 || s > 0) ? 1u : 0u);
         mma_commit(mb_mma);
       }
+      __syncwarp();
       m_pending = true;
       ok = mbar_wait(mb_mma, pm);
       if (ok) {
@@ -788,14 +830,14 @@ __global__ void k_adam(Net net, Layout lay, float* p, const float* g, float* m1,
   const int r = t / net.Kr[l], c = t % net.Kr[l];
   const __nv_bfloat16 h = __float2bfloat16_rn(x);
   *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(const_cast<__nv_bfloat16*>(net.W[l])) +
-                                    pk_off(r, c, net.K[l])) = h;
+                                    w_off(r, c, net.N[l], net.ks[l])) = h;
   *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(const_cast<__nv_bfloat16*>(net.Wt[l])) +
                                     pk_off(c, r, net.N[l])) = h;
 }
 
 // Packed BF16 W (N x K) and W^T (K x N) of one layer from the real FP32
 // row-major weights (nr x kr) and bias, zero padded.
-__global__ void k_pack(const float* w, const float* bias, int nr, int kr, int N, int K,
+__global__ void k_pack(const float* w, const float* bias, int nr, int kr, int N, int K, int ks,
                        __nv_bfloat16* W, __nv_bfloat16* Wt, float* b) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < N) b[k] = k < nr ? bias[k] : 0.0f;
@@ -803,7 +845,7 @@ __global__ void k_pack(const float* w, const float* bias, int nr, int kr, int N,
   const int r = k / K, c = k % K;
   const float v = (r < nr && c < kr) ? w[(size_t)r * kr + c] : 0.0f;
   const __nv_bfloat16 h = __float2bfloat16_rn(v);
-  *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(W) + pk_off(r, c, K)) = h;
+  *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(W) + w_off(r, c, N, ks)) = h;
   *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(Wt) + pk_off(c, r, N)) = h;
 }
 
@@ -853,7 +895,7 @@ akb_status repack(akb_mlp* m) {
     const Net& n = m->net;
     const int total = n.N[l] * n.K[l];
     k_pack<<<(total + 255) / 256, 256, 0, m->stream>>>(
-        m->d_params + m->w_off[l], m->d_params + m->b_off[l], n.Nr[l], n.Kr[l], n.N[l], n.K[l],
+        m->d_params + m->w_off[l], m->d_params + m->b_off[l], n.Nr[l], n.Kr[l], n.N[l], n.K[l], n.ks[l],
         const_cast<__nv_bfloat16*>(n.W[l]), const_cast<__nv_bfloat16*>(n.Wt[l]),
         const_cast<float*>(n.b[l]));
     AKB_CUDA_TRY(cudaGetLastError());
@@ -899,7 +941,8 @@ akb_status gradients(akb_mlp* m, int64_t nb, const double* x, const double* targ
   if ((st = ensure_workspace(m, ntiles)) != AKB_OK) return st;
   const Net& n = m->net;
   AKB_CUDA_TRY(cudaMemsetAsync(m->d_error, 0, sizeof(int), m->stream));
-  k_forward<true><<<(unsigned)ntiles, kFwdThreads, kFwdSmem, m->stream>>>(n, nb, x, nullptr, m->bufs);
+  k_forward<true, false><<<(unsigned)ntiles, kFwdThreads, kFwdSmem, m->stream>>>(n, nb, x, nullptr,
+                                                                                 m->bufs);
   AKB_CUDA_TRY(cudaGetLastError());
   k_backward<<<(unsigned)ntiles, kFwdThreads, kBwdSmem, m->stream>>>(n, nb, target, m->bufs);
   AKB_CUDA_TRY(cudaGetLastError());
@@ -976,6 +1019,7 @@ akb_status akb_mlp_create(int32_t nb_inputs, int32_t nb_outputs, int32_t width,
   for (int l = 0; l < n.nl; ++l) {
     n.K[l] = l == 0 ? kIO : width;
     n.N[l] = l == n.nl - 1 ? kIO : width;
+    n.ks[l] = slice_cols(n.N[l], n.K[l]);
     n.Kr[l] = l == 0 ? nb_inputs : width;
     n.Nr[l] = l == n.nl - 1 ? nb_outputs : width;
     m->w_off.push_back(m->nparams);
@@ -1016,8 +1060,8 @@ akb_status akb_mlp_create(int32_t nb_inputs, int32_t nb_outputs, int32_t width,
   AKB_CUDA_TRY(cudaMemsetAsync(m->d_m2, 0, m->nparams * sizeof(float), m->stream));
   akb_status st;
   if ((st = repack(m.get())) != AKB_OK) return st;
-  AKB_CUDA_TRY(set_smem((const void*)k_forward<true>, kFwdSmem));
-  AKB_CUDA_TRY(set_smem((const void*)k_forward<false>, kFwdSmem));
+  AKB_CUDA_TRY(set_smem((const void*)k_forward<true, false>, kFwdSmem));
+  AKB_CUDA_TRY(set_smem((const void*)k_forward<false, false>, kFwdSmem));
   AKB_CUDA_TRY(set_smem((const void*)k_forward<false, true>, kFwdSmem));
   AKB_CUDA_TRY(set_smem((const void*)k_backward, kBwdSmem));
   AKB_CUDA_TRY(set_smem((const void*)k_wgrad, kWgradSmem));
@@ -1094,7 +1138,7 @@ akb_status akb_mlp_forward(akb_mlp* m, int64_t nb, const double* x, double* y, v
   if (ntiles > INT32_MAX) return fail(AKB_ERR_UNSUPPORTED, "too many samples");
   AKB_CUDA_TRY(cudaSetDevice(m->device));
   cudaStream_t s = stream ? (cudaStream_t)stream : m->stream;
-  k_forward<false><<<(unsigned)ntiles, kFwdThreads, kFwdSmem, s>>>(m->net, nb, x, y, Bufs{});
+  k_forward<false, false><<<(unsigned)ntiles, kFwdThreads, kFwdSmem, s>>>(m->net, nb, x, y, Bufs{});
   AKB_CUDA_TRY(cudaGetLastError());
   return AKB_OK;
 }
@@ -1120,8 +1164,8 @@ akb_status akb_mlp_stress(akb_mlp* m, int64_t nb, const double* grad_u, double* 
   sa.min_det = min_det;
   sa.index = fallback_index;
   sa.count = fallback_count;
-  k_forward<false, true><<<(unsigned)ntiles, kFwdThreads, kFwdSmem, s>>>(m->net, nb, grad_u,
-                                                                         stress, Bufs{}, sa);
+  k_forward<false, true><<<(unsigned)ntiles, kFwdThreads, kFwdSmem, s>>>(m->net, nb, grad_u, stress,
+                                                                         Bufs{}, sa);
   AKB_CUDA_TRY(cudaGetLastError());
   return AKB_OK;
 }
