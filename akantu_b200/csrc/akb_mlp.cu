@@ -369,7 +369,7 @@ __device__ inline void stage_inputs(const Net& net, int64_t nb, const double* __
 // for a 256-wide layer instead of 64 with slices of 64 rows. Thread 0 only
 // waits for slices and issues; the copies have a thread of another warp, whose
 // wait for a slice to be free holds up nobody (with one thread doing both, the
-// wait was 500 of a slice's 1300 cycles). Stress calls, 4 x 256 hidden: 1000
+// wait was 500 of a slice's 1300 cycles). Stress calls, three hidden layers of 256: 1000
 // points 29.0 -> 22.9 us, 20000 33.3 -> 27.1, 262144 206 -> 164, 500000
 // 396 -> 314; a step of 32^3 macro elements 273 -> 231 us, of 8^3 77 -> 65.
 template <bool TRAIN, bool STRESS>

@@ -175,14 +175,10 @@ struct FanDesc {
 
 // Device copy of a PatchHost.
 struct DevPatches {
-  int fans;  // fan records: the step runs k_fan_step
-  int linear;  // fans: every material is small-strain elastic (hexahedra: every
-               // element a parallelepiped)
   int npatch;
   int grid;  // 0: one CTA per patch; > 0: persistent grid of that many CTAs
-  int resident[2];  // fans, grid 0: CTAs on the device at once (without, with f_ext)
   int nbuf;  // chunk record buffers in shared memory (2: next chunk prefetched)
-  int max_nodes, max_interior, max_shared, node_stride, contrib_slots, max_runs, chunk_bytes;
+  int max_nodes, max_shared, node_stride, contrib_slots, max_runs, chunk_bytes;
   const int32_t* elem_ptr;
   const int32_t* ibeg;
   const int32_t* nint;
@@ -193,8 +189,6 @@ struct DevPatches {
   const uint2* chunks;     // ChunkDesc per chunk
   const uint16_t* cdata;   // chunk records (16-byte aligned)
   const uint32_t* emat;    // material of each patch-ordered element, or null
-  const FanDesc* desc;     // fans: per patch
-  const uint2* entries;    // fans: per shared entry, its node and partial slot
   int* err;                // set when a bounded wait gave up
   double* partial;         // nslots x dim
   double* w;               // nn x dim predicted displacement
@@ -219,6 +213,16 @@ struct DevPatches {
   // batches: instance node ranges (ninst + 1), for the w refresh
   const int64_t* node_off;
   int ninst;
+  // Fan records (the step runs k_fan_step). They stand last: the launches of
+  // chunk plans then read their parameters from as few constant lines as they
+  // can (in between, these fields cost a small step 0.06 to 0.12 us of 6).
+  int fans;
+  int linear;        // every material is small-strain elastic (hexahedra: every
+                     // element a parallelepiped)
+  int resident[2];   // grid 0: CTAs on the device at once (without, with f_ext)
+  int max_interior;
+  const FanDesc* desc;   // per patch
+  const uint2* entries;  // per shared entry, its node and partial slot
 };
 
 // Partial slots of a plan's shared entries (sslot), its shared nodes' first
