@@ -245,6 +245,30 @@ void patch_params(int type, int* target, int* max_nodes) {
 template <typename T>
 akb_status upload(akb_model* m, const std::vector<T>& v, const T** out);
 
+// Whether a model steps on fan records (k_fan_step) rather than chunk records
+// (k_patch_step). FP32 does not: its roundings go with the chunk kernel.
+//  - Small meshes: a fan is a serial chain of up to eight elements, and with
+//    few patches nothing else hides it. Chunk records against fan records, us a
+//    step: 312 triangles 5.3 against 5.7, 1600 6.10 against 6.23, 4800 6.4
+//    against 6.1; 288 tetrahedra 6.3 against 6.9, 600 7.0 against 7.1, 1080 7.5
+//    against 7.05. Hexahedra: faster on fan records from 294 elements on.
+//  - Patch sizes chosen by the caller: the fan kernels are built for patches
+//    whose fans fill their CTA about once. 280 k triangles at 768 elements 19.8
+//    against 16.2, at 1024 16.6 against 18.5, at 2048 23.7 against 30.7; 1.6 M
+//    tetrahedra at 512 72 against 87, at 768 65 against 49, at 1536 63 against
+//    40; 262 k hexahedra at 256 141 against 79, at 384 101.2 against 101.6, at
+//    512 95 against 104.
+bool use_fans(const akb_model* m, int64_t ne) {
+  if (m->mode != AKB_MODE_FP64) return false;
+  const int pe = m->opt_patch_elements;
+  switch (m->dm.type) {
+  case AKB_TRIANGLE_3: return pe > 0 ? pe <= 768 : ne >= 2048;
+  case AKB_TETRAHEDRON_4: return pe > 0 ? pe >= 768 : ne >= 768;
+  case AKB_HEXAHEDRON_8: return pe <= 256;
+  default: return false;
+  }
+}
+
 // The same for fan records: patches of at most max_fans fans of at most
 // fan_cap elements (triangles and tetrahedra: a fan per thread of the CTA,
 // FanBuild), or of single elements.
@@ -793,10 +817,9 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
   const double* mesh_X = mesh->nodes;
   const uint32_t* mesh_C = mesh->connectivity;
   if (patched) {
-    // FP64 steps run on fan records, but for segments; a plan whose record or
-    // contributions do not fit an SM (patch sizes far above the defaults) steps
-    // chunk by chunk, as do FP32 steps, whose roundings go with that kernel
-    bool fans = m->mode == AKB_MODE_FP64 && type != AKB_SEGMENT_2;
+    // FP64 steps run on fan records where these are faster (use_fans), but a
+    // plan whose record or contributions do not fit an SM steps chunk by chunk
+    bool fans = use_fans(m.get(), ne);
     if (fans && type == AKB_HEXAHEDRON_8) {
       m->linear = true;
       for (int64_t e = 0; e < ne && m->linear; ++e) {

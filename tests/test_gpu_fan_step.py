@@ -96,3 +96,18 @@ def test_a_patch_above_an_sm_is_refused():
                             precision=_abi.MODE_FP64, patch_elements=4096, patch_nodes=6000)
     with pytest.raises(AkbError, match="shared memory"):
         m.initFull()
+
+
+@pytest.mark.parametrize("kind,n,mats,patch", [
+    ("tri", (33, 31), ELASTIC, {}), ("tri", (32, 32), ELASTIC, {}),
+    ("tet", (127, 1, 1), ELASTIC, {}), ("tet", (8, 4, 4), ELASTIC, {}),
+    ("tri", (60, 20), ELASTIC, dict(patch_elements=768)),
+    ("tri", (60, 20), ELASTIC, dict(patch_elements=769)),
+    ("tet", (9, 8, 6), ELASTIC, dict(patch_elements=767)),
+    ("tet", (9, 8, 6), ELASTIC, dict(patch_elements=768)),
+    ("hex", (8, 8, 8), NEO, dict(patch_elements=256)),
+    ("hex", (8, 8, 8), NEO, dict(patch_elements=257)),
+])
+def test_both_sides_of_the_dispatch(kind, n, mats, patch):
+    """Mesh and patch sizes next to where fan and chunk records change over."""
+    test_against_oracle(kind, n, mats, 1, patch, True)
