@@ -571,6 +571,14 @@ inline int cluster_of(int n) {
   return 0;
 }
 
+// With four CTAs per RVE the layers' exchange costs a cluster about 8 % of its
+// rate against a whole RVE per SM (k_rve, the same updates bit for bit), and what it gains is
+// the slowest instance's time at the end, some 60 ms: 512 RVEs 89 -> 71 ms, 4096
+// 555 -> 537, but 8191 1032 -> 1055 and 262144 17.9 -> 19.4 s. From this many
+// instances on, k_rve.
+// (Fewer CTAs per RVE are faster at any count: 4096 of 8^3 76 -> 28 ms.)
+constexpr int64_t kManyInstances = 6144;
+
 struct ClusterLayout {
   int u, v, im, B, F, mat, red, total;  // byte offsets
 };
@@ -1002,7 +1010,7 @@ akb_status launch(akb_rve* r, int max_it, int64_t nb, const double* grad_u, void
   if (r->mode == AKB_MODE_FP64)
     k_rve<double><<<(unsigned)nb, kRveThreads, r->smem, s>>>(
         a, nb, grad_u, static_cast<double*>(fluct), stress, iterations, residual, force);
-  else if (const int C = cluster_of(r->n))
+  else if (const int C = cluster_of(r->n); C && (C < 4 || nb < kManyInstances))
     AKB_CUDA_TRY(launch_cluster<false>(C, a, nb, nb, nullptr, nullptr, grad_u, fluct, stress,
                                        iterations, residual, force, s));
   else

@@ -41,3 +41,20 @@ def test_fixed_updates_match_oracle(cells):
     Pi = Pi.reshape(-1, 3, 3).transpose(1, 2)
     assert torch.equal(Pi[0], out["stress"][0]) and torch.equal(Pi[2], out["stress"][2])
     assert not bool(Pi[1].any())
+
+
+def test_many_instances_leave_the_clusters():
+    """From 6144 instances of 16^3 on, one CTA per RVE: the same FP32 updates
+    bit for bit; the stress is a FP64 sum of 32768 terms in another order
+    (2^-53 each, of terms at most 30 times the mean)."""
+    import torch
+    from akantu_b200.rve import SolidMechanicsModelRVE
+    vm = (np.random.default_rng(0).random(16 ** 3) < 0.3).astype(np.uint8)
+    H = fe2.sample_gradients(6144, seed=3, amplitude=0.1)
+    R = SolidMechanicsModelRVE(16, vm, fe2.matrix_inclusion_materials(),
+                               precision=_abi.MODE_FP32_BULK, tolerance=-1.0, max_iterations=5)
+    w, w1 = R.zero_fluctuation(6144), R.zero_fluctuation(6143)
+    many, fewer = R.solve(H, w)["stress"], R.solve(H[:6143], w1)["stress"]
+    assert bool(torch.isfinite(many).all())
+    assert torch.equal(w[:6143], w1)
+    assert float((many[:6143] - fewer).abs().max()) <= 1.1e-10 * float(fewer.abs().max())
