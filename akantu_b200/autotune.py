@@ -1,7 +1,7 @@
 """Autotuner of the fused patch step.
 
-Chooses the patch shape (elements per patch, node cap) and the schedule (one
-CTA per patch, or a persistent grid of k CTAs per SM striding over the
+Chooses the patch shape (elements per patch, node cap) and the schedule (the
+library's default, or a persistent grid of k CTAs per SM striding over the
 patches) by timing a few steps of each candidate with CUDA events on the
 model's stream, in three stages per element type: the patch size at the
 type's usual nodes-per-element ratio, then the node cap around the best

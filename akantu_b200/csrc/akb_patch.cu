@@ -1,6 +1,10 @@
 // akb_patch.cu -- the fused explicit step (AKB_MODE_FP64, AKB_MODE_FP32_BULK).
 //
-// k_patch_step: one CTA per patch (akb_patch.cuh for the node order, the
+// k_fan_step (FP64 triangles, tetrahedra, hexahedra: plans on fan records): a
+// resident grid over the patches, a fan of elements per thread; described
+// below, before its layout.
+// k_patch_step (FP32, segments, plans too large for a fan record's shared
+// memory): one CTA per patch (akb_patch.cuh for the node order, the
 // predicted displacement w and the shared-node protocol).
 //   1. stage: thread 0 starts TMA bulk copies of the interior nodes' X and w
 //      (two contiguous slices) and of the first chunk records, and prefetches

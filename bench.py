@@ -348,12 +348,12 @@ def run_ours(args, dist):
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": peak_kind,
                          "algorithmic_bytes_per_step": balg,
-                         # DRAM bytes of one k_patch_step launch from an ncu capture
-                         # (dram__bytes_read.sum + dram__bytes_write.sum) of the
-                         # 90^3-cell cube (4.374 M elements, 232.7 MB), scaled by
+                         # DRAM bytes of one k_fan_step launch from an ncu capture
+                         # (dram__bytes rate x duration) of the
+                         # 90^3-cell cube (4.374 M elements, 134.7 MB), scaled by
                          # elements; the capture is not taken inside this run
-                         "traffic": 232.7e6 * E / 4.374e6,
-                         "traffic_kernel": "k_patch_step (ncu, 90^3 cells, scaled by elements)",
+                         "traffic": 134.7e6 * E / 4.374e6,
+                         "traffic_kernel": "k_fan_step (ncu, 90^3 cells, scaled by elements)",
                          "kernels_ms": {n: t for n, t in ktimes},
                          "dominant": top[0]},
             "clocks": clocks,
@@ -553,12 +553,12 @@ def run_hex8(args, device, peak):
             "rel_err_displacement": float(np.abs(u32 - u64).max() / np.abs(u64).max()),
             "rel_err_internal_force": float(np.abs(f32 - f64).max() / np.abs(f64).max())}
     out["time_step"] = dt
-    # compute roofline of the FP64 launch, from an ncu capture of this
-    # workload (sm__inst_executed_pipe_fp64, % of peak; not taken in this run)
+    # pipe use of the FP32-bulk launch, from an ncu capture of this workload
+    # (% of peak; not taken in this run)
     out["compute_roofline"] = {"bound": "fp64 pipe (FP64) / fma pipe (FP32-bulk)",
-                               "fp64_pipe_active": 0.445, "fp32_bulk_fma_pipe_active": 0.413,
-                               "kernel": "k_patch_step<hex8, double> / <hex8, float>",
-                               "source": "ncu captures of the 96^3 block "
+                               "fp32_bulk_fma_pipe_active": 0.413,
+                               "kernel": "k_patch_step<hex8, float>",
+                               "source": "ncu capture of the 96^3 block "
                                          "(profiles/k_patch_step_block_hex8_96.md)"}
     return out
 

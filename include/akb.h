@@ -118,8 +118,10 @@ typedef struct {
   void* stream;           /* cudaStream_t to run on; NULL = library-owned stream */
   int32_t patch_elements; /* fast modes: elements per patch (0 = per-type default) */
   int32_t patch_nodes;    /* fast modes: node cap of a patch (0 = per-type default) */
-  int32_t patch_grid;     /* fast modes: 0 = one CTA per patch; > 0 = persistent grid
-                             of that many CTAs striding over the patches */
+  int32_t patch_grid;     /* fast modes: 0 = the default (FP64 triangles, tetrahedra and
+                             hexahedra: as many CTAs as run at once, striding over the
+                             patches; otherwise one CTA per patch); > 0 = a grid of that
+                             many CTAs striding over the patches */
 } akb_model_options;
 
 typedef struct {
