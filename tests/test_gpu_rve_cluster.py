@@ -58,3 +58,33 @@ def test_many_instances_leave_the_clusters():
     assert bool(torch.isfinite(many).all())
     assert torch.equal(w[:6143], w1)
     assert float((many[:6143] - fewer).abs().max()) <= 1.1e-10 * float(fewer.abs().max())
+
+
+def test_a_list_takes_as_long_as_the_batch():
+    """The listed RVEs are strided over by no more clusters than run at once: the
+    same 1024 RVEs of 16^3 (40 updates each) take about as long listed as in a
+    batch (the tail of 1024 over some 36 clusters: at most 1 / 28). With clusters
+    beyond the resident ones the list waits for a second round: twice as long."""
+    import torch
+    from akantu_b200.rve import SolidMechanicsModelRVE
+    vm = (np.random.default_rng(0).random(16 ** 3) < 0.3).astype(np.uint8)
+    H = torch.as_tensor(fe2.sample_gradients(1024, seed=3, amplitude=0.1), device="cuda")
+    R = SolidMechanicsModelRVE(16, vm, fe2.matrix_inclusion_materials(),
+                               precision=_abi.MODE_FP32_BULK, tolerance=-1.0, max_iterations=40)
+    Hc = H.transpose(1, 2).reshape(-1, 9).contiguous()
+    P = torch.empty_like(Hc)
+    idx = torch.arange(1024, dtype=torch.int32, device="cuda")
+    cnt = torch.tensor([1024], dtype=torch.int32, device="cuda")
+
+    def ms(call):
+        best = float("inf")
+        for _ in range(5):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            call()
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+    listed, batch = ms(lambda: R.solve_indexed(idx, cnt, Hc, P)), ms(lambda: R.solve(H))
+    assert listed <= 1.3 * batch, (listed, batch)
