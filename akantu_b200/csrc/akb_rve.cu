@@ -285,8 +285,32 @@ __device__ __forceinline__ void voxel_edge_sums(const S* B, const MatParams& mp,
   }
 }
 
+// CTAs of the cluster that relaxes an FP32 RVE (k_rve_cluster)
+constexpr int kClusterThreads = 512;
+constexpr int kClusterVoxels = 1024;
+
+// CTAs per RVE of n^3 cells, 0: not this way.
+__host__ __device__ inline int cluster_of(int n) {
+  for (int c = 1; c <= 4; c *= 2)
+    if (n % c == 0 && (n / c) % 2 == 0 && (int64_t)n * n * n / c <= kClusterVoxels) return c;
+  return 0;
+}
+
+// An RVE of 16^3 is relaxed by a cluster of four CTAs or, in large numbers, by
+// one CTA (kManyInstances), and its stress must not tell which: one CTA adds the
+// voxels' w P up as the four would. There a thread has a voxel of colour c and
+// the one of colour c + 4 at the same place t in the colour, c = 0..3, t a
+// quarter of the colour's places for each CTA; then come its warp, the CTA's 16
+// warps and the CTAs. Here thread x has t = x and x + 256: eight sums.
+template <typename S>
+__host__ __device__ inline bool sums_by_quarters(int n) {
+  return sizeof(S) == 4 && cluster_of(n) == 4;
+}
+constexpr int kQuarterSums = 8;
+
 // f -= element forces of every voxel (8 colours); PSUM also adds
-// sum_q w_q P (row-major) of this thread's voxels to psum.
+// sum_q w_q P (row-major) of this thread's voxels to psum (with `quarters`, to
+// its eight sums there).
 //
 // The voxel is a cube, so its shape gradients factor along its 12 edges:
 // with corners o = ox + 2 oy + 4 oz and s(b) = 2 b - 1,
@@ -298,7 +322,7 @@ __device__ __forceinline__ void voxel_edge_sums(const S* B, const MatParams& mp,
 // Same arithmetic content as the shape-gradient form, half the operations.
 template <typename S, bool PSUM>
 __device__ void voxel_forces(const RveArgs& R, const RveSmem<S>& s, const S* hH,
-                             const MatParams* mats, double* psum) {
+                             const MatParams* mats, double* psum, bool quarters = false) {
   const int n = R.n, nn = R.nn, hn = n >> 1, nc = hn * hn * hn;
   const S wq = S(R.h * R.h * R.h / 8.0);
   for (int color = 0; color < 8; ++color) {
@@ -329,7 +353,10 @@ __device__ void voxel_forces(const RveArgs& R, const RveSmem<S>& s, const S* hH,
       }
       const MatParams& mp = mats[s.mat[pidx(ex, ey, ez, n)]];
       S T[3][4][3];
-      voxel_edge_sums<S, PSUM>(s.B, mp, D, wq, T, psum);
+      double* to = psum;
+      if constexpr (PSUM && sizeof(S) == 4)
+        if (quarters) to += ((color & 3) * 2 + t / kRveThreads) * 9;
+      voxel_edge_sums<S, PSUM>(s.B, mp, D, wq, T, to);
 #pragma unroll
       for (int o = 0; o < 8; ++o) {
         const int ox = o & 1, oy = (o >> 1) & 1, oz = o >> 2;
@@ -492,19 +519,37 @@ __device__ __forceinline__ void rve_instance(const RveArgs& R, int64_t inst,
   // homogenised stress (and force) of the final state
   for (int idx = tid; idx < 3 * nn; idx += bs) s.f[idx] = 0;
   __syncthreads();
-  double ps[9];
+  const bool quarters = sums_by_quarters<S>(R.n);
+  constexpr int kSums = sizeof(S) == 4 ? kQuarterSums : 1;
+  double ps[kSums * 9];
 #pragma unroll
-  for (int q = 0; q < 9; ++q) ps[q] = 0.0;
-  voxel_forces<S, true>(R, s, hH, mats, ps);
+  for (int q = 0; q < kSums * 9; ++q) ps[q] = 0.0;
+  voxel_forces<S, true>(R, s, hH, mats, ps, quarters);
+  // the warps' sums: of all voxels, or [colour mod 4][32 consecutive places] (the
+  // velocities are done with)
+  double* sums = quarters ? reinterpret_cast<double*>(s.v) : s.red;
 #pragma unroll
-  for (int q = 0; q < 9; ++q) {
-    const double x = warp_sum(ps[q]);
-    if (lane == 0) s.red[warp * 9 + q] = x;
+  for (int j = 0; j < kSums; ++j) {
+    if (j > 0 && !quarters) break;
+    const int at = quarters ? (j >> 1) * 16 + (j & 1) * 8 + warp : warp;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      const double x = warp_sum(ps[j * 9 + q]);
+      if (lane == 0) sums[at * 9 + q] = x;
+    }
   }
   __syncthreads();
   if (tid < 9) {
     double t = 0.0;
-    for (int w = 0; w < nwarps; ++w) t += s.red[w * 9 + tid];
+    if (quarters) {
+      for (int z = 0; z < 4; ++z) {
+        double tz = 0.0;
+        for (int w = 0; w < 16; ++w) tz += sums[((w >> 2) * 16 + z * 4 + (w & 3)) * 9 + tid];
+        t += tz;
+      }
+    } else {
+      for (int w = 0; w < nwarps; ++w) t += sums[w * 9 + tid];
+    }
     const int i = tid / 3, j = tid % 3;
     stress[inst * 9 + i + 3 * j] = t / (R.L * R.L * R.L);
   }
@@ -562,16 +607,7 @@ __global__ void __launch_bounds__(kRveThreads, 1)
 //  - the planes are spread over C SMs. A CTA reads the forces of the layer
 //    below its first plane, and writes the displacements of that plane, in the
 //    neighbour's shared memory.
-constexpr int kClusterThreads = 512;
-constexpr int kClusterVoxels = 1024;
-
-// CTAs per RVE of n^3 cells, 0: not this way.
-inline int cluster_of(int n) {
-  for (int c = 1; c <= 4; c *= 2)
-    if (n % c == 0 && (n / c) % 2 == 0 && (int64_t)n * n * n / c <= kClusterVoxels) return c;
-  return 0;
-}
-
+//
 // With four CTAs per RVE the layers' exchange costs a cluster about 8 % of its
 // rate against a whole RVE per SM (k_rve, the same updates bit for bit), and what it gains is
 // the slowest instance's time at the end, some 60 ms: 512 RVEs 89 -> 71 ms, 4096

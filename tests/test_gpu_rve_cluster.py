@@ -88,3 +88,34 @@ def test_a_list_takes_as_long_as_the_batch():
         return best
     listed, batch = ms(lambda: R.solve_indexed(idx, cnt, Hc, P)), ms(lambda: R.solve(H))
     assert listed <= 1.3 * batch, (listed, batch)
+
+
+@pytest.mark.parametrize("kinds", ["neohookean", "elastic inclusion"])
+def test_stress_does_not_tell_the_kernel(kinds):
+    """An RVE of 16^3 has the same bits alone, in a list and in a batch large
+    enough for one CTA per RVE: fluctuation, stress, residual and, of the relaxed
+    state, the internal force."""
+    import torch
+    from akantu_b200.rve import SolidMechanicsModelRVE
+    vm = (np.random.default_rng(1).random(16 ** 3) < 0.3).astype(np.uint8)
+    mats = fe2.matrix_inclusion_materials()
+    if kinds != "neohookean":
+        mats[1]["kind"] = _abi.MATERIAL_ELASTIC
+    nb, few = 6144, 40
+    H = torch.as_tensor(fe2.sample_gradients(nb, seed=5, amplitude=0.1), device="cuda")
+    R = SolidMechanicsModelRVE(16, vm, mats, precision=_abi.MODE_FP32_BULK, tolerance=-1.0,
+                               max_iterations=12)
+    w, w1 = R.zero_fluctuation(nb), R.zero_fluctuation(few)
+    many, alone = R.solve(H, w), R.solve(H[:few], w1)
+    assert torch.equal(w[:few], w1)
+    for k in ("stress", "residual"):
+        assert torch.equal(many[k][:few], alone[k]), k
+    P, f = R.stress(H, w)
+    P1, f1 = R.stress(H[:few], w1)
+    assert torch.equal(P[:few], P1) and torch.equal(P, many["stress"])
+    assert torch.equal(f[:few], f1)
+    Hc = H[:few].transpose(1, 2).reshape(-1, 9).contiguous()
+    Pi = torch.zeros_like(Hc)
+    idx = torch.arange(few, dtype=torch.int32, device="cuda")
+    R.solve_indexed(idx, torch.tensor([few], dtype=torch.int32, device="cuda"), Hc, Pi)
+    assert torch.equal(Pi.reshape(-1, 3, 3).transpose(1, 2), alone["stress"])
