@@ -608,13 +608,15 @@ __global__ void __launch_bounds__(kRveThreads, 1)
 //    below its first plane, and writes the displacements of that plane, in the
 //    neighbour's shared memory.
 //
-// With four CTAs per RVE the layers' exchange costs a cluster about 8 % of its
-// rate against a whole RVE per SM (k_rve, the same updates bit for bit), and what it gains is
-// the slowest instance's time at the end, some 60 ms: 512 RVEs 89 -> 71 ms, 4096
-// 555 -> 537, but 8191 1032 -> 1055 and 262144 17.9 -> 19.4 s. From this many
-// instances on, k_rve.
+// With four CTAs per RVE the layers' exchange costs a cluster 8 to 12 % of its
+// rate against a whole RVE per SM (k_rve, the same bits), and what it gains is
+// the time of the slowest instances at the end. From this many instances on,
+// k_rve. Random gradients up to 0.3 (mean of five draws), ms by clusters and by
+// k_rve: 512 74 and 100, 1024 137 and 154, 2048 272 and 289, 2560 334 and 334,
+// 3072 398 and 376, 4096 531 and 505; of gradients up to 0.06, which all take
+// about the same number of updates, 512 43 and 43, 1024 85 and 77, 2048 171 and 152.
 // (Fewer CTAs per RVE are faster at any count: 4096 of 8^3 76 -> 28 ms.)
-constexpr int64_t kManyInstances = 6144;
+constexpr int64_t kManyInstances = 2560;
 
 struct ClusterLayout {
   int u, v, im, B, F, mat, red, total;  // byte offsets
@@ -1208,7 +1210,11 @@ akb_status akb_rve_solve_indexed(akb_rve* r, int64_t capacity, const int32_t* in
     // no more clusters than run at once: the rest would start when one of these
     // has worked off its whole share (37 clusters of four where fewer fit: 32768
     // listed 16^3 RVEs 7388 ms, the resident ones 4349; an empty list in a macro
-    // step of 32^3 cells 228 -> 226 us)
+    // step of 32^3 cells 228 -> 226 us). Long lists stay with the clusters: the
+    // host does not know the length, and a second, mostly empty launch of
+    // k_rve_indexed costs every macro step 1.5 to 2.5 us. Strong gradients, as
+    // they leave a surrogate's envelope: 4096 listed 571 ms by clusters, 582 by
+    // k_rve_indexed, 16384 2199 and 2183; equal small ones 340 and 325, 1358 and 1275.
     AKB_CUDA_TRY(launch_cluster<true>(C, a, std::min<int64_t>(capacity, std::max(r->clusters, 1)),
                                       capacity, index, count, grad_u, fluctuation, stress,
                                       iterations, residual, nullptr, s));
