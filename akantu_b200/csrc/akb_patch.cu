@@ -212,30 +212,6 @@ __device__ inline void arrive(uint32_t mbar) {
   asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
 
-// Finishing inputs of a patch's interior nodes [ib, ib + nint): v, a (rows
-// of d doubles), 1/M (one double), blocked flags (d bytes), f_ext (d
-// doubles, when used). Each slice is bulk-copied from the 16-byte boundary at
-// or below its start to the one at or above its end (inside the arrays'
-// 16-byte slack); off[k]: where the slice's first item lands, from the
-// buffer's start; returns the bytes of all copies.
-template <int d, bool FEXT>
-__device__ inline uint32_t finish_regions(int ib, int nint, uint32_t* off, uint32_t* lo,
-                                          uint32_t* bytes) {
-  constexpr int nf = FEXT ? 5 : 4;
-  const uint32_t rowb[5] = {8u * d, 8u * d, 8u, (uint32_t)d, 8u * d};
-  uint32_t total = 0;
-#pragma unroll
-  for (int k = 0; k < nf; ++k) {
-    const size_t s0 = (size_t)ib * rowb[k], s1 = (size_t)(ib + nint) * rowb[k];
-    const size_t c0 = s0 & ~size_t(15), c1 = (s1 + 15) & ~size_t(15);
-    off[k] = total + (uint32_t)(s0 - c0);
-    lo[k] = (uint32_t)c0;  // (byte offsets below 4 GB: nn x d doubles < 2^32 bytes)
-    bytes[k] = (uint32_t)(c1 - c0);
-    total += bytes[k];
-  }
-  return total;
-}
-
 // Corrector of one free DOF from its total force r (with f_ext), and the
 // next predictor: u = w (the predicted displacement this step's forces were
 // evaluated at), v* = v + dt a recomputed bit for bit, then
@@ -334,14 +310,16 @@ __device__ __forceinline__ bool patch_body(const DevModel& m, const DevPatches& 
   // buffers are used and they fit; the finish then reads shared memory
   bool pre;
   {
-    uint32_t f_off[5], f_lo[5], f_bytes[5];
+    uint32_t f_off[5], f_bytes[5];
+    size_t f_lo[5];
     pre = two && nint > 0 &&
           finish_regions<d, FEXT>(ib, nint, f_off, f_lo, f_bytes) <= lay.buf_stride;
   }
   const uint32_t spare = buffer(uses + nchunks);
   auto issue_finish = [&]() {  // by thread 0
     const void* src[5] = {m.v, m.a, m.inv_mass, m.blocked, m.fext};
-    uint32_t f_off[5], f_lo[5], f_bytes[5];
+    uint32_t f_off[5], f_bytes[5];
+    size_t f_lo[5];
     const uint32_t total = finish_regions<d, FEXT>(ib, nint, f_off, f_lo, f_bytes);
     const uint32_t dst = saddr(smem + lay.buf + spare * lay.buf_stride);
     expect_tx(mbs, total);
@@ -509,7 +487,8 @@ __device__ __forceinline__ bool patch_body(const DevModel& m, const DevPatches& 
   const unsigned char* fin = smem + lay.buf + spare * lay.buf_stride;
   uint32_t f_off[5];
   {
-    uint32_t f_lo[5], f_bytes[5];
+    size_t f_lo[5];
+    uint32_t f_bytes[5];
     finish_regions<d, FEXT>(ib, nint, f_off, f_lo, f_bytes);
   }
 
@@ -966,7 +945,8 @@ __global__ void __launch_bounds__(FanBuild<TY, LIN>::threads, (FanBuild<TY, LIN>
           bulk_copy(saddr(smem + lay.ws), reinterpret_cast<const char*>(P.w) + c_lo, slice, mb);
         if (nint > 0) {  // inputs of the interior nodes' finish
           const void* src[5] = {m.v, m.a, m.inv_mass, m.blocked, m.fext};
-          uint32_t off[5], lo[5], nbytes[5];
+          uint32_t off[5], nbytes[5];
+          size_t lo[5];
           expect_tx(mb + 8, finish_regions<d, FEXT>(ib, nint, off, lo, nbytes));
           uint32_t at = saddr(smem + lay.fin);
 #pragma unroll
@@ -1048,7 +1028,8 @@ __global__ void __launch_bounds__(FanBuild<TY, LIN>::threads, (FanBuild<TY, LIN>
     const uint16_t* goff = rec + rec[6];
     uint32_t off[5];
     {
-      uint32_t lo[5], nbytes[5];
+      size_t lo[5];
+      uint32_t nbytes[5];
       finish_regions<d, FEXT>(ib, nint, off, lo, nbytes);
     }
     unsigned char* fin = smem + lay.fin;

@@ -225,6 +225,31 @@ struct DevPatches {
   const uint2* entries;  // per shared entry, its node and partial slot
 };
 
+// Finishing inputs of a patch's interior nodes [ib, ib + nint): v, a (rows
+// of d doubles), 1/M (one double), blocked flags (d bytes), f_ext (d
+// doubles, when used). Each slice is bulk-copied from the 16-byte boundary at
+// or below its start to the one at or above its end (inside the arrays'
+// 16-byte slack); lo[k]: the copy's byte offset in its array (beyond 32 bits from
+// 179 million nodes on); off[k]: where the slice's first item lands, from the
+// buffer's start; returns the bytes of all copies.
+template <int d, bool FEXT>
+__host__ __device__ inline uint32_t finish_regions(int ib, int nint, uint32_t* off, size_t* lo,
+                                                   uint32_t* bytes) {
+  constexpr int nf = FEXT ? 5 : 4;
+  const uint32_t rowb[5] = {8u * d, 8u * d, 8u, (uint32_t)d, 8u * d};
+  uint32_t total = 0;
+#pragma unroll
+  for (int k = 0; k < nf; ++k) {
+    const size_t s0 = (size_t)ib * rowb[k], s1 = (size_t)(ib + nint) * rowb[k];
+    const size_t c0 = s0 & ~size_t(15), c1 = (s1 + 15) & ~size_t(15);
+    off[k] = total + (uint32_t)(s0 - c0);
+    lo[k] = c0;
+    bytes[k] = (uint32_t)(c1 - c0);
+    total += bytes[k];
+  }
+  return total;
+}
+
 // Partial slots of a plan's shared entries (sslot), its shared nodes' first
 // overflow slots (shared_part) and nslots, from sgid, srank, shared_nodes and
 // shared_k (run after building, and again after merging the plans of a
