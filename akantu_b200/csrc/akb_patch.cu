@@ -647,11 +647,13 @@ template <bool PAR> struct FanBuild<AKB_HEXAHEDRON_8, PAR> {
 };
 
 // w P of one element from G = det * grad u (row-major), P the Cauchy (small
-// strain) or first Piola stress, w the reference volume of the simplex.
+// strain) or first Piola stress, w the reference volume of the simplex. A
+// small-strain elastic material's P is rounded the same whether or not the model
+// has others (LIN): an instance of a batch steps as it does alone.
 template <int d, bool LIN>
 __device__ inline void fan_stress(const MatParams& mp, const double* G, double det, double* P) {
   constexpr double w = d == 3 ? 1.0 / 6.0 : 0.5;
-  if constexpr (LIN) {
+  if (LIN || !mp.finite) {
     const double s = w * (1.0 / det), mu = mp.mu * s;
     double tr = G[0] + G[d + 1];
     if (d == 3) tr += G[2 * d + 2];
