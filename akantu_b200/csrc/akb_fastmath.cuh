@@ -423,21 +423,64 @@ __device__ inline double hex_derivative(const double (*E0)[3], const double (*Fp
   return E0[k][i] + s[m] * Fp[k + m - 1][i] + s[n] * Fp[k + n - 1][i] + (s[m] * s[n]) * F3[i];
 }
 
+// neo-Hookean P in 3D (stress_P) with every rounding spelled out: which product
+// of a sum is fused is the compiler's choice otherwise, and it chose differently
+// in the two forms of hex_force_f64, whose bits must agree. (64^3 block 79.2 ->
+// 77.1 us a step; for tetrahedra stress_P's form is faster, 31.3 against 32.7 us
+// for 50^3 cells.)
+__device__ inline void neohookean_P(double lam, double mu, const double* g, double* P) {
+  auto dot = [](double a0, double b0, double a1, double b1, double a2, double b2) {
+    return __fma_rn(a2, b2, __fma_rn(a0, b0, __dmul_rn(a1, b1)));
+  };
+  auto det2 = [](double a, double b, double c, double d) {  // a b - c d
+    return __fma_rn(a, b, -__dmul_rn(c, d));
+  };
+  double gg[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      gg[i * 3 + j] = dot(g[i * 3], g[j], g[i * 3 + 1], g[3 + j], g[i * 3 + 2], g[6 + j]);
+  const double t = __dadd_rn(__dadd_rn(g[0], g[4]), g[8]);
+  const double I2 = 0.5 * __fma_rn(t, t, -__dadd_rn(__dadd_rn(gg[0], gg[4]), gg[8]));
+  const double dg = dot(g[0], det2(g[4], g[8], g[5], g[7]), -g[1], det2(g[3], g[8], g[5], g[6]),
+                        g[2], det2(g[3], g[7], g[4], g[6]));
+  const double jm1 = __dadd_rn(__dadd_rn(t, I2), dg);
+  const double iJ = 1.0 / __dadd_rn(1.0, jm1);
+  const double a = __dmul_rn(mu, iJ), b = __dmul_rn(__dmul_rn(lam, log1p(jm1)), iJ);
+  const double c = __dadd_rn(1.0, t);
+  const double amb = __dsub_rn(a, b), diag = __fma_rn(a, dg, __dmul_rn(b, __dadd_rn(c, I2)));
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double u = __fma_rn(c, g[j * 3 + i], -gg[j * 3 + i]);
+      const double p = __fma_rn(amb, u, __dmul_rn(mu, g[i * 3 + j]));
+      P[i * 3 + j] = i == j ? __dadd_rn(p, diag) : p;
+    }
+}
+
 // FP64 hexahedron force by the signed sums (hex_parallelepiped_force, whose
 // accuracy notes concern FP32): with PAR the element map is affine, one
 // Jacobian for all points and 1 / det J folded into it; otherwise the Jacobian
 // of each point comes from the coordinates' sums, at 27 operations instead of
 // the 63 of the shape derivatives, and so do the displacement derivatives and
-// the corner forces (36 instead of 72).
+// the corner forces (36 instead of 72). In that form an element whose map is
+// affine (`affine`) leaves the trilinear sums out and gets the bits of the other:
+// its force does not depend on what else is in the mesh, or in the batch.
 template <bool PAR>
 __device__ inline void hex_force_f64(const MatParams& p, const double* dX, const double* du,
-                                     double* fe) {
+                                     double* fe, bool affine = PAR) {
   constexpr int d = 3;
   const int sg[3][8] = {{-1, 1, 1, -1, -1, 1, 1, -1},
                         {-1, -1, 1, 1, -1, -1, 1, 1},
                         {-1, -1, -1, -1, 1, 1, 1, 1}};
   double X0[3][3], Xp[3][3], X3[3], E0[3][3], Fp[3][3], F3[3], A[9], Ai[9];
   hex_sums(dX, X0, Xp, X3);
+  if (!PAR && affine) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) Xp[0][i] = Xp[1][i] = Xp[2][i] = X3[i] = 0.0;
+  }
   hex_sums(du, E0, Fp, F3);
   if (PAR) {
     double J[9];
@@ -475,7 +518,10 @@ __device__ inline void hex_force_f64(const MatParams& p, const double* dX, const
       for (int j = 0; j < d; ++j)
         g[i * 3 + j] = H[0] * Ai[j * 3] + H[1] * Ai[j * 3 + 1] + H[2] * Ai[j * 3 + 2];
     }
-    stress_P<3, double>(p, g, P);
+    if (p.kind == AKB_MATERIAL_NEOHOOKEAN)
+      neohookean_P(p.lambda, p.mu, g, P);
+    else
+      stress_P<3, double>(p, g, P);
 #pragma unroll
     for (int i = 0; i < d; ++i)
 #pragma unroll

@@ -403,6 +403,25 @@ akb_status plan_patches(akb_model* m, const akb_mesh_desc* mesh, const BatchLayo
   return AKB_OK;
 }
 
+// Sets kFanAffine in the records of a plan of single hexahedra; whether all of
+// them are parallelepipeds.
+bool mark_affine(const akb_mesh_desc* mesh, PatchHost& P) {
+  bool all = true;
+  for (int p = 0; p < P.npatch; ++p) {
+    uint16_t* rec = &P.cdata[(size_t)P.chunks[P.chunk_base[p]].off16 * 8];
+    for (int32_t i = P.elem_ptr[p]; i < P.elem_ptr[p + 1]; ++i) {
+      const uint32_t* c = mesh->connectivity + (int64_t)P.elem_order[i] * 8;
+      double dX[24];
+      for (int k = 0; k < 24; ++k)
+        dX[k] = mesh->nodes[(int64_t)c[k / 3] * 3 + k % 3] - mesh->nodes[(int64_t)c[0] * 3 + k % 3];
+      const bool affine = fast::hex_is_parallelepiped(dX);
+      if (affine) rec[rec[4] + 2 * (i - P.elem_ptr[p])] |= kFanAffine;
+      all = all && affine;
+    }
+  }
+  return all;
+}
+
 // Device copy of a patch plan; the model's arrays are already in the plan's
 // internal node order.
 akb_status build_device_patches(akb_model* m, const PatchHost& P,
@@ -820,20 +839,11 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
     // FP64 steps run on fan records where these are faster (use_fans), but a
     // plan whose record or contributions do not fit an SM steps chunk by chunk
     bool fans = use_fans(m.get(), ne);
-    if (fans && type == AKB_HEXAHEDRON_8) {
-      m->linear = true;
-      for (int64_t e = 0; e < ne && m->linear; ++e) {
-        double dX[24];
-        for (int k = 0; k < 24; ++k)
-          dX[k] = mesh->nodes[(int64_t)mesh->connectivity[e * 8 + k / 3] * 3 + k % 3] -
-                  mesh->nodes[(int64_t)mesh->connectivity[e * 8] * 3 + k % 3];
-        m->linear = fast::hex_is_parallelepiped(dX);
-      }
-    }
     if (fans) {
       st = plan_patches(m.get(), mesh, batch, part, true, plan, patch_inst, orphan_inst);
       fans = st == AKB_OK && fan_smem_bytes(plan, d) <= 227 * 1024;
     }
+    if (fans && type == AKB_HEXAHEDRON_8) m->linear = mark_affine(mesh, plan);
     if (!fans &&
         (st = plan_patches(m.get(), mesh, batch, part, false, plan, patch_inst, orphan_inst)) != AKB_OK)
       return st;

@@ -816,6 +816,7 @@ __device__ __forceinline__ void hex_forces(const uint16_t* rec, int t, const dou
   constexpr int d = 3, n = 8;
   const int nf = rec[0];
   const uint32_t* node = reinterpret_cast<const uint32_t*>(rec + rec[3]) + t;
+  const bool affine = rec[rec[4] + 2 * t] & kFanAffine;
   const MatParams& mp = emat ? table[emat[t]] : mp0;
   double dX[d * n], du[d * n], fe[d * n];
   {
@@ -824,7 +825,7 @@ __device__ __forceinline__ void hex_forces(const uint16_t* rec, int t, const dou
     for (int a = 0; a < n; ++a) lc[a] = (int)(node[a * nf] & 0xffff);
     gather_differences<d, n, double>(xs, ws, lc, dX, du);
   }
-  fast::hex_force_f64<PAR>(mp, dX, du, fe);
+  fast::hex_force_f64<PAR>(mp, dX, du, fe, affine);
 #pragma unroll
   for (int a = 0; a < n; ++a) {
     const int s = (int)(node[a * nf] >> 16);

@@ -96,7 +96,8 @@ inline int place_group(int dim) { return dim == 2 ? 8 : 16; }
 //   cnt      per position the number of its contributions
 //   goff     per 32 positions, where their list starts in the record: entry q
 //            of position 32 g + l at goff[g] + 32 q + l
-// Hexahedra: fans of one element, row j its corner j. The slots are a colouring
+// Hexahedra: fans of one element, row j its corner j, info | kFanAffine for a
+// parallelepiped (set by the model that has the plan built). The slots are a colouring
 // as the chunk records', 16 colours in 3D and 8 in 2D (16-byte rows): scatter
 // and sum are free of bank conflicts.
 // Partial slot of rank r of shared node s (ns shared nodes; over: the node's
@@ -143,6 +144,7 @@ struct PatchHost {
 };
 
 constexpr int kSingles = -1;
+constexpr uint16_t kFanAffine = 0x4000;
 
 // Builds the patches and the internal node order. target_elems: elements per
 // patch; max_nodes: local node cap (<= 60000); contrib_bytes: element vector
@@ -238,7 +240,6 @@ __host__ __device__ inline uint32_t finish_regions(int ib, int nint, uint32_t* o
   constexpr int nf = FEXT ? 5 : 4;
   const uint32_t rowb[5] = {8u * d, 8u * d, 8u, (uint32_t)d, 8u * d};
   uint32_t total = 0;
-#pragma unroll
   for (int k = 0; k < nf; ++k) {
     const size_t s0 = (size_t)ib * rowb[k], s1 = (size_t)(ib + nint) * rowb[k];
     const size_t c0 = s0 & ~size_t(15), c1 = (s1 + 15) & ~size_t(15);

@@ -57,3 +57,21 @@ def test_small_strain_boxes_beside_other_laws(patch_elements):
               for nx, ny, nz in ((9, 8, 7), (2, 3, 1), (6, 5, 11))]
     compare(meshes, [SMALL, FINITE, SMALL], dict(patch_elements=patch_elements))
     compare(meshes, [SMALL, NEOHOOKEAN, FINITE], dict(patch_elements=patch_elements))
+
+
+def distorted_block(nx, ny, nz, seed):
+    m = mesh_mod.box_hexahedron8(nx, ny, nz, 0.1 * nx, 0.1 * ny, 0.1 * nz)
+    nodes = m.nodes + 0.015 * np.random.default_rng(seed).uniform(-1, 1, m.nodes.shape)
+    return mesh_mod.Mesh(3, _abi.HEXAHEDRON_8, nodes, m.connectivity)
+
+
+@pytest.mark.parametrize("patch_elements", [0, 100, 256])
+def test_blocks_of_parallelepipeds_beside_others(patch_elements):
+    """Undistorted, distorted and partly distorted blocks of hexahedra."""
+    sheared = mesh_mod.box_hexahedron8(5, 7, 6, 0.5, 0.7, 0.6)
+    sheared = mesh_mod.Mesh(3, _abi.HEXAHEDRON_8,
+                            sheared.nodes @ np.array([[1, 0, 0], [0.3, 1, 0], [0.1, -0.2, 1]]),
+                            sheared.connectivity)
+    meshes = [mesh_mod.box_hexahedron8(7, 6, 9, 0.7, 0.6, 0.9), distorted_block(6, 5, 8, 1), sheared]
+    compare(meshes, [NEOHOOKEAN, SMALL, FINITE], dict(patch_elements=patch_elements))
+    compare(meshes, [SMALL, NEOHOOKEAN, NEOHOOKEAN], dict(patch_elements=patch_elements))
