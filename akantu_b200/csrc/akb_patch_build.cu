@@ -210,6 +210,23 @@ Fans build_fans(const double* X, const uint32_t* conn, int64_t nn, int64_t ne, i
   std::vector<Link> links;
   std::vector<int> from_of, seq;
   std::vector<char> taken;
+  auto alone = [&](uint32_t e) {  // a fan of this element only
+    const uint32_t* c = conn + (int64_t)e * n;
+    used[e] = 1;
+    F.elem.push_back(e);
+    F.node.insert(F.node.end(), c, c + n);
+    F.eptr.push_back((int32_t)F.elem.size());
+    F.nptr.push_back((int32_t)F.node.size());
+    F.closed.push_back(0);
+  };
+  // an element that names a node twice has no ring around its hinges
+  for (uint32_t e : order) {
+    const uint32_t* c = conn + (int64_t)e * n;
+    bool twice = false;
+    for (int a = 1; a < n; ++a)
+      for (int b = 0; b < a; ++b) twice = twice || c[a] == c[b];
+    if (twice) alone(e);
+  }
   for (uint32_t seed : order) {
     if (used[seed]) continue;
     const uint32_t* c = conn + (int64_t)seed * n;
@@ -299,14 +316,7 @@ Fans build_fans(const double* X, const uint32_t* conn, int64_t nn, int64_t ne, i
       F.nptr.push_back((int32_t)F.node.size());
       F.closed.push_back(closed);
     }
-    if (!used[seed]) {  // an element that names a node twice: a fan of its own
-      used[seed] = 1;
-      F.elem.push_back(seed);
-      F.node.insert(F.node.end(), c, c + n);
-      F.eptr.push_back((int32_t)F.elem.size());
-      F.nptr.push_back((int32_t)F.node.size());
-      F.closed.push_back(0);
-    }
+    if (!used[seed]) alone(seed);  // not among the hinge's first kMostLinks
   }
   return F;
 }
