@@ -4,12 +4,12 @@ Chooses the patch shape (elements per patch, node cap) and the schedule (the
 library's default, or a persistent grid of k CTAs per SM striding over the
 patches) by timing a few steps of each candidate with CUDA events on the
 model's stream, in three stages per element type: the patch size at the
-type's usual nodes-per-element ratio, then the node cap around the best
-size, then the persistent schedules of the best shape. Candidates the
-library refuses (a node cap too small for the mesh, shared memory over the
-limit) are skipped. The winner is cached in a JSON file keyed by GPU name,
-element type, precision mode and problem size (log2 bucket of the element
-count).
+type's usual nodes-per-element ratio (size 0: the library's default shape),
+then the node cap around the best size, then the persistent schedules of the
+best shape. Candidates the library refuses (a node cap too small for the mesh,
+shared memory over the limit) are skipped. The winner is cached in a JSON file
+keyed by GPU name, element type, precision mode, problem size (log2 bucket of
+the element count) and the version of the library's plans.
 """
 from __future__ import annotations
 
@@ -21,17 +21,23 @@ from . import _abi
 
 DEFAULT_CACHE = os.path.join(os.path.expanduser("~"), ".cache", "akantu_b200", "tuning.json")
 
-# Search space per element type: patch sizes (elements), node caps as
-# multiples of the patch size (the middle one is the usual ratio of a compact
-# patch of that type), persistent CTAs per SM tried for the best shape.
+# Raised when the plans or the kernels behind a shape change: a shape measured
+# on others is measured again.
+PLAN_VERSION = 2
+
+# Search space per element type: patch sizes (elements; 0: the default shape,
+# which depends on the mesh's size and no explicit one need reproduce), node
+# caps as multiples of the patch size (the middle one lets a compact patch of
+# that type have its size), persistent CTAs per SM tried for the best shape.
 SPACE = {
-    _abi.SEGMENT_2: dict(elements=(256, 512, 1024, 2048), ratios=(1.02, 1.08, 1.15), persist=(2, 4)),
-    _abi.TRIANGLE_3: dict(elements=(256, 384, 512, 768, 1024, 1536, 2048),
+    _abi.SEGMENT_2: dict(elements=(0, 256, 512, 1024, 2048), ratios=(1.02, 1.08, 1.15), persist=(2, 4)),
+    _abi.TRIANGLE_3: dict(elements=(0, 256, 384, 512, 768, 1024, 1536, 2048),
                           ratios=(0.56, 0.625, 0.70), persist=(2, 3)),
-    _abi.TETRAHEDRON_4: dict(elements=(256, 384, 512, 768, 1024, 1536),
+    _abi.TETRAHEDRON_4: dict(elements=(0, 256, 384, 512, 768, 1024, 1536),
                              ratios=(0.33, 0.39, 0.47), persist=(2, 3)),
-    _abi.HEXAHEDRON_8: dict(elements=(128, 192, 256, 384, 512),
-                            ratios=(1.35, 1.56, 1.8), persist=(1, 2)),
+    # (128 hexahedra have some 240 nodes)
+    _abi.HEXAHEDRON_8: dict(elements=(0, 128, 192, 256, 384, 512),
+                            ratios=(1.56, 1.9, 3.1), persist=(1, 2)),
 }
 
 
@@ -51,7 +57,7 @@ def _gpu_key():
 def cache_key(element_type, precision, nb_elements):
     name, _ = _gpu_key()
     bucket = int(math.log2(max(nb_elements, 1)))
-    return "%s|%d|%d|%d" % (name, element_type, precision, bucket)
+    return "%s|%d|%d|%d|plan%d" % (name, element_type, precision, bucket, PLAN_VERSION)
 
 
 def load_cache(path=DEFAULT_CACHE):

@@ -612,7 +612,11 @@ def run_batch(args, device, log=None):
                                     "algorithmic_bytes_per_step": balg},
                        "trials_ms_per_step": [[t[0], t[1]] for t in trials]}}
     b.close()
-    # the same sample as separate models (one model per plate, graph replays)
+    # the same sample as separate models (one model per plate, graph replays), with
+    # explicit patches: the default shape goes by the mesh's size, the batch's or
+    # the plate's
+    if not best["patch_elements"]:
+        best = dict(patch_elements=768, patch_nodes=500, patch_grid=0)
     sub_steps = 20
     models = []
     for i in sample:

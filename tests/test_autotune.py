@@ -74,3 +74,27 @@ def test_refused_shapes_are_skipped(tmp_path):
 def test_nothing_buildable_raises(tmp_path):
     with pytest.raises(RuntimeError):
         run(tmp_path, _abi.SEGMENT_2, lambda *a: 1.0, refuse=lambda *a: True)
+
+
+def test_the_default_shape_is_a_candidate(tmp_path):
+    def cost(pe, pn, grid):  # the default is the fastest, with its own schedule
+        return (0.5 if pe == 0 else 1.0) + (0.1 if grid else 0.0)
+    for etype in autotune.SPACE:
+        best, trials, built = run(tmp_path, etype, cost)
+        assert best == dict(patch_elements=0, patch_nodes=0, patch_grid=0)
+        assert built.count((0, 0, 0)) == 1 and len(built) == len(set(built))
+
+
+def test_shapes_of_other_plans_are_measured_again(tmp_path, monkeypatch):
+    """A cache written for other plans (another version, or the keys without one)
+    does not answer."""
+    import json
+    path = tmp_path / "tuning.json"
+    name = autotune._gpu_key()[0]
+    stale = dict(patch_elements=512, patch_nodes=1, patch_grid=7)
+    path.write_text(json.dumps({"%s|%d|%d|%d" % (name, _abi.HEXAHEDRON_8, _abi.MODE_FP64,
+                                                 int(math.log2(10 ** 6))): stale}))
+    best, trials, built = run(tmp_path, _abi.HEXAHEDRON_8, lambda pe, pn, grid: 1.0 + grid)
+    assert best != stale and trials
+    monkeypatch.setattr(autotune, "PLAN_VERSION", autotune.PLAN_VERSION + 1)
+    assert run(tmp_path, _abi.HEXAHEDRON_8, lambda pe, pn, grid: 1.0 + grid)[1]
