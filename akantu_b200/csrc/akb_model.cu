@@ -225,6 +225,7 @@ cudaError_t enqueue_step(akb_model* m, StepTimer* t = nullptr) {
 }
 
 const char* kernel_name(const akb_model* m, int slot) {
+  if (m->use_patches && slot == 0 && m->patches.fans) return "fan_step";
   if (m->use_patches) return (slot >= 0 && slot < 2) ? kPatchKernels[slot] : "";
   const char* const* names = m->mode == AKB_MODE_FP64_REFERENCE ? kRefKernels : kFastKernels;
   return (slot >= 0 && slot < 3) ? names[slot] : "";

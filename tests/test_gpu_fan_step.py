@@ -111,3 +111,33 @@ def test_a_patch_above_an_sm_is_refused():
 def test_both_sides_of_the_dispatch(kind, n, mats, patch):
     """Mesh and patch sizes next to where fan and chunk records change over."""
     test_against_oracle(kind, n, mats, 1, patch, True)
+
+
+@pytest.mark.parametrize("kind,n,patch,name", [
+    ("tri", (33, 31), {}, "patch_step"), ("tri", (31, 33), {}, "patch_step"),
+    ("tri", (32, 32), {}, "fan_step"), ("tri", (341, 3), {}, "patch_step"),
+    ("tet", (8, 4, 4), {}, "fan_step"), ("tet", (127, 1, 1), {}, "patch_step"),
+    ("tri", (60, 20), dict(patch_elements=768), "fan_step"),
+    ("tri", (60, 20), dict(patch_elements=769), "patch_step"),
+    ("tri", (8, 3), dict(patch_elements=256), "fan_step"),
+    ("tet", (9, 8, 6), dict(patch_elements=767), "patch_step"),
+    ("tet", (9, 8, 6), dict(patch_elements=768), "fan_step"),
+    ("hex", (1, 1, 1), {}, "fan_step"),
+    ("hex", (8, 8, 8), dict(patch_elements=256), "fan_step"),
+    ("hex", (8, 8, 8), dict(patch_elements=257), "patch_step"),
+    ("tet", (20, 20, 20), dict(patch_elements=8191, patch_nodes=6000), "patch_step"),
+])
+def test_kernel_of_each_side(kind, n, patch, name):
+    """akb_kernel_name says which kernel steps the model: fan records from 2048
+    triangles and 768 tetrahedra on and for the patch sizes they are built for;
+    chunk records below, beside them, in FP32 and where a patch of fans does not
+    fit an SM."""
+    from akantu_b200._lib import lib
+    from akantu_b200.model import SolidMechanicsModel, material_from_dict
+    for mode, want in ((_abi.MODE_FP64, name), (_abi.MODE_FP32_BULK, "patch_step")):
+        m = SolidMechanicsModel(build(kind, n, 0), [material_from_dict(ELASTIC)], precision=mode,
+                                **patch)
+        m.initFull()
+        assert lib().akb_kernel_name(m.handle, 0).decode() == want
+        assert lib().akb_kernel_name(m.handle, 1).decode() == "patch_finish_list"
+        m.close()
