@@ -35,3 +35,17 @@ def test_adam_leaves_the_weights_it_reports(width, nh):
     y = net.forward_features(X).cpu().numpy()
     net.set_parameters(net.get_parameters())
     assert np.array_equal(net.forward_features(X).cpu().numpy(), y)
+
+
+@pytest.mark.parametrize("width,nh", [(256, 3), (128, 1)])
+def test_adam_leaves_the_transposed_weights_too(width, nh):
+    """The transposed copies, which only the backward pass reads: the gradients
+    after some steps are those of a fresh upload of the same weights."""
+    from tests.test_gpu_mlp import setup
+    net, X, T, x, t, O = setup(nb=300, seed=6, width=width, nh=nh)
+    for _ in range(3):
+        net.train_step_features(X, T, 1e-2)
+    loss, g = net.gradients_features(X, T)
+    net.set_parameters(net.get_parameters())
+    loss2, g2 = net.gradients_features(X, T)
+    assert loss == loss2 and np.array_equal(g, g2)

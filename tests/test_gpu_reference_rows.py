@@ -42,3 +42,34 @@ def test_bitwise_at_tile_edges(k):
               _abi.FIELD_INTERNAL_FORCE):
         assert np.array_equal(dev.getField(f), cpu.get(f)), f
     dev.close()
+
+
+@pytest.mark.parametrize("k", range(len(MESHES)))
+def test_the_step_leaves_its_gradients_and_stresses(k):
+    """grad u and the stress as the step's element kernel writes them (read in
+    place: a copy to the host computes them anew), bit for bit."""
+    import torch
+    from akantu_b200.model import MaterialElastic, SolidMechanicsModel
+    mesh = MESHES[k]()
+    x = np.asarray(mesh.nodes)
+    rng = np.random.default_rng(100 + k)
+    v0 = rng.normal(size=x.shape)
+    cpu = OracleAdapter(mesh, dict(kind=_abi.MATERIAL_ELASTIC, rho=2700.0, E=70e9, nu=0.3))
+    dev = SolidMechanicsModel(mesh, [MaterialElastic(rho=2700.0, E=70e9, nu=0.3)])
+    dev.initFull()
+    dt = 0.3 * dev.getStableTimeStep()
+    dev.setTimeStep(dt)
+    cpu.set_time_step(dt)
+    dev.setField(_abi.FIELD_VELOCITY, v0)
+    cpu.set(_abi.FIELD_VELOCITY, v0)
+    views = {f: dev.deviceTensor(f) for f in (_abi.FIELD_GRAD_U, _abi.FIELD_STRESS)}
+    for t in views.values():
+        t.fill_(7.0)
+    torch.cuda.synchronize()
+    dev.solveSteps(3)
+    dev.synchronize()
+    cpu.solve_steps(3)
+    for f, t in views.items():
+        rows = t.transpose(1, 2).reshape(t.shape[0], -1).cpu().numpy()  # column-major again
+        assert np.array_equal(rows, np.asarray(cpu.get(f)).reshape(rows.shape)), f
+    dev.close()

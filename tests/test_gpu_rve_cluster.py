@@ -119,3 +119,27 @@ def test_stress_does_not_tell_the_kernel(kinds):
     idx = torch.arange(few, dtype=torch.int32, device="cuda")
     R.solve_indexed(idx, torch.tensor([few], dtype=torch.int32, device="cuda"), Hc, Pi)
     assert torch.equal(Pi.reshape(-1, 3, 3).transpose(1, 2), alone["stress"])
+
+
+@pytest.mark.parametrize("cells", [2, 4, 6, 8, 10, 12, 14, 16])
+def test_internal_force_matches_oracle(cells):
+    """The internal force of given states, the reads of the neighbour CTA's
+    planes among them, against the FP64 oracle on the same (FP32) fluctuation.
+    A node's force adds 8 voxels' corner forces, each the sum of three edge
+    sums of 8 Gauss points: at most some 100 roundings of 6e-8 on terms of the
+    size of the largest force, 2e-5 with a margin of three."""
+    import torch
+    from akantu_b200.rve import SolidMechanicsModelRVE
+    from tests.fe2_cases import oracle_rve
+    rng = np.random.default_rng(cells)
+    vm = (rng.random(cells ** 3) < 0.3).astype(np.uint8)
+    mats = fe2.matrix_inclusion_materials()
+    H = fe2.sample_gradients(3, seed=cells, amplitude=0.1)
+    w = (0.05 / cells * rng.uniform(-1, 1, (3, cells ** 3, 3))).astype(np.float32)
+    R = SolidMechanicsModelRVE(cells, vm, mats, precision=_abi.MODE_FP32_BULK)
+    P, f = R.stress(H, torch.as_tensor(w, device="cuda"))
+    O = oracle_rve(cells, vm, mats)
+    for k in range(3):
+        Po, fo = O.stress(H[k], w[k].astype(np.float64))
+        assert np.abs(f[k].cpu().numpy() - fo).max() <= 2e-5 * np.abs(fo).max(), k
+        assert np.abs(P[k].cpu().numpy() - Po).max() <= 2e-5 * np.abs(Po).max(), k
