@@ -842,7 +842,7 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
     bool fans = use_fans(m.get(), ne);
     if (fans) {
       st = plan_patches(m.get(), mesh, batch, part, true, plan, patch_inst, orphan_inst);
-      fans = st == AKB_OK && fan_smem_bytes(plan, d) <= 227 * 1024;
+      fans = st == AKB_OK && fan_smem_bytes(plan, d) <= kFanSmemLimit;
     }
     if (fans && type == AKB_HEXAHEDRON_8) m->linear = mark_affine(mesh, plan);
     if (!fans &&

@@ -261,6 +261,7 @@ size_t patch_smem_bytes(const DevPatches& p, int dim, bool fp32, int nbuf);
 // Shared memory of k_fan_step for a plan; its configuration on the device
 // (resident[2]: its CTAs that run at the same time, without and with f_ext).
 size_t fan_smem_bytes(const PatchHost& p, int dim);
+constexpr size_t kFanSmemLimit = 227 * 1024 - 256;  // (its static 128 bytes count too)
 cudaError_t fan_configure(const DevModel& m, const DevPatches& p, int device, int* resident);
 // Chunk record buffers (1 or 2) that keep the most CTAs per SM.
 int patch_buffers(const DevPatches& p, int type, bool fp32);

@@ -141,3 +141,27 @@ def test_kernel_of_each_side(kind, n, patch, name):
         assert lib().akb_kernel_name(m.handle, 0).decode() == want
         assert lib().akb_kernel_name(m.handle, 1).decode() == "patch_finish_list"
         m.close()
+
+
+def test_a_plan_that_just_misses_an_sm():
+    """One patch whose fan layout takes 48 bytes less than an SM's 227 KB, which
+    the kernel's static shared memory no longer leaves: chunk records."""
+    from akantu_b200._lib import lib
+    from akantu_b200.mesh import Mesh
+    from akantu_b200.model import SolidMechanicsModel, material_from_dict
+    box = box_tetrahedron4(8, 8, 8, 8.0, 8.0, 8.0)
+    nodes, conn = [box.nodes], [box.connectivity.astype(np.int64)]
+    for j in range(1, 15):  # tetrahedra of their own
+        z = 100.0 + 3 * j
+        conn.append(np.arange(4)[None] + sum(len(x) for x in nodes))
+        nodes.append(np.array([[0, 0, z], [1, 0, z], [0, 1, z], [0, 0, z + 1]], dtype=float))
+    mesh = Mesh(3, _abi.TETRAHEDRON_4, np.concatenate(nodes),
+                np.concatenate(conn).astype(np.uint32))
+    m = SolidMechanicsModel(mesh, [material_from_dict(ELASTIC)], precision=_abi.MODE_FP64,
+                            patch_elements=8191, patch_nodes=6000)
+    m.initFull()
+    assert lib().akb_kernel_name(m.handle, 0).decode() == "patch_step"
+    m.setTimeStep(0.5 * m.getStableTimeStep())
+    m.solveSteps(2)
+    assert np.isfinite(m.getDisplacement()).all()
+    m.close()
