@@ -4,7 +4,8 @@ One BatchModel holds thousands of meshes of one element type, each with its
 own material and time step. Each instance is split into patches on its own,
 so the fused patch kernel advances every instance in the same launch and each
 instance's state is bitwise the one a SolidMechanicsModel of that mesh alone
-produces with the same patch options.
+produces with the same patch_elements > 0 (by default, 0, the patch size goes by
+the number of elements, here of the whole batch) and patch_nodes.
 """
 from __future__ import annotations
 

@@ -118,13 +118,16 @@ cudaError_t apply_dirichlet(const DevModel& m, const uint32_t* nodes, int64_t n,
                             const double* values, const uint32_t* perm, double* w,
                             cudaStream_t s);
 
-// A list short enough for the kernel's parameters (the model takes about 0.7 of
-// their 4 KB): at most kInlineDirichlet values.
+// A list short enough for the kernel's parameters: at most kInlineDirichlet
+// values (2.3 KB beside the model's 0.7 KB, copied at every launch; the
+// parameters end at 4 KB on older toolkits).
 constexpr int kInlineDirichlet = 192;
 struct InlineDirichlet {
   double values[kInlineDirichlet];
   uint32_t nodes[kInlineDirichlet];
 };
+static_assert(sizeof(DevModel) + sizeof(InlineDirichlet) + 4 * sizeof(void*) <= 4096,
+              "the launch parameters of k_apply_dirichlet_inline");
 cudaError_t apply_dirichlet_inline(const DevModel& m, const InlineDirichlet& list, int n, int comp,
                                    const uint32_t* perm, double* w, cudaStream_t s);
 

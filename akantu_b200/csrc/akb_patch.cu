@@ -581,13 +581,13 @@ __global__ void __launch_bounds__(kThreads, (PatchOccupancy<T, S>::value))
 }
 
 // ------------------------------------------------------------- fan records
-// The fused step on fan records (akb_patch.cuh: FP64 triangles and
-// tetrahedra). As k_patch_step, with two differences:
-//  - a thread computes a fan, a row of elements around a hinge, keeping the
-//    hinge and the last ring node in registers: each further element loads one
-//    node and writes one contribution. An element costs about 105 FP64
-//    operations (the hinge's cross products are shared between neighbours)
-//    and a quarter of the shared-memory traffic of its corner-by-corner form;
+// The fused step on fan records (akb_patch.cuh: FP64 triangles, tetrahedra and
+// hexahedra). As k_patch_step, with two differences:
+//  - triangles and tetrahedra: a thread computes a fan, a row of elements around
+//    a hinge, keeping the last ring node in registers: each further element loads
+//    one node, re-reads the hinge and writes one contribution. A tetrahedron costs
+//    about 105 FP64 operations (the hinge's cross products are shared between
+//    neighbours). Hexahedra are fans of one element (hex_force_f64);
 //  - all contributions of the patch stay in shared memory, so that the node
 //    sums run once per patch and feed the finish directly: two barriers a
 //    patch instead of two per 256 elements, and no force accumulators.

@@ -1,6 +1,9 @@
 // akb_rve.cu -- batched periodic RVE solves (the micro problems of FE^2).
 //
-// One CTA relaxes one RVE with its whole state on chip: the fluctuation w,
+// FP32 RVEs of up to 16^3 cells (but 14^3, whose planes divide by neither 2 x 2
+// nor 4 x 2; of 16^3 fewer than kManyInstances) are relaxed by a cluster of CTAs
+// each: k_rve_cluster, below. All others by k_rve and k_rve_indexed:
+// one CTA relaxes one RVE with its whole state on chip: the fluctuation w,
 // the velocity and the force of the n^3 periodic nodes (component-major),
 // the inverse fictitious mass, the voxel materials and the voxel shape
 // gradients live in shared memory (n = 16 in FP32: 170 KB), so an iteration
@@ -603,7 +606,9 @@ __global__ void __launch_bounds__(kRveThreads, 1)
 //    and each node then adds its 8 voxels' in colour order, the order in which
 //    the coloured scatter added them (the same sums bit for bit), so that a
 //    step is two cluster barriers instead of ten CTA barriers and all voxels
-//    are computed at once: 16 warps of 128 registers instead of 8 of 213;
+//    are computed at once: 16 warps of 128 registers instead of 8 of 227. The
+//    edge differences, edge sums and stresses of a voxel do not fit 128: 324 to
+//    340 bytes a thread are spilled (220 with one CTA), 548 to 576 (348) read back;
 //  - the planes are spread over C SMs. A CTA reads the forces of the layer
 //    below its first plane, and writes the displacements of that plane, in the
 //    neighbour's shared memory.

@@ -348,12 +348,13 @@ def run_ours(args, dist):
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": peak_kind,
                          "algorithmic_bytes_per_step": balg,
-                         # DRAM bytes of one k_fan_step launch from an ncu capture
-                         # (dram__bytes rate x duration) of the
-                         # 90^3-cell cube (4.374 M elements, 134.7 MB), scaled by
-                         # elements; the capture is not taken inside this run
-                         "traffic": 134.7e6 * E / 4.374e6,
-                         "traffic_kernel": "k_fan_step (ncu, 90^3 cells, scaled by elements)",
+                         # DRAM bytes of one cold launch of each of the step's two
+                         # kernels (k_fan_step 134.7 MB, k_finish_list 47.8 MB) from an
+                         # ncu capture of the 90^3-cell cube; not taken inside this run,
+                         # and without the write-back of what a launch leaves in L2
+                         "traffic": 134.7e6 + 47.8e6,
+                         "traffic_kernel": "k_fan_step + k_finish_list, one cold launch each "
+                                           "(ncu, 90^3 cells, 203 MB of algorithmic bytes)",
                          "kernels_ms": {n: t for n, t in ktimes},
                          "dominant": top[0]},
             "clocks": clocks,
@@ -553,13 +554,12 @@ def run_hex8(args, device, peak):
             "rel_err_displacement": float(np.abs(u32 - u64).max() / np.abs(u64).max()),
             "rel_err_internal_force": float(np.abs(f32 - f64).max() / np.abs(f64).max())}
     out["time_step"] = dt
-    # pipe use of the FP32-bulk launch, from an ncu capture of this workload
-    # (% of peak; not taken in this run)
+    # pipe use of the fused launches, from ncu captures of the 96^3 block
+    # (share of peak; not taken in this run)
     out["compute_roofline"] = {"bound": "fp64 pipe (FP64) / fma pipe (FP32-bulk)",
-                               "fp32_bulk_fma_pipe_active": 0.413,
-                               "kernel": "k_patch_step<hex8, float>",
-                               "source": "ncu capture of the 96^3 block "
-                                         "(profiles/k_patch_step_block_hex8_96.md)"}
+                               "fp64_pipe_active": 0.484, "fp32_bulk_fma_pipe_active": 0.413,
+                               "kernel": "k_fan_step<hex8> / k_patch_step<hex8, float>",
+                               "source": "ncu captures of the 96^3 block"}
     return out
 
 
@@ -731,7 +731,9 @@ def run_fe2(args, device, log=None):
         torch.cuda.synchronize()
         return a.elapsed_time(b), r
 
-    # RVE solves: held-out samples (another seed than the training set's)
+    # RVE solves: held-out samples (another seed than the training set's), after
+    # one pass that loads the kernel and the host's sampling
+    fe2.generate_dataset(rve, args.fe2_heldout, seed=7)
     ms, (Xh, Yh, it, _) = timed(lambda: fe2.generate_dataset(rve, args.fe2_heldout, seed=7))
     out["rve"] = {"solves": args.fe2_heldout, "ms": ms,
                   "solves_per_s": args.fe2_heldout / ms * 1e3,

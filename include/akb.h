@@ -118,10 +118,10 @@ typedef struct {
   void* stream;           /* cudaStream_t to run on; NULL = library-owned stream */
   int32_t patch_elements; /* fast modes: elements per patch (0 = per-type default) */
   int32_t patch_nodes;    /* fast modes: node cap of a patch (0 = per-type default) */
-  int32_t patch_grid;     /* fast modes: 0 = the default (FP64 triangles, tetrahedra and
-                             hexahedra: as many CTAs as run at once, striding over the
-                             patches; otherwise one CTA per patch); > 0 = a grid of that
-                             many CTAs striding over the patches */
+  int32_t patch_grid;     /* fast modes: 0 = the default (where akb_kernel_name says
+                             "fan_step", most FP64 meshes: as many CTAs as run at once,
+                             striding over the patches; otherwise one CTA per patch);
+                             > 0 = a grid of that many CTAs striding over the patches */
 } akb_model_options;
 
 typedef struct {
@@ -212,13 +212,14 @@ akb_status akb_compute_stresses(akb_model* model);
 
 /* SolidMechanicsModel::getEnergy (solid_mechanics_model.cc:665-683). */
 akb_status akb_get_energy(akb_model* model, int32_t kind, double* value);
-/* The same without waiting: the reduction and the copy of its result to
- * *value are queued on the model's stream, and *value is written when the
- * stream reaches them; read it after akb_synchronize (the copy itself runs
- * on a stream of the library's, so an event of the model's stream does not
- * cover it). value: host memory (pinned, for the copy to run
- * asynchronously) or device memory. Lets a time loop that records the
- * energies of every step (examples/explicit/explicit_dynamic.cc:87-99) run
+/* The same without waiting: *value is written when the model's stream reaches
+ * this call; read it after akb_synchronize. 8-byte aligned memory of the
+ * model's device, or pinned host memory mapped to it, is written by the
+ * reduction itself, on the model's stream (an event of that stream covers it).
+ * Any other memory (pageable, managed, unaligned, another device's) gets a
+ * copy on a stream of the library's, which such an event does not cover; to
+ * pageable memory the copy is not asynchronous. Lets a time loop that records
+ * the energies of every step (examples/explicit/explicit_dynamic.cc:87-99) run
  * without a host round trip per step. No reference counterpart. */
 akb_status akb_get_energy_async(akb_model* model, int32_t kind, double* value);
 
@@ -252,8 +253,13 @@ const char* akb_kernel_name(const akb_model* model, int32_t slot);
  * Batches: many independent meshes of one element type stepped together.
  * No counterpart in the reference (it runs one SolidMechanicsModel per
  * process); each instance follows the single-model path exactly: its own
- * material (one per instance), its own time step, the same per-instance
- * patches, so its state is bitwise the one a model of that mesh alone gives.
+ * material (one per instance), its own time step, patches of its own, so its
+ * state is bitwise the one a model of that mesh alone gives with the same
+ * patch_elements > 0 (and patch_nodes). With patch_elements = 0 the patch
+ * size goes by the number of elements, the whole batch's here, and the bits of
+ * a smaller model can differ (hexahedra in AKB_MODE_FP64 excepted: one size).
+ * They can also where patch_nodes above the default lets a patch outgrow an
+ * SM's shared memory: all instances then step on the other kind of records.
  * The batch is an akb_model over the union mesh (instances concatenated in
  * order; fields, blocked DOFs, Dirichlet values and akb_solve_steps work on
  * the union arrays). Fast modes only (AKB_MODE_FP64, AKB_MODE_FP32_BULK). */

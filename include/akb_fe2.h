@@ -73,7 +73,8 @@ typedef struct {
   int32_t precision_mode;
   int64_t nb_nodes;          /* n^3 unique periodic nodes */
   double volume_fraction[8]; /* voxel fraction of each material */
-  int64_t shared_bytes;      /* shared memory of one RVE solve */
+  int64_t shared_bytes;      /* shared memory of a solve by one CTA (a cluster's
+                                CTAs, which relax small FP32 RVEs, take less each) */
 } akb_rve_info;
 
 typedef struct akb_rve akb_rve;
@@ -92,7 +93,9 @@ akb_status akb_rve_get_info(const akb_rve* rve, akb_rve_info* info);
  *   stress     [nb][9]        homogenised first Piola-Kirchhoff stress;
  *   iterations [nb]           updates done (may be NULL);
  *   residual   [nb]           final max|f| / (h^2 max(mu) max(|H_ij|, 1e-6))
- *                             (may be NULL; +inf if the relaxation diverged). */
+ *                             (may be NULL; +inf if the relaxation diverged).
+ * An RVE's results have the same bits alone, in a batch of any size and listed
+ * (akb_rve_solve_indexed), whichever kernel relaxes it. */
 akb_status akb_rve_solve(akb_rve* rve, int64_t nb, const double* grad_u, void* fluctuation,
                          double* stress, int32_t* iterations, double* residual, void* stream);
 
