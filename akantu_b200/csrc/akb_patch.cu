@@ -639,9 +639,10 @@ template <bool LIN> struct FanBuild<AKB_TRIANGLE_3, LIN> {
 // Hexahedra: FP64 issue bound, 255 registers for the signed sums and the 36
 // accumulators, so 8 warps an SM; 128-thread CTAs (a 128-element patch each)
 // overlap one patch's staging and finish with the other's elements. 64^3
-// neo-Hookean block: 79.5 us a step (256-element chunks in one 256-thread CTA
-// 95.1; 4 x 64 threads 81.4; 1 x 256 threads 126; 3 x 128 at 168 registers,
-// spilling, 86.8); 37 x 31 x 33 distorted 17.0 against 31.3.
+// neo-Hookean block: 77.1 us a step, and 79.5 when the others were measured
+// (256-element chunks in one 256-thread CTA 95.1; 4 x 64 threads 81.4; 1 x 256
+// threads 126; 3 x 128 at 168 registers, spilling, 86.8); 37 x 31 x 33 distorted
+// 16.7 against 31.3.
 template <bool PAR> struct FanBuild<AKB_HEXAHEDRON_8, PAR> {
   static constexpr int threads = 128, ctas = 2;
 };
