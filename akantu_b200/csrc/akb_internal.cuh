@@ -86,9 +86,11 @@ akb_status fail(akb_status s, const std::string& msg);
 #define AKB_CUDA_TRY(expr)                                                  \
   do {                                                                      \
     cudaError_t _e = (expr);                                                \
-    if (_e != cudaSuccess)                                                  \
+    if (_e != cudaSuccess) {                                                \
+      cudaGetLastError(); /* reported here, not by the next launch */       \
       return ::akb::fail(AKB_ERR_CUDA, std::string(#expr) + ": " +          \
                                            cudaGetErrorString(_e));         \
+    }                                                                       \
   } while (0)
 
 // Kernel launchers (reference-order path: akb_reference.cu).

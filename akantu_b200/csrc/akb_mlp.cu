@@ -915,8 +915,13 @@ Layout layout_of(const akb_mlp* m) {
 
 akb_status ensure_workspace(akb_mlp* m, int64_t ntiles) {
   if (ntiles <= m->cap_tiles) return AKB_OK;
+  // nothing of the old workspace is left to use, should an allocation fail
   for (void* p : m->work) cudaFree(p);
   m->work.clear();
+  m->bufs = Bufs{};
+  m->cap_tiles = 0;
+  if (m->h_loss) cudaFreeHost(m->h_loss);
+  m->h_loss = nullptr;
   const Net& n = m->net;
   const size_t rows = (size_t)ntiles * kTile;
   Bufs b{};
@@ -927,9 +932,8 @@ akb_status ensure_workspace(akb_mlp* m, int64_t ntiles) {
   }
   AKB_CUDA_TRY(dmalloc(m->work, &b.ynorm, rows * 16));
   AKB_CUDA_TRY(dmalloc(m->work, &b.loss_tiles, (size_t)ntiles));
-  m->bufs = b;
-  if (m->h_loss) cudaFreeHost(m->h_loss);
   AKB_CUDA_TRY(cudaMallocHost((void**)&m->h_loss, ntiles * sizeof(float) + sizeof(int)));
+  m->bufs = b;
   m->cap_tiles = ntiles;
   return AKB_OK;
 }

@@ -49,3 +49,20 @@ def test_adam_leaves_the_transposed_weights_too(width, nh):
     net.set_parameters(net.get_parameters())
     loss2, g2 = net.gradients_features(X, T)
     assert loss == loss2 and np.array_equal(g, g2)
+
+
+def test_a_batch_too_large_for_memory_leaves_the_network_usable():
+    """The workspace of 2^34 samples (550 GB for the inputs alone) is refused
+    before any launch; the next call of an ordinary size has a workspace again."""
+    import ctypes as C
+    from akantu_b200._lib import AkbError, check, lib
+    from tests.test_gpu_mlp import setup
+    net, X, T, x, t, O = setup(nb=300, seed=7, width=128, nh=1)
+    loss, g = net.gradients_features(X, T)
+    out = np.zeros(net.nb_parameters, np.float32)
+    value = C.c_float()
+    with pytest.raises(AkbError, match="memory"):
+        check(lib().akb_mlp_gradients(net._h, 2 ** 34, X.data_ptr(), T.data_ptr(),
+                                      out.ctypes.data_as(C.POINTER(C.c_float)), C.byref(value)))
+    loss2, g2 = net.gradients_features(X, T)
+    assert loss == loss2 and np.array_equal(g, g2)
