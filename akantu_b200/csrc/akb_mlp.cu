@@ -445,6 +445,16 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
       used += K / net.ks[l];
       while (ok && ll < net.nl && loaded < used + kRing) load_next();
     }
+    // the biases of the epilogue's first columns, requested under the MMAs (and
+    // each next 32 under the activations of the ones before): one hidden layer of
+    // 128, 8192 samples 6.98 -> 6.24 us, three of 256 19.4 -> 18.5
+    const float* __restrict__ bias = net.b[l];
+    const bool last = l == net.nl - 1;
+    const int cbeg = last ? 0 : half * (N >> 1), cend = (half + 1) * (N >> 1);
+    float4 b4[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < 4 || !last) b4[q] = __ldg(reinterpret_cast<const float4*>(bias + cbeg) + q);
     // lanes that waited on the barrier below while one of their warp still
     // issues would suspend the warp, 3000 cycles at a time
     __syncwarp();
@@ -455,20 +465,21 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
       break;
     }
     fence_after();
-    const float* __restrict__ bias = net.b[l];
-    const bool last = l == net.nl - 1;
     if (!last) {
-      for (int c0 = half * (N >> 1); c0 < (half + 1) * (N >> 1); c0 += 32) {
+      for (int c0 = cbeg; c0 < cend; c0 += 32) {
         float v[32];
         tmem_ld32(mine + c0, v);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const float4 b4 = __ldg(reinterpret_cast<const float4*>(bias + c0) + q);
-          v[4 * q] += b4.x;
-          v[4 * q + 1] += b4.y;
-          v[4 * q + 2] += b4.z;
-          v[4 * q + 3] += b4.w;
+          v[4 * q] += b4[q].x;
+          v[4 * q + 1] += b4[q].y;
+          v[4 * q + 2] += b4[q].z;
+          v[4 * q + 3] += b4[q].w;
         }
+        if (c0 + 32 < cend)
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            b4[q] = __ldg(reinterpret_cast<const float4*>(bias + c0 + 32) + q);
         if (TRAIN && row < nb) {  // the pre-activations: eight 16-byte stores
           float4* z4 = reinterpret_cast<float4*>(bufs.z[l] + (size_t)row * N + c0);
 #pragma unroll
@@ -490,8 +501,15 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
       tmem_ld16(mine, v);
       if (row < nb) {
         const double scale = STRESS ? hnorm : 1.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          v[4 * q] += b4[q].x;
+          v[4 * q + 1] += b4[q].y;
+          v[4 * q + 2] += b4[q].z;
+          v[4 * q + 3] += b4[q].w;
+        }
         for (int j = 0; j < 16; ++j) {
-          const float yy = v[j] + bias[j];
+          const float yy = v[j];
           if (TRAIN) bufs.ynorm[row * 16 + j] = yy;
           if (!TRAIN && j < net.nout)
             y[row * net.nout + j] = scale * ((double)yy * net.out_scale[j] + net.out_shift[j]);
