@@ -622,6 +622,11 @@ __global__ void __launch_bounds__(kRveThreads, 1)
 // about the same number of updates, 512 43 and 43, 1024 85 and 77, 2048 171 and 152.
 // (Fewer CTAs per RVE are faster at any count: 4096 of 8^3 76 -> 28 ms.)
 constexpr int64_t kManyInstances = 2560;
+// Calls without updates (akb_rve_stress) have no slowest instance: four CTAs per
+// RVE are faster only while few waves of clusters hold them all. 16^3, us by
+// clusters and by k_rve: 20 states 98 and 196, 72 190 and 196, 100 236 and 204,
+// 1000 1600 and 1130.
+constexpr int kStressWaves = 2;
 
 struct ClusterLayout {
   int u, v, im, B, F, mat, red, total;  // byte offsets
@@ -1064,7 +1069,8 @@ akb_status launch(akb_rve* r, int max_it, int64_t nb, const double* grad_u, void
   if (r->mode == AKB_MODE_FP64)
     k_rve<double><<<(unsigned)nb, kRveThreads, r->smem, s>>>(
         a, nb, grad_u, static_cast<double*>(fluct), stress, iterations, residual, force);
-  else if (const int C = cluster_of(r->n); C && (C < 4 || nb < kManyInstances))
+  else if (const int C = cluster_of(r->n);
+           C && (C < 4 || nb < (max_it ? kManyInstances : kStressWaves * r->clusters + 1)))
     AKB_CUDA_TRY(launch_cluster<false>(C, a, nb, nb, nullptr, nullptr, grad_u, fluct, stress,
                                        iterations, residual, force, s));
   else
