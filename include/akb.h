@@ -214,11 +214,12 @@ akb_status akb_compute_stresses(akb_model* model);
 akb_status akb_get_energy(akb_model* model, int32_t kind, double* value);
 /* The same without waiting: *value is written when the model's stream reaches
  * this call; read it after akb_synchronize. 8-byte aligned memory of the
- * model's device, or pinned host memory mapped to it, is written by the
- * reduction itself, on the model's stream (an event of that stream covers it).
- * Any other memory (pageable, managed, unaligned, another device's) gets a
- * copy on a stream of the library's, which such an event does not cover; to
- * pageable memory the copy is not asynchronous. Lets a time loop that records
+ * model's device and, for the kinetic energy, pinned host memory mapped to it
+ * are written by the reduction itself, on the model's stream (an event of that
+ * stream covers it). Anything else (the other energies to pinned memory;
+ * pageable, managed, unaligned, another device's memory) is copied on a stream
+ * of the library's, which such an event does not cover; to pageable memory the
+ * copy is not asynchronous. Lets a time loop that records
  * the energies of every step (examples/explicit/explicit_dynamic.cc:87-99) run
  * without a host round trip per step. No reference counterpart. */
 akb_status akb_get_energy_async(akb_model* model, int32_t kind, double* value);
