@@ -251,22 +251,30 @@ akb_status upload(akb_model* m, const std::vector<T>& v, const T** out);
 // (912 k tetrahedra 42.1 us a step against 42.3, 422 k hexahedra 104.7 against
 // 98.9), and fans of several elements exist for FP64 only.
 //  - Small meshes: a fan is a serial chain of up to eight elements, and with
-//    few patches nothing else hides it. Chunk records against fan records, us a
-//    step: 312 triangles 5.3 against 5.7, 1600 6.10 against 6.23, 4800 6.4
-//    against 6.1; 288 tetrahedra 6.3 against 6.9, 600 7.0 against 7.1, 1080 7.5
-//    against 7.05. Hexahedra: faster on fan records from 294 elements on.
+//    few patches nothing else hides it, the less the longer the material law.
+//    Steps of chunk records against fan records, us. Small strain: 2048 triangles
+//    5.72 against 5.78, 3200 5.97 and 6.17, 4802 6.17 and 5.97, 24 k 6.60 and 6.23;
+//    1296 tetrahedra 7.19 and 7.50, 3072 7.64 and 7.76, 4860 8.15 and 7.95, 41 k
+//    10.3 and 9.1. Finite-strain elastic: 24 k triangles 6.54 and 6.80, 40 k 6.96
+//    and 7.03, 80 k 8.7 and 7.7; 20 k tetrahedra 8.7 and 9.6, 41 k 10.7 and 10.8, 79 k
+//    14.3 and 10.9. Neo-Hookean: 40 k triangles 7.5 and 9.3, 80 k 9.7 and 9.9, 160 k
+//    15.7 and 10.8; 20 k tetrahedra 9.2 and 12.0, 41 k 11.5 and 13.4, 79 k 15.5 and
+//    13.5. (A step by itself, which nothing follows, takes the fans of 5 k to 30 k
+//    small-strain triangles 1 us longer.) Hexahedra: faster on fan records at any size.
 //  - Patch sizes chosen by the caller: the fan kernels are built for patches
 //    whose fans fill their CTA about once. 280 k triangles at 768 elements 19.8
 //    against 16.2, at 1024 16.6 against 18.5, at 2048 23.7 against 30.7; 1.6 M
 //    tetrahedra at 512 72 against 87, at 768 65 against 49, at 1536 63 against
 //    40; 262 k hexahedra at 256 141 against 79, at 384 101.2 against 101.6, at
 //    512 95 against 104.
-bool use_fans(const akb_model* m, int64_t ne) {
+bool use_fans(const akb_model* m, int64_t ne, bool neohookean) {
   if (m->mode != AKB_MODE_FP64) return false;
   const int pe = m->opt_patch_elements;
   switch (m->dm.type) {
-  case AKB_TRIANGLE_3: return pe > 0 ? pe <= 768 : ne >= 2048;
-  case AKB_TETRAHEDRON_4: return pe > 0 ? pe >= 768 : ne >= 768;
+  case AKB_TRIANGLE_3:
+    return pe > 0 ? pe <= 768 : ne >= (neohookean ? 88000 : m->linear ? 4096 : 45000);
+  case AKB_TETRAHEDRON_4:
+    return pe > 0 ? pe >= 768 : ne >= (neohookean ? 56000 : m->linear ? 4096 : 44000);
   case AKB_HEXAHEDRON_8: return pe <= 256;
   default: return false;
   }
@@ -815,14 +823,17 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
   dm.nn = nn;
   dm.ne = ne;
   dm.nmat = nb_materials;
+  bool neohookean = false;  // any of the materials
   akb_status st;
   {
     std::vector<MatParams> table(nb_materials);
     for (int k = 0; k < nb_materials; ++k) table[k] = make_params(materials[k], d);
     for (int k = 0; k < nb_materials && k < kMaxMaterials; ++k) dm.mats[k] = table[k];
     m->linear = true;
-    for (const MatParams& t : table)
+    for (const MatParams& t : table) {
       m->linear = m->linear && t.kind == AKB_MATERIAL_ELASTIC && !t.finite;
+      neohookean = neohookean || t.kind == AKB_MATERIAL_NEOHOOKEAN;
+    }
     if ((st = upload(m.get(), table, &dm.mat_table)) != AKB_OK) return st;
     AKB_CUDA_TRY(cudaStreamSynchronize(m->stream));
   }
@@ -841,7 +852,7 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
   if (patched) {
     // FP64 steps run on fan records where these are faster (use_fans), but a
     // plan whose record or contributions do not fit an SM steps chunk by chunk
-    bool fans = use_fans(m.get(), ne);
+    bool fans = use_fans(m.get(), ne, neohookean);
     if (fans) {
       st = plan_patches(m.get(), mesh, batch, part, true, plan, patch_inst, orphan_inst);
       fans = st == AKB_OK && fan_smem_bytes(plan, d) <= kFanSmemLimit;

@@ -113,34 +113,54 @@ def test_both_sides_of_the_dispatch(kind, n, mats, patch):
     test_against_oracle(kind, n, mats, 1, patch, True)
 
 
-@pytest.mark.parametrize("kind,n,patch,name", [
-    ("tri", (33, 31), {}, "patch_step"), ("tri", (31, 33), {}, "patch_step"),
-    ("tri", (32, 32), {}, "fan_step"), ("tri", (341, 3), {}, "patch_step"),
-    ("tet", (8, 4, 4), {}, "fan_step"), ("tet", (127, 1, 1), {}, "patch_step"),
-    ("tri", (60, 20), dict(patch_elements=768), "fan_step"),
-    ("tri", (60, 20), dict(patch_elements=769), "patch_step"),
-    ("tri", (8, 3), dict(patch_elements=256), "fan_step"),
-    ("tet", (9, 8, 6), dict(patch_elements=767), "patch_step"),
-    ("tet", (9, 8, 6), dict(patch_elements=768), "fan_step"),
-    ("hex", (1, 1, 1), {}, "fan_step"),
-    ("hex", (8, 8, 8), dict(patch_elements=256), "fan_step"),
-    ("hex", (8, 8, 8), dict(patch_elements=257), "patch_step"),
-    ("tet", (20, 20, 20), dict(patch_elements=8191, patch_nodes=6000), "patch_step"),
+@pytest.mark.parametrize("kind,n,law,patch,name", [
+    ("tri", (2047, 1), ELASTIC, {}, "patch_step"), ("tri", (64, 32), ELASTIC, {}, "fan_step"),
+    ("tet", (31, 11, 2), ELASTIC, {}, "patch_step"), ("tet", (683, 1, 1), ELASTIC, {}, "fan_step"),
+    ("tri", (149, 151), FINITE, {}, "patch_step"), ("tri", (150, 150), FINITE, {}, "fan_step"),
+    ("tet", (19, 19, 20), FINITE, {}, "patch_step"), ("tet", (20, 20, 19), FINITE, {}, "fan_step"),
+    ("tri", (200, 219), NEO, {}, "patch_step"), ("tri", (200, 220), NEO, {}, "fan_step"),
+    ("tet", (21, 21, 21), NEO, {}, "patch_step"), ("tet", (21, 21, 22), NEO, {}, "fan_step"),
+    ("tri", (60, 20), ELASTIC, dict(patch_elements=768), "fan_step"),
+    ("tri", (60, 20), ELASTIC, dict(patch_elements=769), "patch_step"),
+    ("tri", (8, 3), NEO, dict(patch_elements=256), "fan_step"),
+    ("tet", (9, 8, 6), ELASTIC, dict(patch_elements=767), "patch_step"),
+    ("tet", (9, 8, 6), NEO, dict(patch_elements=768), "fan_step"),
+    ("hex", (1, 1, 1), NEO, {}, "fan_step"),
+    ("hex", (8, 8, 8), NEO, dict(patch_elements=256), "fan_step"),
+    ("hex", (8, 8, 8), NEO, dict(patch_elements=257), "patch_step"),
+    ("tet", (20, 20, 20), ELASTIC, dict(patch_elements=8191, patch_nodes=6000), "patch_step"),
 ])
-def test_kernel_of_each_side(kind, n, patch, name):
-    """akb_kernel_name says which kernel steps the model: fan records from 2048
-    triangles and 768 tetrahedra on and for the patch sizes they are built for;
-    chunk records below, beside them, in FP32 and where a patch of fans does not
-    fit an SM."""
+def test_kernel_of_each_side(kind, n, law, patch, name):
+    """akb_kernel_name says which kernel steps the model: fan records from 4096
+    small-strain triangles or tetrahedra on, later for the longer laws, and for
+    the patch sizes they are built for; chunk records below, beside them, in FP32
+    and where a patch of fans does not fit an SM."""
     from akantu_b200._lib import lib
     from akantu_b200.model import SolidMechanicsModel, material_from_dict
     for mode, want in ((_abi.MODE_FP64, name), (_abi.MODE_FP32_BULK, "patch_step")):
-        m = SolidMechanicsModel(build(kind, n, 0), [material_from_dict(ELASTIC)], precision=mode,
+        m = SolidMechanicsModel(build(kind, n, 0), [material_from_dict(law)], precision=mode,
                                 **patch)
         m.initFull()
         assert lib().akb_kernel_name(m.handle, 0).decode() == want
         assert lib().akb_kernel_name(m.handle, 1).decode() == "patch_finish_list"
         m.close()
+
+
+@pytest.mark.parametrize("load", [False, True], ids=["free", "loaded"])
+@pytest.mark.parametrize("kind,n,mats,jitter,patch", [
+    ("tet", (1, 1, 1), ELASTIC, 0, dict(patch_elements=1536)),
+    ("tet", (7, 6, 5), [ELASTIC, STIFF], 1, dict(patch_elements=1536)),
+    ("tet", (9, 9, 4), FINITE, 0, dict(patch_elements=768, patch_grid=1)),
+    ("tet", (8, 7, 9), [FINITE, ELASTIC], 1, dict(patch_elements=1024)),
+    ("tet", (6, 5, 7), NEO, 1, dict(patch_elements=768)),
+    ("tri", (1, 1), ELASTIC, 0, dict(patch_elements=768)),
+    ("tri", (40, 31), [STIFF, ELASTIC], 1, dict(patch_elements=768)),
+    ("tri", (33, 20), [FINITE, STIFF], 1, dict(patch_elements=200, patch_grid=1)),
+    ("tri", (40, 21), NEO, 0, dict(patch_elements=512)),
+])
+def test_fans_of_small_meshes(kind, n, mats, jitter, patch, load):
+    """Meshes that step on fan records only where the caller gives the patch size."""
+    test_against_oracle(kind, n, mats, jitter, patch, load)
 
 
 def test_a_plan_that_just_misses_an_sm():
