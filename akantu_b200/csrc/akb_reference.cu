@@ -122,12 +122,19 @@ __device__ inline void rows_out(double* buf, const double* mine, double* row, in
 // every store instruction touched 32 sectors (99.7 us for 664k tetrahedra).
 // The rows go through shared memory, a warp's 32 elements at a time, so that
 // global accesses are consecutive.
+//
+// A mesh of a few hexahedra has nothing to gain from that, and its warps pay for
+// every exchange alone: up to kFewHexahedra, lanes read and write their own rows
+// (ROWS false). us a step with the exchange and without: small strain one 18.4 and
+// 11.4, 48 21.5 and 19.3, 64 21.9 and 22.5, 128 22.8 and 34.1; neo-Hookean 34.0 and
+// 24.3, 37.1 and 32.5, 37.9 and 33.1, 38.6 and 38.9.
 constexpr int kElementThreads = 128;
-template <int T>
+constexpr int kFewHexahedra = 48;
+template <int T, bool ROWS>
 __global__ void __launch_bounds__(kElementThreads) k_element_forces(DevModel m) {
   constexpr int d = ET<T>::dim, n = ET<T>::nnpe, q = ET<T>::nqp;
   constexpr int dn = d * n, dd = d * d, SN = dn | 1, SD = dd | 1;
-  __shared__ double buffers[kElementThreads / 32][32 * SN];
+  __shared__ double buffers[kElementThreads / 32][ROWS ? 32 * SN : 1];
   const int lane = threadIdx.x & 31;
   double* buf = buffers[threadIdx.x >> 5];
   const int64_t e0 = blockIdx.x * (int64_t)kElementThreads + (threadIdx.x & ~31);
@@ -138,7 +145,7 @@ __global__ void __launch_bounds__(kElementThreads) k_element_forces(DevModel m) 
   const MatParams& p = (m.mat_of ? m.mat_table[m.mat_of[e]] : m.mats[0]);
   double uel[dn], inte[dn], r[dn], B[dn];
   // the first point's derivatives are requested ahead of the predictor's end
-  rows_load<dn>(m.B + e0 * q * dn, q * dn, cnt, lane, B);
+  if constexpr (ROWS) rows_load<dn>(m.B + e0 * q * dn, q * dn, cnt, lane, B);
   grid_wait();
   gather_el<T>(m, e, m.u, uel);
 #pragma unroll
@@ -147,22 +154,40 @@ __global__ void __launch_bounds__(kElementThreads) k_element_forces(DevModel m) 
     const int64_t row = e0 * q + pq;
     const double jq = m.jac[e * q + pq];
     double gl[9], sl[9];
-    if (pq > 0) rows_load<dn>(m.B + row * dn, q * dn, cnt, lane, B);
-    rows_put<dn, SN>(buf, B, lane);
+    if constexpr (ROWS) {
+      if (pq > 0) rows_load<dn>(m.B + row * dn, q * dn, cnt, lane, B);
+      rows_put<dn, SN>(buf, B, lane);
 #pragma unroll
-    for (int k = 0; k < dn; ++k) B[k] = buf[(on ? lane : 0) * SN + k];
+      for (int k = 0; k < dn; ++k) B[k] = buf[(on ? lane : 0) * SN + k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < dn; ++k) B[k] = m.B[(e * q + pq) * dn + k];
+    }
     ref::mmt<d, d, n>(uel, B, gl);  // nabla_u.mul<false,true>(u_el, B)
 #pragma unroll
     for (int k = 0; k < dd; ++k) gl[k] -= 0.;  // eigengradu
     ref::stress<d>(p, gl, sl);
-    rows_out<dd, SD>(buf, gl, m.gradu + row * dd, q * dd, cnt, lane);
-    rows_out<dd, SD>(buf, sl, m.stress + row * dd, q * dd, cnt, lane);
+    if constexpr (ROWS) {
+      rows_out<dd, SD>(buf, gl, m.gradu + row * dd, q * dd, cnt, lane);
+      rows_out<dd, SD>(buf, sl, m.stress + row * dd, q * dd, cnt, lane);
+    } else if (on) {
+#pragma unroll
+      for (int k = 0; k < dd; ++k) {
+        m.gradu[(e * q + pq) * dd + k] = gl[k];
+        m.stress[(e * q + pq) * dd + k] = sl[k];
+      }
+    }
     ref::qp_force<T>(p, B, gl, sl, r);
 #pragma unroll
     for (int k = 0; k < dn; ++k) inte[k] += r[k] * jq;
-    __syncwarp();  // the buffer is read out
+    if constexpr (ROWS) __syncwarp();  // the buffer is read out
   }
-  rows_out<dn, SN>(buf, inte, static_cast<double*>(m.fe) + e0 * dn, dn, cnt, lane);
+  if constexpr (ROWS) {
+    rows_out<dn, SN>(buf, inte, static_cast<double*>(m.fe) + e0 * dn, dn, cnt, lane);
+  } else if (on) {
+#pragma unroll
+    for (int k = 0; k < dn; ++k) static_cast<double*>(m.fe)[e * dn + k] = inte[k];
+  }
 }
 
 // One thread per DOF: internal force gathered in ascending element order,
@@ -313,10 +338,13 @@ cudaError_t ref_element_forces(const DevModel& m, cudaStream_t s) {
   constexpr int t = kElementThreads;
   const int blocks = (int)((m.ne + t - 1) / t);
   switch (m.type) {
-  case AKB_SEGMENT_2: return launch_pdl(k_element_forces<AKB_SEGMENT_2>, blocks, t, 0, s, m);
-  case AKB_TRIANGLE_3: return launch_pdl(k_element_forces<AKB_TRIANGLE_3>, blocks, t, 0, s, m);
-  case AKB_TETRAHEDRON_4: return launch_pdl(k_element_forces<AKB_TETRAHEDRON_4>, blocks, t, 0, s, m);
-  default: return launch_pdl(k_element_forces<AKB_HEXAHEDRON_8>, blocks, t, 0, s, m);
+  case AKB_SEGMENT_2: return launch_pdl(k_element_forces<AKB_SEGMENT_2, true>, blocks, t, 0, s, m);
+  case AKB_TRIANGLE_3: return launch_pdl(k_element_forces<AKB_TRIANGLE_3, true>, blocks, t, 0, s, m);
+  case AKB_TETRAHEDRON_4: return launch_pdl(k_element_forces<AKB_TETRAHEDRON_4, true>, blocks, t, 0, s, m);
+  default:
+    return m.ne <= kFewHexahedra
+               ? launch_pdl(k_element_forces<AKB_HEXAHEDRON_8, false>, blocks, t, 0, s, m)
+               : launch_pdl(k_element_forces<AKB_HEXAHEDRON_8, true>, blocks, t, 0, s, m);
   }
 }
 

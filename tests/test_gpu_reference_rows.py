@@ -73,3 +73,34 @@ def test_the_step_leaves_its_gradients_and_stresses(k):
         rows = t.transpose(1, 2).reshape(t.shape[0], -1).cpu().numpy()  # column-major again
         assert np.array_equal(rows, np.asarray(cpu.get(f)).reshape(rows.shape)), f
     dev.close()
+
+
+@pytest.mark.parametrize("n", [(2, 1, 1), (8, 4, 1), (11, 3, 1), (6, 4, 2), (7, 7, 1)])
+def test_few_hexahedra(n):
+    """Up to 48 hexahedra the lanes move their own rows: either side of the change
+    and of a warp, bit for bit, the step's gradients and stresses included."""
+    import torch
+    from akantu_b200.model import MaterialElastic, SolidMechanicsModel
+    mesh = box_hexahedron8(*n, *[0.5 * k for k in n])
+    mat = dict(kind=_abi.MATERIAL_ELASTIC, rho=2700.0, E=70e9, nu=0.3)
+    rng = np.random.default_rng(sum(n))
+    v0 = rng.normal(size=np.asarray(mesh.nodes).shape)
+    cpu = OracleAdapter(mesh, mat)
+    dev = SolidMechanicsModel(mesh, [MaterialElastic(rho=2700.0, E=70e9, nu=0.3)])
+    dev.initFull()
+    dt = 0.3 * dev.getStableTimeStep()
+    dev.setTimeStep(dt)
+    cpu.set_time_step(dt)
+    dev.setField(_abi.FIELD_VELOCITY, v0)
+    cpu.set(_abi.FIELD_VELOCITY, v0)
+    views = {f: dev.deviceTensor(f) for f in (_abi.FIELD_GRAD_U, _abi.FIELD_STRESS)}
+    dev.solveSteps(5)
+    dev.synchronize()
+    cpu.solve_steps(5)
+    for f, t in views.items():
+        rows = t.transpose(1, 2).reshape(t.shape[0], -1).cpu().numpy()
+        assert np.array_equal(rows, np.asarray(cpu.get(f)).reshape(rows.shape)), f
+    for f in (_abi.FIELD_DISPLACEMENT, _abi.FIELD_VELOCITY, _abi.FIELD_ACCELERATION,
+              _abi.FIELD_INTERNAL_FORCE):
+        assert np.array_equal(dev.getField(f), cpu.get(f)), f
+    dev.close()
