@@ -261,20 +261,33 @@ akb_status upload(akb_model* m, const std::vector<T>& v, const T** out);
 //    15.7 and 10.8; 20 k tetrahedra 9.2 and 12.0, 41 k 11.5 and 13.4, 79 k 15.5 and
 //    13.5. (A step by itself, which nothing follows, takes the fans of 5 k to 30 k
 //    small-strain triangles 1 us longer.) Hexahedra: faster on fan records at any size.
+//  - Batches of small instances: a patch is at most one of them, and its few fans
+//    leave most of a CTA's threads idle (256 for tetrahedra, two CTAs an SM). us a
+//    step, chunk records and fan records: 1000 boxes of 216 tetrahedra 14.5 and
+//    20.6 (finite-strain 15.2 and 26.9, neo-Hookean 17.0 and 38.0), 400 of 600 12.4 and
+//    11.2 (13.5, 13.5; 15.2, 18.6), 200 of 1296 14.9 and 14.5 (16.3, 17.5; 17.9, 22.9),
+//    80 of 3456 18.3 and 14.7 (19.8, 18.0; 21.9, 23.5), 30 of 10 368 19.2 and 12.1
+//    (20.6, 14.8; 23.1, 18.1); 1000 plates of some 214 triangles 11.6 and 6.4 (12.0, 10.8;
+//    13.8, 15.3), 1000 of 512 14.4 and 12.3 (neo-Hookean 17.4, 19.1), 300 of some 756
+//    12.0 and 8.3 (12.3, 9.2; 14.4, 11.9).
 //  - Patch sizes chosen by the caller: the fan kernels are built for patches
 //    whose fans fill their CTA about once. 280 k triangles at 768 elements 19.8
 //    against 16.2, at 1024 16.6 against 18.5, at 2048 23.7 against 30.7; 1.6 M
 //    tetrahedra at 512 72 against 87, at 768 65 against 49, at 1536 63 against
 //    40; 262 k hexahedra at 256 141 against 79, at 384 101.2 against 101.6, at
 //    512 95 against 104.
-bool use_fans(const akb_model* m, int64_t ne, bool neohookean) {
+bool use_fans(const akb_model* m, int64_t ne, int64_t per_instance, bool neohookean) {
   if (m->mode != AKB_MODE_FP64) return false;
   const int pe = m->opt_patch_elements;
   switch (m->dm.type) {
   case AKB_TRIANGLE_3:
-    return pe > 0 ? pe <= 768 : ne >= (neohookean ? 88000 : m->linear ? 4096 : 45000);
+    if (pe > 0) return pe <= 768;
+    return ne >= (neohookean ? 88000 : m->linear ? 4096 : 45000) &&
+           per_instance >= (neohookean ? 640 : 0);
   case AKB_TETRAHEDRON_4:
-    return pe > 0 ? pe >= 768 : ne >= (neohookean ? 56000 : m->linear ? 4096 : 44000);
+    if (pe > 0) return pe >= 768;
+    return ne >= (neohookean ? 56000 : m->linear ? 4096 : 44000) &&
+           per_instance >= (neohookean ? 6000 : m->linear ? 500 : 2000);
   case AKB_HEXAHEDRON_8: return pe <= 256;
   default: return false;
   }
@@ -852,7 +865,8 @@ static akb_status create_model(const akb_mesh_desc* mesh, int32_t nb_materials,
   if (patched) {
     // FP64 steps run on fan records where these are faster (use_fans), but a
     // plan whose record or contributions do not fit an SM steps chunk by chunk
-    bool fans = use_fans(m.get(), ne, neohookean);
+    bool fans = use_fans(m.get(), ne, batch ? ne / std::max(batch->ninst, 1) : ne,
+                         neohookean);
     if (fans) {
       st = plan_patches(m.get(), mesh, batch, part, true, plan, patch_inst, orphan_inst);
       fans = st == AKB_OK && fan_smem_bytes(plan, d) <= kFanSmemLimit;

@@ -146,6 +146,25 @@ def test_kernel_of_each_side(kind, n, law, patch, name):
         m.close()
 
 
+@pytest.mark.parametrize("kind,n,count,law,name", [
+    ("tet", (4, 4, 5), 12, ELASTIC, "patch_step"), ("tet", (5, 4, 5), 12, ELASTIC, "fan_step"),
+    ("tet", (6, 6, 6), 40, FINITE, "patch_step"), ("tet", (7, 7, 7), 25, FINITE, "fan_step"),
+    ("tet", (6, 8, 7), 30, NEO, "patch_step"), ("tet", (11, 11, 11), 8, NEO, "fan_step"),
+    ("tri", (15, 15), 200, NEO, "patch_step"), ("tri", (21, 21), 100, NEO, "fan_step"),
+    ("tri", (8, 8), 40, ELASTIC, "fan_step"), ("hex", (2, 2, 2), 20, NEO, "fan_step"),
+])
+def test_kernel_of_batches(kind, n, count, law, name):
+    """The same of batches, whose instances can be too small for fans."""
+    from akantu_b200._lib import lib
+    from akantu_b200.batch import BatchModel
+    from akantu_b200.model import material_from_dict
+    b = BatchModel([build(kind, n, 0)] * count, [material_from_dict(law)] * count,
+                   precision=_abi.MODE_FP64)
+    b.initFull()
+    assert lib().akb_kernel_name(b.handle, 0).decode() == name
+    b.close()
+
+
 @pytest.mark.parametrize("load", [False, True], ids=["free", "loaded"])
 @pytest.mark.parametrize("kind,n,mats,jitter,patch", [
     ("tet", (1, 1, 1), ELASTIC, 0, dict(patch_elements=1536)),
