@@ -271,8 +271,12 @@ akb_status upload(akb_model* m, const std::vector<T>& v, const T** out);
 //    13.8, 15.3), 1000 of 512 14.4 and 12.3 (neo-Hookean 17.4, 19.1), 300 of some 756
 //    12.0 and 8.3 (12.3, 9.2; 14.4, 11.9).
 //  - Patch sizes chosen by the caller: the fan kernels are built for patches
-//    whose fans fill their CTA about once. 280 k triangles at 768 elements 19.8
-//    against 16.2, at 1024 16.6 against 18.5, at 2048 23.7 against 30.7; 1.6 M
+//    whose fans fill their CTA about once. The rule goes by the size alone, which
+//    a batch and a model of one of its instances share, not by the law.
+//    280 k triangles at 768 elements 19.8
+//    against 16.2, at 1024 16.6 against 18.5, at 2048 23.7 against 30.7; 240 k at
+//    512 11.2 against 8.3 (neo-Hookean 13.1 and 11.7), at 256 12.5 and 12.5 (14.1 and
+//    18.5), at 128 19.3 and 14.5 (21.3 and 23.9; 6000 of them 6.9 and 8.7); 1.6 M
 //    tetrahedra at 512 72 against 87, at 768 65 against 49, at 1536 63 against
 //    40; 262 k hexahedra at 256 141 against 79, at 384 101.2 against 101.6, at
 //    512 95 against 104.
@@ -281,7 +285,7 @@ bool use_fans(const akb_model* m, int64_t ne, int64_t per_instance, bool neohook
   const int pe = m->opt_patch_elements;
   switch (m->dm.type) {
   case AKB_TRIANGLE_3:
-    if (pe > 0) return pe <= 768;
+    if (pe > 0) return pe > 256 && pe <= 768;
     return ne >= (neohookean ? 88000 : m->linear ? 4096 : 45000) &&
            per_instance >= (neohookean ? 640 : 0);
   case AKB_TETRAHEDRON_4:

@@ -42,7 +42,7 @@ def compare(meshes, materials, opts, steps=40):
     b.close()
 
 
-@pytest.mark.parametrize("patch_elements", [128, 512])
+@pytest.mark.parametrize("patch_elements", [128, 300, 512])
 def test_small_strain_plates_beside_other_laws(patch_elements):
     meshes = [mesh_mod.plate_triangle3(nx, ny, 0.1 * nx, 0.1 * ny)
               for nx, ny in ((30, 20), (7, 3), (41, 9), (25, 17))]

@@ -122,7 +122,8 @@ def test_both_sides_of_the_dispatch(kind, n, mats, patch):
     ("tet", (21, 21, 21), NEO, {}, "patch_step"), ("tet", (21, 21, 22), NEO, {}, "fan_step"),
     ("tri", (60, 20), ELASTIC, dict(patch_elements=768), "fan_step"),
     ("tri", (60, 20), ELASTIC, dict(patch_elements=769), "patch_step"),
-    ("tri", (8, 3), NEO, dict(patch_elements=256), "fan_step"),
+    ("tri", (8, 3), NEO, dict(patch_elements=256), "patch_step"),
+    ("tri", (8, 3), NEO, dict(patch_elements=257), "fan_step"),
     ("tet", (9, 8, 6), ELASTIC, dict(patch_elements=767), "patch_step"),
     ("tet", (9, 8, 6), NEO, dict(patch_elements=768), "fan_step"),
     ("hex", (1, 1, 1), NEO, {}, "fan_step"),
@@ -174,7 +175,7 @@ def test_kernel_of_batches(kind, n, count, law, name):
     ("tet", (6, 5, 7), NEO, 1, dict(patch_elements=768)),
     ("tri", (1, 1), ELASTIC, 0, dict(patch_elements=768)),
     ("tri", (40, 31), [STIFF, ELASTIC], 1, dict(patch_elements=768)),
-    ("tri", (33, 20), [FINITE, STIFF], 1, dict(patch_elements=200, patch_grid=1)),
+    ("tri", (33, 20), [FINITE, STIFF], 1, dict(patch_elements=300, patch_grid=1)),
     ("tri", (40, 21), NEO, 0, dict(patch_elements=512)),
 ])
 def test_fans_of_small_meshes(kind, n, mats, jitter, patch, load):
