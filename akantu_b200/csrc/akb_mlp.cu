@@ -371,7 +371,8 @@ __device__ inline void stage_inputs(const Net& net, int64_t nb, const double* __
 // wait for a slice to be free holds up nobody (with one thread doing both, the
 // wait was 500 of a slice's 1300 cycles). Stress calls, three hidden layers of 256: 1000
 // points 29.0 -> 22.9 us, 20000 33.3 -> 27.1, 262144 206 -> 164, 500000
-// 396 -> 314; a step of 32^3 macro elements 273 -> 231 us, of 8^3 77 -> 65.
+// 396 -> 314 (now 22.5, 25.4, 153 and 296); a step of 32^3 macro elements
+// 273 -> 231 us, of 8^3 77 -> 65.
 template <bool TRAIN, bool STRESS>
 __global__ void __launch_bounds__(kFwdThreads, 2)
     k_forward(Net net, int64_t nb, const double* __restrict__ x, double* __restrict__ y,
@@ -445,19 +446,20 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
       used += K / net.ks[l];
       while (ok && ll < net.nl && loaded < used + kRing) load_next();
     }
-    // the biases of the epilogue's first columns, requested under the MMAs (and
-    // each next 32 under the activations of the ones before): one hidden layer of
-    // 128, 8192 samples 6.98 -> 6.24 us, three of 256 19.4 -> 18.5
     const float* __restrict__ bias = net.b[l];
     const bool last = l == net.nl - 1;
     const int cbeg = last ? 0 : half * (N >> 1), cend = (half + 1) * (N >> 1);
     float4 b4[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (q < 4 || !last) b4[q] = __ldg(reinterpret_cast<const float4*>(bias + cbeg) + q);
     // lanes that waited on the barrier below while one of their warp still
     // issues would suspend the warp, 3000 cycles at a time
     __syncwarp();
+    // the biases of the epilogue's first columns are requested under the MMAs,
+    // the others' ahead of their accumulators: one hidden layer of 128, 8192
+    // samples 7.1 -> 6.3 us, three of 256 19.3 -> 18.4; stresses of 262144 points
+    // 161 -> 153. (Each next 32 under the activations before: 161.)
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < 4 || !last) b4[q] = __ldg(reinterpret_cast<const float4*>(bias + cbeg) + q);
     // (a wait that gave up in one thread ends the layer loop in all)
     if (ok) ok = mbar_wait(mb_done, l & 1);
     if (__syncthreads_or(!ok)) {
@@ -468,6 +470,9 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
     if (!last) {
       for (int c0 = cbeg; c0 < cend; c0 += 32) {
         float v[32];
+        if (c0 > cbeg)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) b4[q] = __ldg(reinterpret_cast<const float4*>(bias + c0) + q);
         tmem_ld32(mine + c0, v);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -476,10 +481,6 @@ __global__ void __launch_bounds__(kFwdThreads, 2)
           v[4 * q + 2] += b4[q].z;
           v[4 * q + 3] += b4[q].w;
         }
-        if (c0 + 32 < cend)
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            b4[q] = __ldg(reinterpret_cast<const float4*>(bias + c0 + 32) + q);
         if (TRAIN && row < nb) {  // the pre-activations: eight 16-byte stores
           float4* z4 = reinterpret_cast<float4*>(bufs.z[l] + (size_t)row * N + c0);
 #pragma unroll
